@@ -1,0 +1,132 @@
+// Checks of the resident PCG's host partition (csrc/partition.cpp) on random
+// meshes: every row has one part, every block one lane of its row with the
+// right local column, every halo row exactly one sender, and the layout's
+// maxima bound every part.  Prints "ok" or the first violation.
+#include <algorithm>
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <set>
+#include <vector>
+
+#include "internal.h"
+
+using namespace mfem;
+
+#define CHECK(cond)                                                     \
+    do {                                                                \
+        if (!(cond)) {                                                  \
+            printf("trial %d, line %d: %s\n", trial, __LINE__, #cond); \
+            return 1;                                                   \
+        }                                                               \
+    } while (0)
+
+int main() {
+    std::mt19937 rng(7);
+    auto below = [&](int k) { return (int)(rng() % (unsigned)k); };
+    for (int trial = 0; trial < 80; ++trial) {
+        // a Kuhn grid, shuffled in half of the trials; degenerate positions and
+        // extra long-range couplings in some
+        const int nx = 1 + below(14), ny = 1 + below(7), nz = 1 + below(7);
+        const int n = (nx + 1) * (ny + 1) * (nz + 1), lo = trial % 3 == 0 ? 5 : 0;
+        std::vector<int> perm(n);
+        for (int i = 0; i < n; ++i) perm[i] = i;
+        if (trial & 1) std::shuffle(perm.begin(), perm.end(), rng);
+        std::vector<float> q(3 * (size_t)(n + lo), 0.0f);
+        std::vector<std::set<int>> adj(n);
+        auto id = [&](int i, int j, int k) { return perm[(i * (ny + 1) + j) * (nz + 1) + k]; };
+        for (int i = 0; i <= nx; ++i)
+            for (int j = 0; j <= ny; ++j)
+                for (int k = 0; k <= nz; ++k) {
+                    const int v = id(i, j, k);
+                    adj[v].insert(v);
+                    const float c[3] = {(float)i, (float)j, (float)k};
+                    for (int a = 0; a < 3; ++a) q[3 * (size_t)(v + lo) + a] = trial % 7 == 3 ? 0.0f : c[a];
+                    for (int d = 1; d < 8; ++d) {
+                        const int i2 = i + (d & 1), j2 = j + ((d >> 1) & 1), k2 = k + (d >> 2);
+                        if (i2 > nx || j2 > ny || k2 > nz) continue;
+                        adj[v].insert(id(i2, j2, k2));
+                        adj[id(i2, j2, k2)].insert(v);
+                    }
+                }
+        if (trial % 11 == 4)
+            for (int t = 0; t < n / 3; ++t) {
+                const int a = below(n), b = below(n);
+                adj[a].insert(b);
+                adj[b].insert(a);
+            }
+        if (trial % 13 == 5) q[3 * (size_t)(lo + below(n))] = NAN;
+        // the body's rows are [lo, lo + n) of the plan's
+        std::vector<int32_t> rp(n + lo + 1, 0), ci;
+        for (int i = 0; i < lo; ++i) {
+            ci.push_back(i);
+            rp[i + 1] = (int32_t)ci.size();
+        }
+        for (int i = 0; i < n; ++i) {
+            for (int c : adj[i]) ci.push_back(c + lo);
+            rp[lo + i + 1] = (int32_t)ci.size();
+        }
+        const int parts = trial % 5 == 0 ? 1 + below(13) : 1 << below(5);
+        ResidentHost h;
+        resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true);
+        CHECK((int)h.parts.size() == parts && h.tasks.size() == 1 && h.tasks[0].y == parts);
+        std::vector<int> seen(n, 0);
+        std::vector<std::vector<int>> sender(parts);
+        for (int p = 0; p < parts; ++p) sender[p].assign(h.parts[p].nhalo, -1);
+        int most = 0, least = n;
+        for (int p = 0; p < parts; ++p) {
+            const ResPart &P = h.parts[p];
+            most = std::max(most, P.nown);
+            least = std::min(least, P.nown);
+            CHECK(P.nown <= h.nown_max && P.nhalo <= h.nhalo_max && P.nown + P.nhalo <= h.nlocal_max);
+            CHECK(P.push_passes * P.nslices * 32 <= h.push_max);
+            for (int s = 0; s < P.nslices; ++s)
+                for (int lane = 0; lane < 32; ++lane)
+                    for (int e = 0; e < P.push_passes; ++e) {
+                        const int d = h.push[P.push_off + (e * P.nslices + s) * 32 + lane];
+                        const int r = s * kPartSliceRows + lane % kPartSliceRows;
+                        if (d < 0) continue;
+                        CHECK(r < P.nown && (d >> 16) < parts && (d >> 16) != p);
+                        CHECK((d & 0xffff) < h.parts[d >> 16].nhalo && sender[d >> 16][d & 0xffff] < 0);
+                        sender[d >> 16][d & 0xffff] = h.rows[P.row_off + r];
+                    }
+            std::vector<std::set<int>> blocks(P.nown);
+            std::vector<int> warp(kPartWarps, 0), reg(kPartWarps, 0);
+            for (int s = 0; s < P.nslices; ++s) {
+                const int t0 = h.trip_ptr[P.slice_off + s], t1 = h.trip_ptr[P.slice_off + s + 1];
+                CHECK(t1 > t0 && t1 - t0 <= h.slice_trips_max);
+                warp[s % kPartWarps] += t1 - t0;
+                if (s < kPartWarps) reg[s] = std::min(t1 - t0, kPartRegTrips);
+                for (int t = t0; t < t1; ++t)
+                    for (int lane = 0; lane < 32; ++lane) {
+                        const int k = h.src[32 * t + lane], c = h.col[32 * t + lane];
+                        const int r = s * kPartSliceRows + lane % kPartSliceRows;
+                        if (k < 0) {
+                            CHECK(c == 0);
+                            continue;
+                        }
+                        CHECK(r < P.nown);
+                        const int row = h.rows[P.row_off + r];
+                        CHECK(k >= rp[row] && k < rp[row + 1]);
+                        CHECK(c >= 0 && c < P.nown + P.nhalo);
+                        CHECK((c < P.nown ? h.rows[P.row_off + c] : h.halo[P.halo_off + c - P.nown]) == ci[k]);
+                        blocks[r].insert(k);
+                    }
+            }
+            for (int w = 0; w < kPartWarps; ++w)
+                CHECK(warp[w] <= h.trips_max && warp[w] - reg[w] <= h.trips_max_reg);
+            for (int i = 0; i < P.nown; ++i) {
+                const int row = h.rows[P.row_off + i];
+                CHECK(row >= lo && row < lo + n);
+                ++seen[row - lo];
+                CHECK((int)blocks[i].size() == rp[row + 1] - rp[row]);
+            }
+        }
+        CHECK(most - least <= 2);
+        for (int v : seen) CHECK(v == 1);
+        for (int p = 0; p < parts; ++p)
+            for (int i = 0; i < h.parts[p].nhalo; ++i) CHECK(sender[p][i] == h.halo[h.parts[p].halo_off + i]);
+    }
+    puts("ok");
+    return 0;
+}

@@ -48,7 +48,12 @@ struct mfem_plan {
     PcgLayout pl{};
     // block-Jacobi plans: the persistent factor PCG's layout (block-Jacobi
     // only) for the inner solves of the mixed refinement, when it fits
+    // (plan_refinement)
     PcgLayout ir_pl{};
+    bool ir_pl_tried = false;
+    // block-Jacobi plans of a mesh that one cluster holds: its parts
+    // (mfem_plan_create); cluster 0: none
+    ResidentLayout rl{};
     LineSearchWork ls{};
     float stage_dt = 0.0f;     // dt of the last mfem_assemble (the line search's 1/dt^2)
     int stage_slot = 0;        // slot of the last mfem_global_solve
@@ -109,6 +114,10 @@ struct mfem_plan {
 
 namespace {
 
+// Rows a CTA up to which one cluster beats a grid: 16 CTAs of 370 rows 3.0 us
+// an iteration.
+constexpr int kClusterRows = 400;
+
 struct DeviceGuard {
     int prev = -1;
     bool ok = true;
@@ -140,6 +149,7 @@ int cuda_fail(mfem_plan *p, cudaError_t err, const char *what) {
 // next launch's barriers early) and the flag cleared.
 cudaError_t rearm_barriers(mfem_plan *p) {
     cudaError_t e = cudaMemset(p->pw.counter, 0, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemset(p->pw.res_counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(p->ls.counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess && p->ir.counter) e = cudaMemset(p->ir.counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess && p->bw.n_bodies > 0 && p->bw.counter)
@@ -238,11 +248,14 @@ cudaError_t global_solve(mfem_plan *p, int slot, cudaStream_t s) {
     if (p->ir.mode != 0)
         return launch_mixed_solve(p->bv, p->vv, p->ir, p->pw, p->bw,
                                   p->pl.variant == PcgLayout::kFactor ? p->pl : p->ir_pl,
-                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr, p->pcg_ctas, slot,
-                                  p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
+                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr, p->rl, p->pcg_ctas,
+                                  slot, p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
     if (p->pl.variant == PcgLayout::kFactor)
         return launch_pcg_factor(p->bv, p->vv, p->pw, p->bw, p->pl, p->pcg_ctas, slot, p->cfg.cg_tolerance,
                                  p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
+    if (p->bw.n_bodies == 0 && p->rl.cluster > 0)
+        return launch_resident(p->bv, p->vv, p->rl, 1, 1, p->pw, p->pw.stats, slot, p->cfg.cg_tolerance,
+                               p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr, s);
     if (p->bw.n_bodies > 0)
         return launch_batched_pcg(p->bv, p->vv, p->bw, p->pw.error, slot, p->cfg.cg_tolerance,
                                   p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
@@ -354,6 +367,98 @@ void batch_schedule(const std::vector<int32_t> &nnzb, const std::vector<int32_t>
         task_ptr.push_back((int)tasks.size());
     }
     ctas = capacity;
+}
+
+// Uploads a host partition; its arrays live in `allocs`.
+cudaError_t upload_resident(std::vector<void *> &allocs, const ResidentHost &h, ResidentViews &v) {
+    cudaError_t e = cudaSuccess;
+    auto put = [&](auto **dst, const auto &src) {
+        if (e != cudaSuccess) return;
+        void *raw = nullptr;
+        e = cudaMalloc(&raw, std::max<size_t>(src.size() * sizeof(src[0]), 16));
+        if (e != cudaSuccess) return;
+        allocs.push_back(raw);
+        if (!src.empty()) e = cudaMemcpy(raw, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice);
+        *dst = static_cast<std::remove_reference_t<decltype(*dst)>>(raw);
+    };
+    put(&v.parts, h.parts);
+    put(&v.tasks, h.tasks);
+    put(&v.rows, h.rows);
+    put(&v.halo, h.halo);
+    put(&v.trip_ptr, h.trip_ptr);
+    put(&v.src, h.src);
+    put(&v.col, h.col);
+    put(&v.push, h.push);
+    return e;
+}
+
+// A block-Jacobi plan's layout of the persistent factor PCG (without factor
+// rows) for the inner solves of the mixed refinement, where it fits; made by
+// the first mfem_plan_set_solver that refines.
+cudaError_t plan_refinement(mfem_plan *p) {
+    if (p->ir_pl_tried || p->global_memory_pcg || p->cfg.preconditioner != 1) return cudaSuccess;
+    p->ir_pl_tried = true;
+    std::string lerr;
+    PcgLayout il{};
+    std::vector<int4> cta, fcta;
+    if (pcg_factor_layout(p->device, il, p->h_row_ptr.data(), p->h_col_idx.data(), p->n, p->pcg_ctas, 2, cta, fcta,
+                          lerr, false) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaSuccess;
+    }
+    int4 *d_cta = nullptr, *d_fcta = nullptr;
+    cudaError_t e = dev_alloc(p, &d_cta, cta.size());
+    if (e == cudaSuccess) e = upload(d_cta, cta.data(), cta.size());
+    if (e == cudaSuccess) e = dev_alloc(p, &d_fcta, fcta.size());
+    if (e == cudaSuccess) e = upload(d_fcta, fcta.data(), fcta.size());
+    if (e != cudaSuccess) return e;
+    il.cta_info = d_cta;
+    il.factor_info = d_fcta;
+    p->ir_pl = il;
+    return cudaSuccess;
+}
+
+// The trips that a layout streams: a buffer of the plan's.
+cudaError_t alloc_stream(std::vector<void *> &allocs, size_t parts, ResidentLayout &L) {
+    if (L.stream_trips == 0) return cudaSuccess;
+    void *raw = nullptr;
+    const cudaError_t e = cudaMalloc(&raw, parts * kPartWarps * (size_t)L.stream_trips * 1280);
+    if (e != cudaSuccess) return e;
+    allocs.push_back(raw);
+    L.v.stream = static_cast<float4 *>(raw);
+    return e;
+}
+
+// The resident PCG of one mesh: a cluster, or past what 16 CTAs hold on the
+// chip a grid of one CTA an SM.  A part takes at most 128 rows, one slice a
+// warp, while the cluster may grow: an iteration takes 1.0 us on one CTA and
+// 1.43 us in clusters of 4 to 16 (99 to 1,225 rows), a further slice a warp
+// 0.45 us.
+cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q, int max_ctas) {
+    constexpr int kRows = kPartWarps * kPartSliceRows;
+    for (int form = 0; form < 2; ++form) {
+        const bool grid = form == 1;
+        int parts = 1;
+        if (grid) {
+            parts = std::min(std::min(max_ctas, kPartMaxGrid), (p->n + kRows - 1) / kRows);
+        } else {
+            while (parts < kPartMaxCluster && parts * kRows < p->n) parts *= 2;
+            if (p->n > kPartMaxCluster * kClusterRows) continue;
+        }
+        if (p->n > parts * 2 * kPartThreads) return cudaSuccess;
+        ResidentHost h;
+        resident_add_body(h, sym.row_ptr.data(), sym.col_idx.data(), rest_q, 0, p->n, parts, 0, !grid);
+        bool fits = false;
+        ResidentLayout L;
+        cudaError_t e = resident_layout(p->device, h, parts, grid, L, fits);
+        if (e != cudaSuccess) return e;
+        if (!fits || (!grid && L.stream_trips > 0)) continue;
+        e = upload_resident(p->allocs, h, L.v);
+        if (e == cudaSuccess) e = alloc_stream(p->allocs, h.parts.size(), L);
+        if (e == cudaSuccess) p->rl = L;
+        return e;
+    }
+    return cudaSuccess;
 }
 
 uint64_t count_kernel_nodes(cudaGraph_t g) {
@@ -546,9 +651,10 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     ALLOC(chunk_ptr, (size_t)n_chunks + 1);
     ALLOC(ccode, sym.contrib_code.size());
     ALLOC(cslot, sym.contrib_slot.size());
-    ALLOC(p->pw.pub, 6 * n_pad * 3);
+    ALLOC(p->pw.pub, 6 * n_pad * 3);  // also the resident PCG's [2][n] float4
     ALLOC(p->pw.partials, 2 * 256 * 4);
     ALLOC(p->pw.counter, 1);
+    ALLOC(p->pw.res_counter, 1);
     ALLOC(p->pw.error, 1);
     ALLOC(p->pw.stats, (size_t)p->max_stats);
     ALLOC(p->resid, 2);
@@ -632,19 +738,9 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
             cta_info.assign(1, make_int4(0, 0, 0, 0));
         }
     }
-    std::vector<int4> ir_cta, ir_fcta;
-    if (e == cudaSuccess && !p->global_memory_pcg && cfg.preconditioner == 1) {
-        std::string lerr;
-        PcgLayout il{};
-        if (pcg_factor_layout(device, il, sym.row_ptr.data(), sym.col_idx.data(), n, p->pcg_ctas, 2, ir_cta, ir_fcta,
-                              lerr, false) == cudaSuccess) {
-            p->ir_pl = il;
-        } else {
-            cudaGetLastError();
-            ir_cta.clear();
-            ir_fcta.clear();
-        }
-    }
+    if (e == cudaSuccess && !p->global_memory_pcg && cfg.preconditioner <= 1 && cfg.pcg_ctas == 0 &&
+        (cfg.pcg_variant == PcgLayout::kAuto || cfg.pcg_variant == PcgLayout::kSingleReduction))
+        e = plan_resident(p, sym, h_rest_q, max_ctas);
     int4 *d_cta = nullptr;
     if (e == cudaSuccess) e = dev_alloc(p, &d_cta, cta_info.size());
     if (e == cudaSuccess) e = upload(d_cta, cta_info.data(), cta_info.size());
@@ -654,15 +750,6 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
         e = dev_alloc(p, &d_fcta, factor_info.size());
         if (e == cudaSuccess) e = upload(d_fcta, factor_info.data(), factor_info.size());
         p->pl.factor_info = d_fcta;
-    }
-    if (e == cudaSuccess && p->ir_pl.variant == PcgLayout::kFactor) {
-        int4 *d_icta = nullptr, *d_ifcta = nullptr;
-        e = dev_alloc(p, &d_icta, ir_cta.size());
-        if (e == cudaSuccess) e = upload(d_icta, ir_cta.data(), ir_cta.size());
-        if (e == cudaSuccess) e = dev_alloc(p, &d_ifcta, ir_fcta.size());
-        if (e == cudaSuccess) e = upload(d_ifcta, ir_fcta.data(), ir_fcta.size());
-        p->ir_pl.cta_info = d_icta;
-        p->ir_pl.factor_info = d_ifcta;
     }
     if (e == cudaSuccess) e = upload(tets, reinterpret_cast<const int4 *>(h_tets), nT);
     if (e == cudaSuccess) e = upload(dminv, h_poses, nT * 9);
@@ -681,6 +768,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     if (e == cudaSuccess) e = upload(cslot, sym.contrib_slot.data(), sym.contrib_slot.size());
     if (e == cudaSuccess) e = cudaMemset(p->pw.partials, 0, 2 * 256 * 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(p->pw.counter, 0, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemset(p->pw.res_counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(p->pw.error, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->ls.counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(p->ls.stats, 0, sizeof(LineSearchStats) * p->max_stats);
@@ -761,10 +849,12 @@ int mfem_plan_sizes(const mfem_plan *p, int32_t *n, int32_t *T, int64_t *nnzb) {
 int mfem_plan_pcg_layout(const mfem_plan *p, int32_t *variant, int32_t *ctas, int32_t *cache_matrix,
                          int64_t *smem_bytes) {
     if (!p) return MFEM_BAD_ARG;
-    if (variant) *variant = p->pl.variant;
-    if (ctas) *ctas = p->pcg_ctas;
-    if (cache_matrix) *cache_matrix = p->pl.cache_matrix;
-    if (smem_bytes) *smem_bytes = (int64_t)p->pl.smem;
+    // the resident PCG is the single-reduction iteration with H on the chip
+    const bool resident = p->rl.cluster > 0 && p->bw.n_bodies == 0 && (p->ir.mode == 0 || p->ir.mode == kIrFp32);
+    if (variant) *variant = resident ? (int)PcgLayout::kSingleReduction : p->pl.variant;
+    if (ctas) *ctas = resident ? p->rl.cluster : p->pcg_ctas;
+    if (cache_matrix) *cache_matrix = resident ? p->rl.stream_trips == 0 : p->pl.cache_matrix;
+    if (smem_bytes) *smem_bytes = (int64_t)(resident ? p->rl.smem : p->pl.smem);
     return MFEM_OK;
 }
 
@@ -1151,6 +1241,8 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     if (cfg.factor_refresh < 0) return fail(p, MFEM_BAD_ARG, "factor_refresh must be >= 0");
     p->factor_refresh = std::max(1, cfg.factor_refresh);
     if (cfg.precision == MFEM_PRECISION_FP32) return MFEM_OK;
+    e = plan_refinement(p);
+    if (e != cudaSuccess) return cuda_fail(p, e, "refinement layout");
 
     const size_t n3 = (size_t)p->n * 3, nz = (size_t)p->nnzb;
     auto alloc = [&](auto **ptr, size_t bytes) {

@@ -171,6 +171,7 @@ struct PcgWork {
     float *pub;                // 6 x [n_pad][3] vectors published between CTAs each iteration
     float *partials;           // [2][256][4] per-CTA partial sums, double buffered by barrier parity
     unsigned long long *counter;  // grid barrier arrivals, never reset
+    unsigned long long *res_counter;  // the resident PCG's (its grid has another size)
     int *error;                // sticky device error flag (timeouts)
     SolveStats *stats;         // [max solves per step]
 };
@@ -295,6 +296,62 @@ struct PcgLayout {
     size_t smem = 0;           // dynamic shared memory per CTA
 };
 
+// The resident PCG (pcg_resident.cu): each body's rows are split into parts,
+// one CTA a part, that keep their vectors in registers and their blocks in
+// registers and shared memory for the whole solve.
+constexpr int kPartLanes = 4;       // lanes per block row in the product
+constexpr int kPartSliceRows = 8;   // rows a warp multiplies at once
+constexpr int kPartWarps = 16;
+constexpr int kPartThreads = 32 * kPartWarps;
+constexpr int kPartMaxCluster = 16;
+constexpr int kPartMaxGrid = 256;
+constexpr int kPartRegTrips = 4;    // trips of a warp's first slice whose blocks stay in registers
+
+struct ResPart {
+    int row_off, nown;       // own rows: rows[row_off ..]
+    int halo_off, nhalo;     // rows of other parts that the own rows' columns reach
+    int slice_off, nslices;  // trip_ptr[slice_off + s]: first trip of slice s
+    int push_off, push_passes;  // push[push_off + (pass * nslices + slice) * 32 + lane]
+};
+
+// The parts of a plan's bodies as the host builds them (partition.cpp).
+struct ResidentHost {
+    std::vector<ResPart> parts;
+    std::vector<int4> tasks;                  // per body: (first part, parts, body, rows)
+    std::vector<int32_t> rows, halo;          // vertex ids
+    std::vector<int32_t> trip_ptr, src;       // per trip and lane: slot of the block (-1: none) ...
+    std::vector<uint16_t> col;                // ... and its local column
+    std::vector<int32_t> push;                // (part << 16 | halo index) that a lane sends its row's product to, or -1
+    int nown_max = 0, nhalo_max = 0, nlocal_max = 0, push_max = 0;
+    int trips_max = 0, trips_max_reg = 0;  // most trips of a warp, in all and without its register trips
+    int slice_trips_max = 0;
+};
+void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
+                       int row_lo, int row_hi, int parts, int body, bool push_lists);
+
+struct ResidentViews {
+    const ResPart *parts;
+    const int4 *tasks;
+    const int *rows, *halo, *trip_ptr, *src, *push;
+    const uint16_t *col;
+    float4 *stream;  // trips that fit neither registers nor shared memory
+};
+
+// How a plan runs its PCG on the resident kernels.
+struct ResidentLayout {
+    int cluster = 0;       // parts of a body; 0: the plan has no resident layout
+    bool grid = false;     // the parts meet in global memory (a cooperative grid), else in a cluster
+    int own_slots = 1, row_slots = 1;  // own rows, and rows in all, that a thread keeps
+    int nown_max = 0, nhalo_max = 0;
+    int smem_trips = 0;    // trips a warp keeps in shared memory
+    int stream_trips = 0;  // trips a warp streams from global memory
+    size_t smem = 0;       // dynamic shared memory per CTA
+    ResidentViews v{};
+};
+// `fits` false: the parts do not fit in this layout's registers and shared
+// memory.
+cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool grid, ResidentLayout &L, bool &fits);
+
 // One edge-bisection pass of adaptive refinement (refine.cu) over a plan's
 // mesh.  Edges are the upper off-diagonal slots of H's sparsity (row < col),
 // so a slot index doubles as the edge's id and ascending slots are ascending
@@ -410,6 +467,11 @@ cudaError_t launch_pcg(const BsrViews &bv, const VertexViews &vv, const PcgWork 
 // inner_tol from 0, the correction in ir.e, ir.state updated.
 cudaError_t launch_pcg_inner(const BsrViews &bv, const VertexViews &vv, const IrWork &ir, const PcgWork &w,
                              const PcgLayout &L, int ctas, int slot, int maxiter, cudaStream_t s);
+// n_tasks bodies' PCGs on the resident kernel (L.v.tasks), or with `ir` an
+// inner solve of the refinement's launch sequence (ir.res to ir.e).
+cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const ResidentLayout &L, int n_tasks,
+                            int n_bodies, const PcgWork &w, SolveStats *stats, int slot, float tol, int maxiter,
+                            int use_precond, const IrWork *ir, cudaStream_t s);
 cudaError_t pcg_max_ctas(int device, int *ctas);
 cudaError_t pcg_plan_layout(int device, PcgLayout &L, const int32_t *row_ptr, const int32_t *col_idx, int n,
                             int ctas, int variant, std::vector<int4> &cta_info, std::string &err);
@@ -433,11 +495,13 @@ cudaError_t batch_capacity(int device, int threads, bool factor, int *ctas);
 cudaError_t launch_batched_pcg(const BsrViews &bv, const VertexViews &vv, const BatchViews &bw, int *error, int slot,
                                float tol, int maxiter, int use_precond, cudaStream_t s);
 int ir_residual_blocks(int n);
-// single: the plan's single-reduction layout, or null.  With fp32 blocks and
-// block-Jacobi the inner solves run there, one launch a correction.
+// With fp32 blocks and block-Jacobi the inner solves run on the resident
+// layout rl where the plan has one (rl.cluster > 0), else on its
+// single-reduction layout (single, or null), one launch a correction.
 cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const IrWork &w, const PcgWork &pw,
-                               const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single, int pcg_ctas,
-                               int slot, int maxiter, int use_precond, cudaStream_t s);
+                               const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single,
+                               const ResidentLayout &rl, int pcg_ctas, int slot, int maxiter, int use_precond,
+                               cudaStream_t s);
 // The whole mixed refinement in one launch of the persistent factor PCG
 // (needs IrWork's xf_hi / xf_lo): the warm start in vv.dx, the solution
 // written back there.
