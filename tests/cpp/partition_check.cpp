@@ -68,7 +68,18 @@ int main() {
         }
         const int parts = trial % 5 == 0 ? 1 + below(13) : 1 << below(5);
         ResidentHost h;
-        resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true);
+        const int32_t off[3] = {0, lo, lo + n};
+        if (trial % 4 == 2 && lo > 0) {
+            // behind a body of single rows: joined arrays
+            ResidentHost both;
+            resident_add_bodies(both, rp.data(), ci.data(), q.data(), off, {0, 1}, parts);
+            CHECK((int)both.parts.size() == 2 * parts && both.tasks.size() == 2 && both.tasks[1].x == parts);
+            both.parts.erase(both.parts.begin(), both.parts.begin() + parts);
+            both.tasks.erase(both.tasks.begin());
+            h = both;
+        } else {
+            resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true);
+        }
         CHECK((int)h.parts.size() == parts && h.tasks.size() == 1 && h.tasks[0].y == parts);
         std::vector<int> seen(n, 0);
         std::vector<std::vector<int>> sender(parts);

@@ -140,3 +140,23 @@ def test_set_bodies_rejects_bad_input():
     P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
     rc = solver._lib.mfem_plan_set_bodies(solver._plan, 3, *[P(a) for a in h])
     assert rc == _lib.MFEM_BAD_ARG and b"line_search" in solver._lib.mfem_plan_last_error(solver._plan)
+
+
+@pytest.mark.parametrize("cells", [[(3, 2, 2), (30, 14, 12), (7, 6, 5), (9, 4, 4)],
+                                   [(48, 12, 12), (40, 14, 14), (4, 2, 2)]],
+                         ids=["clusters_1_to_16", "two_rows_a_thread"])
+def test_resident_bodies_agree_with_the_global_memory_pcg(cells):
+    """Bodies on clusters of every size in one batch, up to bodies past 16 x
+    512 rows, against the global-memory PCG: both converge to 1e-6, positions
+    agree to 1e-5 of the largest as between schedules."""
+    bodies = [beams.build_beam(beams.BeamSpec(name=f"b{i}", cells=c, extent=tuple(0.05 * k for k in c),
+                                              energy="arap" if i % 2 else "neohookean", E=(1e4, 1e6), nu=0.4,
+                                              seed=20 + i)) for i, c in enumerate(cells)]
+    batch = beams.concatenate(bodies)
+    outs = []
+    for kw in ({}, dict(pcg_variant="global_memory")):
+        bs = BatchedSolver(batch, device=DEV, **kw)
+        q, stats = run(bs, 2)
+        assert all((s["status"] == _lib.MFEM_OK).all() for s in stats)
+        outs.append(q)
+    assert np.abs(outs[0] - outs[1]).max() <= 1e-5 * np.abs(outs[0]).max()

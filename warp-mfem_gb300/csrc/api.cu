@@ -64,6 +64,7 @@ struct mfem_plan {
     std::vector<void *> contact_allocs;
     // host copies kept to rebuild the assembly's contribution lists
     std::vector<int32_t> h_tets, h_row_ptr, h_col_idx, h_tet_slots;
+    std::vector<float> h_rest;  // [n][3] rest positions (the resident PCG's parts)
     const int32_t *base_chunk_ptr = nullptr, *base_code = nullptr, *base_slot = nullptr;
     int base_chunks = 0;
     // mixed-precision global solve (mfem_plan_set_solver); mode 0 = the
@@ -73,6 +74,18 @@ struct mfem_plan {
     // independent bodies (mfem_plan_set_bodies): per-body PCGs in one launch
     BatchViews bw{};
     std::vector<void *> batch_allocs;
+    // block-Jacobi bodies on the resident PCG: one launch per cluster size, the
+    // largest first, each on a stream of its own (forked from and joined to the
+    // step's); empty: the global-memory PCG
+    struct ResidentClass {
+        ResidentLayout L;
+        int tasks = 0;
+        cudaStream_t stream = nullptr;  // null: the step's own
+        cudaEvent_t done = nullptr;
+    };
+    std::vector<ResidentClass> body_classes;
+    cudaEvent_t body_fork = nullptr;
+    bool bodies_resident = false;  // body_classes in use (mfem_plan_autotune_batch decides)
     int factor_refresh = 1;      // recompute a factor preconditioner every this many Newton iterations
     int bw_max_group = INT_MAX;  // the schedule's group cap and barrier cost
     double bw_c0 = 2048.0;
@@ -242,6 +255,25 @@ bool valid_config(const mfem_config *cfg, std::string &err) {
 // A plan with the learned preconditioner needs its net before any assembly.
 bool net_ready(const mfem_plan *p) { return p->cfg.preconditioner != 3 || p->fv.ready; }
 
+// Every body's PCG on the resident kernel.
+cudaError_t solve_bodies(mfem_plan *p, int slot, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    const size_t classes = p->body_classes.size();
+    if (classes > 1) e = cudaEventRecord(p->body_fork, s);
+    for (size_t i = 0; e == cudaSuccess && i < classes; ++i) {
+        const auto &c = p->body_classes[i];
+        if (c.stream) e = cudaStreamWaitEvent(c.stream, p->body_fork, 0);
+        if (e == cudaSuccess)
+            e = launch_resident(p->bv, p->vv, c.L, c.tasks, p->bw.n_bodies, p->pw, p->bw.stats, slot,
+                                p->cfg.cg_tolerance, p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr,
+                                c.stream ? c.stream : s);
+        if (e == cudaSuccess && c.stream) e = cudaEventRecord(c.done, c.stream);
+    }
+    for (const auto &c : p->body_classes)
+        if (e == cudaSuccess && c.stream) e = cudaStreamWaitEvent(s, c.done, 0);
+    return e;
+}
+
 // The whole step as a launch sequence on one stream.
 // The reference's float32 PCG, or the mixed-precision iterative refinement.
 cudaError_t global_solve(mfem_plan *p, int slot, cudaStream_t s) {
@@ -256,6 +288,7 @@ cudaError_t global_solve(mfem_plan *p, int slot, cudaStream_t s) {
     if (p->bw.n_bodies == 0 && p->rl.cluster > 0)
         return launch_resident(p->bv, p->vv, p->rl, 1, 1, p->pw, p->pw.stats, slot, p->cfg.cg_tolerance,
                                p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr, s);
+    if (p->bodies_resident) return solve_bodies(p, slot, s);
     if (p->bw.n_bodies > 0)
         return launch_batched_pcg(p->bv, p->vv, p->bw, p->pw.error, slot, p->cfg.cg_tolerance,
                                   p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
@@ -544,6 +577,11 @@ void mfem_plan_destroy(mfem_plan *p) {
         for (auto &ge : p->graphs)
             if (ge.exec) cudaGraphExecDestroy(ge.exec);
         if (p->capture_stream) cudaStreamDestroy(p->capture_stream);
+        for (auto &c : p->body_classes) {
+            if (c.done) cudaEventDestroy(c.done);
+            if (c.stream) cudaStreamDestroy(c.stream);
+        }
+        if (p->body_fork) cudaEventDestroy(p->body_fork);
         for (void *a : p->allocs) cudaFree(a);
         for (void *a : p->contact_allocs) cudaFree(a);
         for (void *a : p->ir_allocs) cudaFree(a);
@@ -808,6 +846,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     p->base_slot = cslot;
     p->base_chunks = n_chunks;
     p->h_tets.assign(h_tets, h_tets + (size_t)T * 4);
+    p->h_rest.assign(h_rest_q, h_rest_q + nn * 3);
     p->h_row_ptr = sym.row_ptr;
     p->h_col_idx = sym.col_idx;
     p->h_tet_slots = sym.tet_slots;
@@ -1444,6 +1483,79 @@ int apply_batch_layout(mfem_plan *p, int threads, double c0, int max_group) {
     return MFEM_OK;
 }
 
+void drop_body_classes(mfem_plan *p) {
+    for (auto &c : p->body_classes) {
+        if (c.done) cudaEventDestroy(c.done);
+        if (c.stream) cudaStreamDestroy(c.stream);
+    }
+    p->body_classes.clear();
+    if (p->body_fork) cudaEventDestroy(p->body_fork);
+    p->body_fork = nullptr;
+    p->bodies_resident = false;
+}
+
+// Clusters for block-Jacobi bodies.  A body takes ceil(rows / cap) CTAs,
+// rounded up to a size of the list; the cap is the smallest of 128, 256 and
+// 384 rows (one to three slices a warp) whose clusters all run at once, or 384:
+// fewer rows a CTA shorten an iteration (1.4 us at 128, 0.45 more a further
+// slice), more rows raise the bodies in flight.  Nothing is set (and nothing
+// is wrong) when a body is too large for a cluster of 16.
+cudaError_t plan_bodies(mfem_plan *p, int n_bodies, const int32_t *voff) {
+    static const int kSizes[] = {1, 2, 3, 4, 6, 8, 12, 16};
+    int sms = 1;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
+    std::vector<int> size(n_bodies);
+    for (int cap = 128; cap <= 384; cap += 128) {
+        int64_t ctas = 0;
+        for (int b = 0; b < n_bodies; ++b) {
+            const int need = (voff[b + 1] - voff[b] + cap - 1) / cap;
+            size[b] = kPartMaxCluster;
+            for (int c : kSizes)
+                if (c >= need) {
+                    size[b] = c;
+                    break;
+                }
+            ctas += size[b];
+        }
+        // clusters of 16 leave up to a quarter of the SMs idle
+        if (ctas <= sms * 3 / 4) break;
+    }
+    std::vector<mfem_plan::ResidentClass> classes;
+    for (int i = (int)(sizeof(kSizes) / sizeof(kSizes[0])) - 1; e == cudaSuccess && i >= 0; --i) {
+        std::vector<int> members;
+        for (int b = 0; b < n_bodies; ++b)
+            if (size[b] == kSizes[i]) members.push_back(b);
+        if (members.empty()) continue;
+        // the largest first: clusters start in order as SMs come free
+        std::stable_sort(members.begin(), members.end(),
+                         [&](int a, int b) { return voff[a + 1] - voff[a] > voff[b + 1] - voff[b]; });
+        ResidentHost h;
+        resident_add_bodies(h, p->h_row_ptr.data(), p->h_col_idx.data(), p->h_rest.data(), voff, members,
+                            kSizes[i]);
+        mfem_plan::ResidentClass c;
+        bool fits = false;
+        e = resident_layout(p->device, h, kSizes[i], false, c.L, fits);
+        if (e != cudaSuccess || !fits) return e;
+        c.tasks = (int)members.size();
+        e = upload_resident(p->batch_allocs, h, c.L.v);
+        if (e == cudaSuccess) e = alloc_stream(p->batch_allocs, h.parts.size(), c.L);
+        classes.push_back(c);
+    }
+    p->body_classes = classes;
+    for (size_t i = 0; e == cudaSuccess && i < p->body_classes.size(); ++i) {
+        auto &c = p->body_classes[i];
+        if (i == 0) {
+            if (p->body_classes.size() > 1) e = cudaEventCreateWithFlags(&p->body_fork, cudaEventDisableTiming);
+            continue;
+        }
+        e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c.done, cudaEventDisableTiming);
+    }
+    if (e == cudaSuccess) p->bodies_resident = !p->body_classes.empty();
+    else drop_body_classes(p);
+    return e;
+}
+
 void drop_graphs(mfem_plan *p) {
     for (auto &ge : p->graphs) {
         if (ge.exec) cudaGraphExecDestroy(ge.exec);
@@ -1475,6 +1587,7 @@ int install_bodies(mfem_plan *p, int n_bodies, const int32_t *voff, const int32_
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cuda_fail(p, e, "cudaDeviceSynchronize");
     drop_graphs(p);
+    drop_body_classes(p);
     for (void *a : p->batch_allocs) cudaFree(a);
     p->batch_allocs.clear();
     p->bw = BatchViews{};
@@ -1618,9 +1731,17 @@ int install_bodies(mfem_plan *p, int n_bodies, const int32_t *voff, const int32_
     // bodies: the work-weighted schedule, groups as large as helps
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
-    const int rc = n_bodies == 1 ? apply_batch_layout(p, 512, 2048.0, std::max(1, sms))
-                                 : apply_batch_layout(p, 256, 2048.0, INT_MAX);
+    int rc = n_bodies == 1 ? apply_batch_layout(p, 512, 2048.0, std::max(1, sms))
+                           : apply_batch_layout(p, 256, 2048.0, INT_MAX);
+    // pcg_variant 5 asks for the global-memory PCG; a one-body batch of a mesh
+    // too large for the persistent PCGs has no gravity of its own
+    if (rc == MFEM_OK && gravity && p->cfg.preconditioner <= 1 && p->cfg.pcg_ctas == 0 &&
+        (p->cfg.pcg_variant == PcgLayout::kAuto || p->cfg.pcg_variant == PcgLayout::kSingleReduction)) {
+        e = plan_bodies(p, n_bodies, voff);
+        if (e != cudaSuccess) rc = cuda_fail(p, e, "resident bodies");
+    }
     if (rc != MFEM_OK) {
+        drop_body_classes(p);
         for (void *a : p->batch_allocs) cudaFree(a);
         p->batch_allocs.clear();
         p->bw = BatchViews{};
@@ -1797,6 +1918,12 @@ int mfem_plan_batch_layout(const mfem_plan *p, int32_t *ctas, int32_t *threads) 
     if (!p) return MFEM_BAD_ARG;
     if (ctas) *ctas = p->bw.ctas;
     if (threads) *threads = p->bw.threads;
+    if (p->bodies_resident) {
+        int total = 0;
+        for (const auto &c : p->body_classes) total += c.tasks * c.L.cluster;
+        if (ctas) *ctas = total;
+        if (threads) *threads = kPartThreads;
+    }
     return MFEM_OK;
 }
 
@@ -1837,6 +1964,34 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
             for (size_t b = 0; b < st.size(); ++b) p->h_body_its[b] = std::max(1, st[b].iterations + 1);
         }
     }
+    float best = 1e30f;
+    auto time_solve = [&](float &ms, int &flag) {
+        for (int rep = 0; e == cudaSuccess && rep < 2; ++rep) {
+            e = cudaMemcpyAsync(p->vv.dx, dx0, bytes, cudaMemcpyDeviceToDevice, s);
+            if (e == cudaSuccess) e = cudaEventRecord(e0, s);
+            if (e == cudaSuccess) e = global_solve(p, 0, s);
+            if (e == cudaSuccess) e = cudaEventRecord(e1, s);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+        }
+        if (e == cudaSuccess) e = cudaMemcpy(&flag, p->pw.error, sizeof(int), cudaMemcpyDeviceToHost);
+    };
+    // the resident clusters first, where the bodies have them; the schedules
+    // of the global-memory PCG against them
+    bool resident = !p->body_classes.empty();
+    if (resident) {
+        float ms = 0.0f;
+        int flag = 0;
+        p->bodies_resident = true;
+        time_solve(ms, flag);
+        if (e == cudaSuccess && flag) {
+            e = rearm_barriers(p);
+            resident = false;
+        } else {
+            best = ms;
+        }
+        p->bodies_resident = false;
+    }
     const int threads_opts[3] = {128, 256, 512};
     const double c0_opts[3] = {512.0, 2048.0, 8192.0};
     int sms = 1;
@@ -1848,7 +2003,6 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
     const int n_caps = p->bw.n_bodies == 1 ? 5 : 1;
     int best_t = p->bw.threads, best_g = p->bw_max_group;
     double best_m = p->bw_c0;
-    float best = 1e30f;
     std::vector<std::vector<int4>> tried;
     for (int cand = 0; e == cudaSuccess && cand < 3 * 3 * n_caps; ++cand) {
         const int threads = threads_opts[cand / (3 * n_caps)], cap = group_opts[cand % n_caps];
@@ -1879,15 +2033,7 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
         }
         float ms = 0.0f;
         int flag = 0;
-        for (int rep = 0; e == cudaSuccess && rep < 2; ++rep) {
-            e = cudaMemcpyAsync(p->vv.dx, dx0, bytes, cudaMemcpyDeviceToDevice, s);
-            if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-            if (e == cudaSuccess) e = global_solve(p, 0, s);
-            if (e == cudaSuccess) e = cudaEventRecord(e1, s);
-            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        }
-        if (e == cudaSuccess) e = cudaMemcpy(&flag, p->pw.error, sizeof(int), cudaMemcpyDeviceToHost);
+        time_solve(ms, flag);
         if (e == cudaSuccess && flag) {
             // a wait gave up: this schedule is not a candidate
             e = rearm_barriers(p);
@@ -1898,12 +2044,14 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
             best_t = threads;
             best_m = c0;
             best_g = cap;
+            resident = false;
         }
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (x) cudaFree(x);
     if (dx0) cudaFree(dx0);
+    p->bodies_resident = resident;
     if (e != cudaSuccess) return cuda_fail(p, e, "autotune");
     drop_graphs(p);
     const int rc = apply_batch_layout(p, best_t, best_m, best_g);

@@ -327,7 +327,10 @@ struct ResidentHost {
     int slice_trips_max = 0;
 };
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                       int row_lo, int row_hi, int parts, int body, bool push_lists);
+                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel = true);
+// The same for several bodies of `parts` parts each, the bodies in parallel.
+void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
+                         const int32_t *row_off, const std::vector<int> &bodies, int parts);
 
 struct ResidentViews {
     const ResPart *parts;

@@ -95,9 +95,8 @@ struct Bisector {
 
     // Splits the rows into `parts` runs of nearly equal length, level by
     // level; bounds[p], bounds[p + 1] are run p's.
-    void split(std::vector<int> &rows, int parts, std::vector<int> &bounds) const {
+    void split(std::vector<int> &rows, int parts, std::vector<int> &bounds, int threads) const {
         std::vector<Run> runs{Run{0, (int)rows.size(), parts, 0}}, next;
-        const int threads = thread_count((int)rows.size());
         while (!runs.empty()) {
             next.assign(2 * runs.size(), Run{0, 0, 1, -1});
             parallel_for((int)runs.size(), threads, [&](int i) {
@@ -122,13 +121,13 @@ struct PartArrays {
 }  // namespace
 
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                       int row_lo, int row_hi, int parts, int body, bool push_lists) {
+                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel) {
     const int n = row_hi - row_lo;
     const int first_part = (int)h.parts.size();
+    const int threads = parallel ? thread_count(n) : 1;
     std::vector<int> rows(n), bounds(parts + 1, 0);
     for (int i = 0; i < n; ++i) rows[i] = row_lo + i;
-    Bisector{rest_q}.split(rows, parts, bounds);
-    const int threads = thread_count(n);
+    Bisector{rest_q}.split(rows, parts, bounds, threads);
     std::vector<int> part_of(n), local(n);
     parallel_for(parts, threads, [&](int p) {
         // rows of like length share a slice, so slices carry little padding;
@@ -250,6 +249,41 @@ void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *c
                        e % kPartLanes * kPartSliceRows + (i - lo) % kPartSliceRows] = dst[e];
         }
         h.push_max = std::max(h.push_max, rp.push_passes * rp.nslices * 32);
+    }
+}
+
+void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
+                         const int32_t *row_off, const std::vector<int> &bodies, int parts) {
+    std::vector<ResidentHost> made(bodies.size());
+    int rows = 0;
+    for (int b : bodies) rows += row_off[b + 1] - row_off[b];
+    parallel_for((int)bodies.size(), thread_count(rows), [&](int i) {
+        const int b = bodies[i];
+        resident_add_body(made[i], row_ptr, col_idx, rest_q, row_off[b], row_off[b + 1], parts, b, parts > 1, false);
+    });
+    for (const ResidentHost &m : made) {
+        const int first = (int)h.parts.size(), trips = (int)(h.src.size() / 32);
+        for (ResPart rp : m.parts) {
+            rp.row_off += (int)h.rows.size();
+            rp.halo_off += (int)h.halo.size();
+            rp.slice_off += (int)h.trip_ptr.size();
+            rp.push_off += (int)h.push.size();
+            h.parts.push_back(rp);
+        }
+        for (int4 t : m.tasks) h.tasks.push_back(make_int4(first + t.x, t.y, t.z, t.w));
+        h.rows.insert(h.rows.end(), m.rows.begin(), m.rows.end());
+        h.halo.insert(h.halo.end(), m.halo.begin(), m.halo.end());
+        for (int32_t t : m.trip_ptr) h.trip_ptr.push_back(trips + t);
+        h.src.insert(h.src.end(), m.src.begin(), m.src.end());
+        h.col.insert(h.col.end(), m.col.begin(), m.col.end());
+        h.push.insert(h.push.end(), m.push.begin(), m.push.end());
+        h.nown_max = std::max(h.nown_max, m.nown_max);
+        h.nhalo_max = std::max(h.nhalo_max, m.nhalo_max);
+        h.nlocal_max = std::max(h.nlocal_max, m.nlocal_max);
+        h.push_max = std::max(h.push_max, m.push_max);
+        h.trips_max = std::max(h.trips_max, m.trips_max);
+        h.trips_max_reg = std::max(h.trips_max_reg, m.trips_max_reg);
+        h.slice_trips_max = std::max(h.slice_trips_max, m.slice_trips_max);
     }
 }
 

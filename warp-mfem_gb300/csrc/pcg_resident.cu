@@ -693,9 +693,9 @@ ResKernel pick_form(const ResidentLayout &L) {
                                   : pcg_resident_kernel<kGrid, 1, 4, 0, STREAM>;
     }
     if (L.cluster <= 1) return pcg_resident_kernel<kOne, 1, 1, KR, STREAM>;
-    return L.row_slots <= 1   ? pcg_resident_kernel<kCluster, 1, 1, KR, STREAM>
-           : L.row_slots <= 2 ? pcg_resident_kernel<kCluster, 1, 2, KR, STREAM>
-                              : pcg_resident_kernel<kCluster, 2, 4, 0, STREAM>;
+    if (L.own_slots == 2) return pcg_resident_kernel<kCluster, 2, 4, 0, STREAM>;
+    return L.row_slots <= 1 ? pcg_resident_kernel<kCluster, 1, 1, KR, STREAM>
+                            : pcg_resident_kernel<kCluster, 1, 2, KR, STREAM>;
 }
 
 ResKernel pick(const ResidentLayout &L) { return L.stream_trips > 0 ? pick_form<true>(L) : pick_form<false>(L); }
