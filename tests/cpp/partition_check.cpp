@@ -77,6 +77,19 @@ int main() {
             both.parts.erase(both.parts.begin(), both.parts.begin() + parts);
             both.tasks.erase(both.tasks.begin());
             h = both;
+        } else if (trial % 4 == 1 && lo == 0 && n >= 3 * parts) {
+            // runs of whole blocks of consecutive rows
+            const int blocks = parts + below(2 * parts);
+            resident_add_ranges(h, rp.data(), ci.data(), n, parts, blocks, true);
+            for (int p = 0, b = 0; p < parts; ++p) {
+                const ResPart &P = h.parts[p];
+                CHECK(P.block_lo == b && P.nblocks >= 1 && P.nblocks <= h.block_max);
+                b += P.nblocks;
+                CHECK(P.row_off == (int)((long long)n * P.block_lo / blocks));
+                CHECK(P.row_off + P.nown == (int)((long long)n * b / blocks));
+                for (int i = 0; i < P.nown; ++i)
+                    CHECK(h.rows[P.row_off + i] >= P.row_off && h.rows[P.row_off + i] < P.row_off + P.nown);
+            }
         } else {
             resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true);
         }
@@ -133,7 +146,7 @@ int main() {
                 CHECK((int)blocks[i].size() == rp[row + 1] - rp[row]);
             }
         }
-        CHECK(most - least <= 2);
+        CHECK(h.blocks > 0 || most - least <= 2);
         for (int v : seen) CHECK(v == 1);
         for (int p = 0; p < parts; ++p)
             for (int i = 0; i < h.parts[p].nhalo; ++i) CHECK(sender[p][i] == h.halo[h.parts[p].halo_off + i]);

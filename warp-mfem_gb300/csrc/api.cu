@@ -130,6 +130,8 @@ namespace {
 // Rows a CTA up to which one cluster beats a grid: 16 CTAs of 370 rows 3.0 us
 // an iteration.
 constexpr int kClusterRows = 400;
+// Rows up to which every solve of one mesh adds its sums in the ordered way.
+constexpr int kOrderedRows = 384;
 
 struct DeviceGuard {
     int prev = -1;
@@ -463,24 +465,38 @@ cudaError_t alloc_stream(std::vector<void *> &allocs, size_t parts, ResidentLayo
 }
 
 // The resident PCG of one mesh: a cluster, or past what 16 CTAs hold on the
-// chip a grid of one CTA an SM.  A part takes at most 128 rows, one slice a
-// warp, while the cluster may grow: an iteration takes 1.0 us on one CTA and
-// 1.43 us in clusters of 4 to 16 (99 to 1,225 rows), a further slice a warp
-// 0.45 us.
+// chip a grid.  A part takes at most 128 rows, one slice a warp, while the
+// cluster may grow: an iteration takes 1.1 us on one CTA and 1.5 us in
+// clusters of 4 to 16 (99 to 1,225 rows), a further slice a warp 0.45 us.
+//
+// With ordered sums (the iterates of the windowed single-reduction kernel, bit
+// for bit) where a step's result turns on the PCG's rounding: under the line
+// search, whose decisions late in a step follow the last bits, and on small
+// meshes (two orders of the sums move the velocities of a step by 2e-5 at 96
+// vertices, 7e-6 at 330, 1e-6 at 2,673).  That costs 0.25 us an iteration on
+// one CTA, 0.3 in a cluster and 0.25 on a grid, and needs row ranges with
+// short halos: banded orders, or at most 1,024 rows.  Else, and where that
+// does not fit, on parts bisected by position.
 cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q, int max_ctas) {
     constexpr int kRows = kPartWarps * kPartSliceRows;
-    for (int form = 0; form < 2; ++form) {
-        const bool grid = form == 1;
+    const bool windowed = p->pl.variant == PcgLayout::kSingleReduction && p->pl.cache_matrix;
+    const bool rounding = p->cfg.line_search || p->n <= kOrderedRows;
+    for (int form = windowed && rounding ? 0 : 2; form < 4; ++form) {
+        const bool ordered = form < 2, grid = form & 1;
+        const int blocks = p->pcg_ctas;
         int parts = 1;
         if (grid) {
-            parts = std::min(std::min(max_ctas, kPartMaxGrid), (p->n + kRows - 1) / kRows);
+            parts = ordered ? blocks : std::min(std::min(max_ctas, kPartMaxGrid), (p->n + kRows - 1) / kRows);
         } else {
-            while (parts < kPartMaxCluster && parts * kRows < p->n) parts *= 2;
             if (p->n > kPartMaxCluster * kClusterRows) continue;
+            if (ordered) parts = std::min(kPartMaxCluster, (blocks + 1) / 2);
+            else
+                while (parts < kPartMaxCluster && parts * kRows < p->n) parts *= 2;
         }
         if (p->n > parts * 2 * kPartThreads) return cudaSuccess;
         ResidentHost h;
-        resident_add_body(h, sym.row_ptr.data(), sym.col_idx.data(), rest_q, 0, p->n, parts, 0, !grid);
+        if (ordered) resident_add_ranges(h, sym.row_ptr.data(), sym.col_idx.data(), p->n, parts, blocks, !grid);
+        else resident_add_body(h, sym.row_ptr.data(), sym.col_idx.data(), rest_q, 0, p->n, parts, 0, !grid);
         bool fits = false;
         ResidentLayout L;
         cudaError_t e = resident_layout(p->device, h, parts, grid, L, fits);

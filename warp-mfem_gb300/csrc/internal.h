@@ -305,6 +305,7 @@ constexpr int kPartWarps = 16;
 constexpr int kPartThreads = 32 * kPartWarps;
 constexpr int kPartMaxCluster = 16;
 constexpr int kPartMaxGrid = 256;
+constexpr int kPartMaxBlocks = 8;  // of a part, with ordered sums
 constexpr int kPartRegTrips = 4;    // trips of a warp's first slice whose blocks stay in registers
 
 struct ResPart {
@@ -312,6 +313,7 @@ struct ResPart {
     int halo_off, nhalo;     // rows of other parts that the own rows' columns reach
     int slice_off, nslices;  // trip_ptr[slice_off + s]: first trip of slice s
     int push_off, push_passes;  // push[push_off + (pass * nslices + slice) * 32 + lane]
+    int block_lo, nblocks;   // the sums' blocks of rows that the part holds (ordered sums), else 0
 };
 
 // The parts of a plan's bodies as the host builds them (partition.cpp).
@@ -325,9 +327,15 @@ struct ResidentHost {
     int nown_max = 0, nhalo_max = 0, nlocal_max = 0, push_max = 0;
     int trips_max = 0, trips_max_reg = 0;  // most trips of a warp, in all and without its register trips
     int slice_trips_max = 0;
+    int blocks = 0;         // ordered sums: blocks of the body, row n v / blocks on in block v
+    int block_max = 0;      // most blocks of a part
 };
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
                        int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel = true);
+// The same with the parts runs of `blocks` equal ranges of consecutive rows: for
+// the resident PCG's ordered sums.
+void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
+                         bool push_lists);
 // The same for several bodies of `parts` parts each, the bodies in parallel.
 void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
                          const int32_t *row_off, const std::vector<int> &bodies, int parts);
@@ -345,9 +353,11 @@ struct ResidentLayout {
     int cluster = 0;       // parts of a body; 0: the plan has no resident layout
     bool grid = false;     // the parts meet in global memory (a cooperative grid), else in a cluster
     int own_slots = 1, row_slots = 1;  // own rows, and rows in all, that a thread keeps
-    int nown_max = 0, nhalo_max = 0;
+    int nown_max = 0, nhalo_max = 0, push_max = 0;
     int smem_trips = 0;    // trips a warp keeps in shared memory
     int stream_trips = 0;  // trips a warp streams from global memory
+    int blocks = 0;        // ordered sums over so many blocks of rows; 0: sums over the parts
+    int block_max = 0;
     size_t smem = 0;       // dynamic shared memory per CTA
     ResidentViews v{};
 };

@@ -111,6 +111,10 @@ struct Bisector {
     }
 };
 
+// Adds the parts rows[bounds[p] .. bounds[p + 1]) of one body.
+void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int row_lo, int body,
+               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads);
+
 // One part's arrays before they are joined.
 struct PartArrays {
     std::vector<int32_t> halo, trip_ptr, src;
@@ -123,11 +127,35 @@ struct PartArrays {
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
                        int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel) {
     const int n = row_hi - row_lo;
-    const int first_part = (int)h.parts.size();
     const int threads = parallel ? thread_count(n) : 1;
     std::vector<int> rows(n), bounds(parts + 1, 0);
     for (int i = 0; i < n; ++i) rows[i] = row_lo + i;
     Bisector{rest_q}.split(rows, parts, bounds, threads);
+    add_parts(h, row_ptr, col_idx, row_lo, body, rows, bounds, push_lists, threads);
+}
+
+void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
+                         bool push_lists) {
+    std::vector<int> rows(n), bounds(parts + 1, 0);
+    for (int i = 0; i < n; ++i) rows[i] = i;
+    const int first_part = (int)h.parts.size();
+    for (int p = 1; p <= parts; ++p) bounds[p] = (int)((int64_t)n * ((int64_t)blocks * p / parts) / blocks);
+    add_parts(h, row_ptr, col_idx, 0, 0, rows, bounds, push_lists, thread_count(n));
+    h.blocks = blocks;
+    for (int p = 0; p < parts; ++p) {
+        ResPart &rp = h.parts[first_part + p];
+        rp.block_lo = (int)((int64_t)blocks * p / parts);
+        rp.nblocks = (int)((int64_t)blocks * (p + 1) / parts) - rp.block_lo;
+        h.block_max = std::max(h.block_max, rp.nblocks);
+    }
+}
+
+namespace {
+
+void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int row_lo, int body,
+               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads) {
+    const int n = (int)rows.size(), parts = (int)bounds.size() - 1;
+    const int first_part = (int)h.parts.size();
     std::vector<int> part_of(n), local(n);
     parallel_for(parts, threads, [&](int p) {
         // rows of like length share a slice, so slices carry little padding;
@@ -251,6 +279,8 @@ void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *c
         h.push_max = std::max(h.push_max, rp.push_passes * rp.nslices * 32);
     }
 }
+
+}  // namespace
 
 void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
                          const int32_t *row_off, const std::vector<int> &bodies, int parts) {

@@ -71,7 +71,8 @@ struct ResArgs {
     int slot, bodies;
     float tol;
     int maxiter, use_precond;
-    int nown_max, nhalo_max, smem_trips, stream_trips;
+    int nown_max, nhalo_max, smem_trips, stream_trips, push_max;
+    int blocks, block_warps;  // ordered sums: blocks of the body, warps of the longest one
     // kGrid: published rows [2][n], partial sums [2][CTAs], barrier arrivals
     float4 *pub, *partials;
     unsigned long long *counter;
@@ -144,17 +145,25 @@ __device__ __forceinline__ void block_mac(const float h[9], const float4 v, floa
     a[2] += h[6] * v.x + h[7] * v.y + h[8] * v.z;
 }
 
-// The warp's sums of v[0..2]: lanes 8g .. 8g + 7 return the sum of v[min(g, 2)].
-// Each exchange halves what a lane carries, so three sums take six shuffles
-// (a block's 16 warps otherwise spend most of a reduction issuing shuffles).
+// The warp's sums of v[0..2], each added in the order of a shuffle-down tree
+// (lane i takes lane i + 16, then + 8, ...): lanes 0, 16 and 8 return the sums
+// of v[0], v[1] and v[2].  Each exchange halves what a lane carries, so three
+// sums take six shuffles (a block's 16 warps otherwise spend most of a
+// reduction issuing shuffles).
 __device__ __forceinline__ float warp_sum3(const float v[3], int lane) {
-    const bool b0 = lane & 8, b1 = lane & 16;
-    float k0 = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 8);
-    float k1 = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 8);
-    float k = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 16);
+    const bool b0 = lane & 16, b1 = lane & 8;
+    float k0 = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 16);
+    float k1 = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
+    float k = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 8);
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(0xffffffffu, k, off);
     return k;
+}
+
+__device__ __forceinline__ void spread_sum3(float k, float sum[3]) {
+    sum[0] = __shfl_sync(0xffffffffu, k, 0);
+    sum[1] = __shfl_sync(0xffffffffu, k, 16);
+    sum[2] = __shfl_sync(0xffffffffu, k, 8);
 }
 
 // Adds two values a lane over lanes 8g .. 8g + 7 and hands group g's sum to
@@ -176,11 +185,20 @@ struct Verdict {
 // OS: own rows a thread keeps, RS: rows it keeps in all (the further ones
 // halo rows), KR: trips of a warp's first slice kept in registers, STREAM: some
 // trips do not fit in shared memory.
-template <Scope SCOPE, int OS, int RS, int KR, bool STREAM>
+//
+// ORDERED: the sums are added over the same blocks of consecutive rows, in the
+// same order, whatever CTAs the rows sit on, and the scalars are formed as in
+// the windowed single-reduction kernel (pcg.cu, which sums each CTA's range of
+// rows): such a solve has that kernel's iterates bit for bit.  A part is then a
+// run of whole blocks.
+template <Scope SCOPE, int OS, int RS, int KR, bool STREAM, bool ORDERED>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float s_red[3][kPartWarps];
-    __shared__ __align__(16) float4 s_part[2][kPartMaxCluster];
+    constexpr int kBlocks = ORDERED && SCOPE != kGrid ? kPartMaxBlocks : 1;
+    constexpr int kSums = SCOPE == kCluster ? kPartMaxCluster * kBlocks : 1;  // partial sums of a round
+    __shared__ float s_red[kBlocks][3][kPartWarps];
+    __shared__ __align__(16) float4 s_part[2][kSums];
+
     __shared__ __align__(8) uint64_t s_mbar[2];
     __shared__ __align__(16) Verdict s_verdict;
     __shared__ float s_norm[2];
@@ -190,6 +208,9 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     float4 *trips_s = halo_w + (SCOPE == kCluster ? 2 * a.nhalo_max : 0);   // [warps][smem_trips][80]
     float *minv_s = reinterpret_cast<float *>(trips_s + (size_t)kPartWarps * a.smem_trips * kTripFloats4);
     int *push_s = reinterpret_cast<int *>(minv_s + (RS > 1 ? 9 * (a.nown_max + a.nhalo_max) : 0));
+    // ORDERED: r, u and w of the own rows, component by component
+    float *const own_r = reinterpret_cast<float *>(push_s + a.push_max), *const own_u = own_r + 3 * a.nown_max,
+                 *const own_w = own_u + 3 * a.nown_max;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool inner = a.ir_state != nullptr;
@@ -219,7 +240,28 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         }
     }
     if (SCOPE == kGrid && warp == 0) target = grid_count(a.counter) / ncta * ncta;
-    if (SCOPE == kCluster && tid < 2 * kPartMaxCluster) s_part[0][tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = tid; SCOPE == kCluster && i < 2 * kSums; i += kPartThreads)
+        s_part[i / kSums][i % kSums] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (ORDERED) {
+        for (int i = tid; i < kBlocks * 3 * kPartWarps; i += kPartThreads)
+            s_red[i / (3 * kPartWarps)][i / kPartWarps % 3][i % kPartWarps] = 0.0f;
+    }
+    // ORDERED: the part's first row, and per task of this warp (32 consecutive
+    // components of a block) the lane's component, the block's end and where
+    // the sum goes; -1: no task
+    constexpr int kTasks = SCOPE == kOne ? 1 : SCOPE == kGrid ? 1 : 3;
+    int row0 = 0, task_i[kTasks], task_end[kTasks], task_dst[kTasks];
+    if (ORDERED) {
+        auto block_row = [&](int b) { return (int)((long long)a.n * (part.block_lo + b) / a.blocks); };
+        row0 = block_row(0);
+#pragma unroll
+        for (int q = 0; q < kTasks; ++q) {
+            const int t = warp + kPartWarps * q, b = t / a.block_warps, wi = t - b * a.block_warps;
+            task_dst[q] = b < part.nblocks ? b * 3 * kPartWarps + wi : -1;
+            task_i[q] = 3 * (block_row(b) - row0) + 32 * wi + lane;
+            task_end[q] = b < part.nblocks ? 3 * (block_row(b + 1) - row0) : 0;
+        }
+    }
     __syncthreads();
     int err = s_err;
     if (SCOPE == kCluster) {
@@ -400,6 +442,10 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         if (lane < 8) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) w[0][c] = acc[c];
+            if (ORDERED && own[0]) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) own_w[3 * (row_id[0] - row0) + c] = acc[c];
+            }
         }
         if (more_trips == 0) return;
 #pragma unroll
@@ -418,6 +464,10 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 if ((lane >> 3) == qq) {
 #pragma unroll
                     for (int c = 0; c < 3; ++c) w[o][c] = acc[c];
+                    if (ORDERED && own[o]) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) own_w[3 * (row_id[o] - row0) + c] = acc[c];
+                    }
                 }
             }
     };
@@ -434,26 +484,64 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     // barrier hands them on; with the grid they go to halo_v.  CTA-uniform;
     // the verdict of a wait that gave up is a timeout.
     float halo_v[SCOPE == kGrid ? RS : 1][3];
-    auto exchange = [&](unsigned k, const float v[3], auto decide) -> Verdict {
+    auto exchange = [&](unsigned k, const float v[3], auto term, auto decide) -> Verdict {
         const int buf = k & 1;
-        const float part_sum = warp_sum3(v, lane);
-        if ((lane & 7) == 0 && lane < 24) s_red[lane >> 3][warp] = part_sum;
+        if (ORDERED) {
+            __syncthreads();  // own_r, own_u, own_w
+#pragma unroll
+            for (int q = 0; q < kTasks; ++q) {
+                if (task_dst[q] < 0) break;
+                float acc[3] = {0.0f, 0.0f, 0.0f};
+                if (task_i[q] < task_end[q]) term(task_i[q], acc);
+                if (SCOPE == kGrid)  // blocks of more than 170 rows
+                    for (int i = task_i[q] + kPartThreads; i < task_end[q]; i += kPartThreads) term(i, acc);
+                const float k3 = warp_sum3(acc, lane);
+                if ((lane & 7) == 0 && lane < 24)
+                    (&s_red[0][0][0])[task_dst[q] + kPartWarps * (lane == 0 ? 0 : lane == 16 ? 1 : 2)] = k3;
+            }
+        } else {
+            const float k3 = warp_sum3(v, lane);
+            if ((lane & 7) == 0 && lane < 24) s_red[0][lane == 0 ? 0 : lane == 16 ? 1 : 2][warp] = k3;
+        }
         __syncthreads();
         float sum[3];
         const int g = min(lane >> 3, 2), i = lane & 7;
         bool ok = true;
+        if (SCOPE == kCluster && tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_mbar[buf])),
+                         "r"(16u * (uint32_t)((ORDERED ? a.blocks : ncta) + part.nhalo))
+                         : "memory");
+        if (warp < (ORDERED ? part.nblocks : 1)) {
+            // a block's sum, by a warp of its own
+            const int b = ORDERED ? warp : 0;
+            group_sum3(s_red[b][g][i] + s_red[b][g][i + 8], sum);
+            if (SCOPE == kCluster && lane < ncta)
+                push16(&s_part[buf][ORDERED ? part.block_lo + b : rank], &s_mbar[buf], lane, sum[0], sum[1], sum[2]);
+        }
         if (warp == 0) {
-            group_sum3(s_red[g][i] + s_red[g][i + 8], sum);
+            if (SCOPE == kOne && ORDERED && part.nblocks > 1) {
+                float second[3];
+                group_sum3(s_red[kBlocks > 1 ? 1 : 0][g][i] + s_red[kBlocks > 1 ? 1 : 0][g][i + 8], second);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) sum[c] += second[c];
+            }
             if (SCOPE == kCluster) {
-                if (lane == 0)
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                                     smem_addr(&s_mbar[buf])),
-                                 "r"(16u * (uint32_t)(ncta + part.nhalo))
-                                 : "memory");
-                if (lane < ncta) push16(&s_part[buf][rank], &s_mbar[buf], lane, sum[0], sum[1], sum[2]);
                 ok = __all_sync(0xffffffffu, wait_phase(&s_mbar[buf], (k >> 1) & 1u));
-                const float *t = reinterpret_cast<const float *>(s_part[buf]) + g;
-                group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
+                if (ORDERED) {
+                    float t[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int b = 0; b < kSums; b += 32)  // zero past the last block
+                        if (b < a.blocks) {
+                            const float4 q = s_part[buf][b + lane < kSums ? b + lane : 0];
+                            t[0] += q.x;
+                            t[1] += q.y;
+                            t[2] += q.z;
+                        }
+                    spread_sum3(warp_sum3(t, lane), sum);
+                } else {
+                    const float *t = reinterpret_cast<const float *>(s_part[buf]) + g;
+                    group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
+                }
             }
             if (SCOPE == kGrid) {
                 target += ncta;
@@ -495,9 +583,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                     t[1] += q.y;
                     t[2] += q.z;
                 }
-                const float tot = warp_sum3(t, lane);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) sum[c] = __shfl_sync(0xffffffffu, tot, 8 * c);
+                spread_sum3(warp_sum3(t, lane), sum);
             }
         }
         if (warp == 0 && lane == 0) {
@@ -554,11 +640,19 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
             if (j < OS) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) u[j < OS ? j : 0][c] = z[c];
+                if (ORDERED && own[j < OS ? j : 0]) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        own_r[3 * (row_id[j] - row0) + c] = r[j][c];
+                        own_u[3 * (row_id[j] - row0) + c] = z[c];
+                    }
+                }
             }
         }
     };
     // partial sums of gamma, delta and (r, r) over the own rows
     auto dots = [&](float (&sum)[3]) {
+        if (ORDERED) return;
         sum[0] = sum[1] = sum[2] = 0.0f;
 #pragma unroll
         for (int o = 0; o < OS; ++o)
@@ -570,6 +664,13 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                     sum[2] = __fmaf_rn(r[o][c], r[o][c], sum[2]);
                 }
             }
+    };
+
+    auto term = [&](int i, float acc[3]) {  // ORDERED: the same of component i
+        const float rc = own_r[i], uc = own_u[i];
+        acc[0] = __fmaf_rn(rc, uc, acc[0]);
+        acc[1] = __fmaf_rn(own_w[i], uc, acc[1]);
+        acc[2] = __fmaf_rn(rc, rc, acc[2]);
     };
 
     // ---- r0 = g - H x0 (x0 = 0 for an inner solve), exchanged in round 0
@@ -592,13 +693,15 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
             for (int c = 0; c < 3; ++c) {
                 const float g = __ldg(a.b + (size_t)3 * row_id[o] + c) * bscale;
                 sum[0] = __fmaf_rn(g, g, sum[0]);
+                if (ORDERED) own_r[3 * (row_id[o] - row0) + c] = g;
             }
         }
     // the recurrence's scalars, kept by thread 0 (||g||^2 and (r, r) in s_norm)
     float thr2 = 0.0f, gamma = 0.0f, alpha = 0.0f;
     int it = 0;
     unsigned round = 0;
-    Verdict d = exchange(round, sum, [&](const float t[3]) {
+    auto rhs_term = [&](int i, float acc[3]) { acc[0] = __fmaf_rn(own_r[i], own_r[i], acc[0]); };
+    Verdict d = exchange(round, sum, rhs_term, [&](const float t[3]) {
         s_norm[0] = t[0];
         s_norm[1] = 0.0f;
         thr2 = a.tol * a.tol * t[0];
@@ -614,7 +717,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         product(false, push_w);
         if (SCOPE == kGrid) publish(round + 1);
         dots(sum);
-        d = exchange(++round, sum, [&](const float t[3]) {
+        d = exchange(++round, sum, term, [&](const float t[3]) {
             gamma = t[0];
             const float rr = t[2];
             s_norm[1] = rr;
@@ -636,14 +739,14 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
             if (SCOPE == kGrid) publish(round + 1);
             dots(sum);
             ++it;
-            d = exchange(++round, sum, [&](const float t[3]) {
+            d = exchange(++round, sum, term, [&](const float t[3]) {
                 const float rr = t[2];
                 s_norm[1] = rr;
                 if (!isfinite(t[0]) || !isfinite(t[1]) || !isfinite(rr)) return Verdict{0.0f, 0.0f, 1, MFEM_NONFINITE};
                 if (rr <= thr2) return Verdict{0.0f, 0.0f, 1, MFEM_OK};
-                const float ga = t[0] / alpha;  // in flight with beta
                 const float beta = t[0] / gamma;
-                const float denom = t[1] - beta * ga;
+                // the ratio in flight with beta, or in the windowed kernel's order
+                const float denom = ORDERED ? t[1] - beta * t[0] / alpha : t[1] - beta * (t[0] / alpha);
                 if (!(denom > 0.0f)) return Verdict{0.0f, 0.0f, 1, MFEM_STAGNATION};
                 alpha = t[0] / denom;
                 gamma = t[0];
@@ -686,19 +789,32 @@ ResKernel pick_form(const ResidentLayout &L) {
     constexpr int KR = kPartRegTrips;
     if (L.grid) {
         if (L.own_slots == 2)
-            return L.row_slots <= 3 ? pcg_resident_kernel<kGrid, 2, 3, 0, STREAM>
-                                    : pcg_resident_kernel<kGrid, 2, 4, 0, STREAM>;
-        return L.row_slots <= 1   ? pcg_resident_kernel<kGrid, 1, 1, KR, STREAM>
-               : L.row_slots <= 2 ? pcg_resident_kernel<kGrid, 1, 2, KR, STREAM>
-                                  : pcg_resident_kernel<kGrid, 1, 4, 0, STREAM>;
+            return L.row_slots <= 3 ? pcg_resident_kernel<kGrid, 2, 3, 0, STREAM, false>
+                                    : pcg_resident_kernel<kGrid, 2, 4, 0, STREAM, false>;
+        return L.row_slots <= 1   ? pcg_resident_kernel<kGrid, 1, 1, KR, STREAM, false>
+               : L.row_slots <= 2 ? pcg_resident_kernel<kGrid, 1, 2, KR, STREAM, false>
+                                  : pcg_resident_kernel<kGrid, 1, 4, 0, STREAM, false>;
     }
-    if (L.cluster <= 1) return pcg_resident_kernel<kOne, 1, 1, KR, STREAM>;
-    if (L.own_slots == 2) return pcg_resident_kernel<kCluster, 2, 4, 0, STREAM>;
-    return L.row_slots <= 1 ? pcg_resident_kernel<kCluster, 1, 1, KR, STREAM>
-                            : pcg_resident_kernel<kCluster, 1, 2, KR, STREAM>;
+    if (L.cluster <= 1) return pcg_resident_kernel<kOne, 1, 1, KR, STREAM, false>;
+    if (L.own_slots == 2) return pcg_resident_kernel<kCluster, 2, 4, 0, STREAM, false>;
+    return L.row_slots <= 1 ? pcg_resident_kernel<kCluster, 1, 1, KR, STREAM, false>
+                            : pcg_resident_kernel<kCluster, 1, 2, KR, STREAM, false>;
 }
 
-ResKernel pick(const ResidentLayout &L) { return L.stream_trips > 0 ? pick_form<true>(L) : pick_form<false>(L); }
+ResKernel pick_ordered(const ResidentLayout &L) {
+    constexpr int KR = kPartRegTrips;
+    if (L.grid)
+        return L.row_slots <= 1 ? pcg_resident_kernel<kGrid, 1, 1, KR, false, true>
+                                : pcg_resident_kernel<kGrid, 1, 2, KR, false, true>;
+    if (L.cluster <= 1) return pcg_resident_kernel<kOne, 1, 1, KR, false, true>;
+    return L.row_slots <= 1 ? pcg_resident_kernel<kCluster, 1, 1, KR, false, true>
+                            : pcg_resident_kernel<kCluster, 1, 2, KR, false, true>;
+}
+
+ResKernel pick(const ResidentLayout &L) {
+    if (L.blocks > 0) return pick_ordered(L);
+    return L.stream_trips > 0 ? pick_form<true>(L) : pick_form<false>(L);
+}
 
 // Launch configuration of n_tasks bodies; attr holds two attributes.
 cudaLaunchConfig_t launch_config(const ResidentLayout &L, int n_tasks, cudaLaunchAttribute attr[1], cudaStream_t s) {
@@ -737,7 +853,14 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     L.row_slots = std::max(1, (h.nlocal_max + kPartThreads - 1) / kPartThreads);
     if (L.own_slots > 2 || L.row_slots > 4 || h.slice_trips_max > 255) return cudaSuccess;
     if (!grid && cluster <= 1 && (L.own_slots > 1 || L.row_slots > 1)) return cudaSuccess;
-    if (!grid && L.row_slots > 2) L.own_slots = 2;  // the cluster form with more than two rows a thread
+    L.blocks = h.blocks;
+    L.block_max = h.block_max;
+    if (L.blocks > 0) {
+        // ordered sums: one own row and at most two rows a thread, nothing streamed
+        if (L.own_slots > 1 || L.row_slots > 2 || L.block_max > (grid ? 1 : kPartMaxBlocks)) return cudaSuccess;
+    } else if (!grid && L.row_slots > 2) {
+        L.own_slots = 2;  // the cluster form with more than two rows a thread
+    }
     cudaFuncAttributes fa;
     e = cudaFuncGetAttributes(&fa, pick(L));
     if (e != cudaSuccess) return e;
@@ -746,13 +869,15 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     const size_t most = (size_t)optin - fa.sharedSizeBytes;
     const size_t base = sizeof(float4) * ((size_t)h.nown_max + (!grid && cluster > 1 ? 3 : 1) * (size_t)h.nhalo_max) +
                         (L.row_slots > 1 ? 9 * sizeof(float) * ((size_t)h.nown_max + h.nhalo_max) : 0) +
-                        (!grid && cluster > 1 ? sizeof(int) * (size_t)h.push_max : 0) + 16;
+                        (!grid && cluster > 1 ? sizeof(int) * (size_t)h.push_max : 0) +
+                        (L.blocks > 0 ? 9 * sizeof(float) * (size_t)h.nown_max : 0) + 16;
     const size_t per_trip = sizeof(float4) * kTripFloats4 * kPartWarps;
     if (base > most) return cudaSuccess;
     L.smem_trips = (int)std::min<size_t>(trips, (most - base) / per_trip);
     L.stream_trips = trips - L.smem_trips;
     L.smem = (base + per_trip * L.smem_trips + 15) & ~(size_t)15;
-    if (L.smem > most) return cudaSuccess;
+    if (L.smem > most || (L.blocks > 0 && L.stream_trips > 0)) return cudaSuccess;
+    L.push_max = !grid && cluster > 1 ? h.push_max : 0;
     const ResKernel k = pick(L);
     // the limit is the kernel's, not the plan's: every plan sets the same one
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
@@ -791,6 +916,10 @@ cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const Res
     a.nhalo_max = L.nhalo_max;
     a.smem_trips = L.smem_trips;
     a.stream_trips = L.stream_trips;
+    a.push_max = L.push_max;
+    a.blocks = L.blocks;
+    const int block_rows = L.blocks > 0 ? (bv.n + L.blocks - 1) / L.blocks : 0;
+    a.block_warps = std::min(kPartWarps, (3 * block_rows + 31) / 32);
     a.pub = reinterpret_cast<float4 *>(w.pub);
     a.partials = reinterpret_cast<float4 *>(w.partials);
     a.counter = w.res_counter;
