@@ -259,9 +259,11 @@ int mfem_plan_sizes(const mfem_plan *plan, int32_t *n_particles, int32_t *n_tets
  * runs the global-memory PCG of mfem_plan_set_bodies as a one-body batch: a
  * mesh too large for the shared-memory slices, pcg_variant 5, or bodies
  * set), CTAs, whether each CTA keeps its slice of H in shared
- * memory, and the dynamic shared memory per CTA.  Variant 2 with pcg_ctas 0
- * is the resident form: one CTA, one cluster of up to 16, or a grid, each CTA
- * holding a compact block of rows chosen from the rest positions.
+ * memory, and the dynamic shared memory per CTA.  With pcg_ctas 0 the plan
+ * runs the resident form where it fits, in place of variants 1 to 4 as its
+ * vertex order allows them: CTAs (one, a cluster of up to 16, or a grid) that
+ * each hold a compact block of rows chosen from the rest positions; the
+ * variant reported is then the one it replaces, the sizes are its own.
  * Diagnostics; no reference counterpart. */
 int mfem_plan_pcg_layout(const mfem_plan *plan, int32_t *variant, int32_t *ctas, int32_t *cache_matrix,
                          int64_t *smem_bytes);

@@ -68,11 +68,24 @@ int main() {
         }
         const int parts = trial % 5 == 0 ? 1 + below(13) : 1 << below(5);
         ResidentHost h;
+        // the lower and upper CSR of a factor preconditioner's form
+        std::vector<int32_t> lrow(n + lo + 1, 0), urow(n + lo + 1, 0), lcol, ucol;
+        for (int r = 0; r < n + lo; ++r) {
+            for (int k = rp[r]; k < rp[r + 1]; ++k) {
+                if (ci[k] <= r) lcol.push_back(ci[k]);
+                if (ci[k] >= r) ucol.push_back(ci[k]);
+            }
+            lrow[r + 1] = (int32_t)lcol.size();
+            urow[r + 1] = (int32_t)ucol.size();
+        }
+        const ResidentFactor form{2 + trial % 2, lrow.data(), urow.data(), trial % 3 != 1};
+        const ResidentFactor *factor = trial % 4 == 3 || trial % 4 == 2 ? &form : nullptr;
+        const bool redundant = factor && form.redundant;
         const int32_t off[3] = {0, lo, lo + n};
         if (trial % 4 == 2 && lo > 0) {
             // behind a body of single rows: joined arrays
             ResidentHost both;
-            resident_add_bodies(both, rp.data(), ci.data(), q.data(), off, {0, 1}, parts);
+            resident_add_bodies(both, rp.data(), ci.data(), q.data(), off, {0, 1}, parts, factor);
             CHECK((int)both.parts.size() == 2 * parts && both.tasks.size() == 2 && both.tasks[1].x == parts);
             both.parts.erase(both.parts.begin(), both.parts.begin() + parts);
             both.tasks.erase(both.tasks.begin());
@@ -91,7 +104,7 @@ int main() {
                     CHECK(h.rows[P.row_off + i] >= P.row_off && h.rows[P.row_off + i] < P.row_off + P.nown);
             }
         } else {
-            resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true);
+            resident_add_body(h, rp.data(), ci.data(), q.data(), lo, lo + n, parts, 0, true, true, factor);
         }
         CHECK((int)h.parts.size() == parts && h.tasks.size() == 1 && h.tasks[0].y == parts);
         std::vector<int> seen(n, 0);
@@ -132,13 +145,63 @@ int main() {
                         CHECK(r < P.nown);
                         const int row = h.rows[P.row_off + r];
                         CHECK(k >= rp[row] && k < rp[row + 1]);
-                        CHECK(c >= 0 && c < P.nown + P.nhalo);
+                        CHECK(c >= 0 && c < (redundant ? P.second_rows : P.nown + P.nhalo));
                         CHECK((c < P.nown ? h.rows[P.row_off + c] : h.halo[P.halo_off + c - P.nown]) == ci[k]);
                         blocks[r].insert(k);
                     }
             }
             for (int w = 0; w < kPartWarps; ++w)
                 CHECK(warp[w] <= h.trips_max && warp[w] - reg[w] <= h.trips_max_reg);
+            auto vertex = [&](int i) {
+                return i < P.nown ? h.rows[P.row_off + i] : h.halo[P.halo_off + i - P.nown];
+            };
+            for (int w = 0; factor && w < 2; ++w) {
+                // pass w's rows, each block once, its column among the rows
+                // that hold the pass's input
+                const bool lower = (w == 0) == (form.mode == 2);
+                const int rows = w == 0 ? P.first_rows : P.second_rows;
+                const int inputs = redundant && w == 1 ? P.first_rows : P.nown + P.nhalo;
+                CHECK(rows >= P.nown && rows <= P.nown + P.nhalo && (redundant || rows == P.nown));
+                CHECK(P.nfslices[w] == (rows + kFactorSliceRows - 1) / kFactorSliceRows);
+                std::vector<int> count(rows, 0);
+                for (int s = 0; s < P.nfslices[w]; ++s) {
+                    const int t0 = h.ftrip_ptr[P.fslice_off[w] + s], t1 = h.ftrip_ptr[P.fslice_off[w] + s + 1];
+                    CHECK(t1 > t0 && t1 - t0 <= h.slice_trips_max);
+                    for (int t = t0; t < t1; ++t)
+                        for (int lane = 0; lane < 32; ++lane) {
+                            const int k = h.fsrc[32 * t + lane], c = h.fcol[32 * t + lane];
+                            if (k < 0) continue;
+                            const int r = s * kFactorSliceRows + lane;
+                            CHECK(r < rows && c < inputs);
+                            const int row = vertex(r);
+                            const std::vector<int32_t> &ptr = lower ? lrow : urow, &cols = lower ? lcol : ucol;
+                            CHECK(k >= ptr[row] && k < ptr[row + 1] && cols[k] == vertex(c));
+                            ++count[r];
+                        }
+                }
+                for (int i = 0; i < rows; ++i)
+                    CHECK(count[i] == (lower ? lrow : urow)[vertex(i) + 1] - (lower ? lrow : urow)[vertex(i)]);
+                CHECK(h.ftrip_ptr[P.fslice_off[w] + P.nfslices[w]] - h.ftrip_ptr[P.fslice_off[w]] <=
+                      h.f_trips_max[w]);
+            }
+            // the passes' push table sends every row where the product's does
+            if (factor) {
+                const int fs = (P.nown + kFactorSliceRows - 1) / kFactorSliceRows;
+                std::vector<std::set<int>> a(P.nown), b(P.nown);
+                for (int s = 0; s < P.nslices; ++s)
+                    for (int e = 0; e < P.push_passes * 32; ++e) {
+                        const int lane = e % 32, d = h.push[P.push_off + (e / 32 * P.nslices + s) * 32 + lane];
+                        if (d >= 0) a[s * kPartSliceRows + lane % kPartSliceRows].insert(d);
+                    }
+                for (int s = 0; s < fs; ++s)
+                    for (int e = 0; e < P.fpush_passes * 32; ++e) {
+                        const int d = h.fpush[P.fpush_off + (e / 32 * fs + s) * 32 + e % 32];
+                        if (d < 0) continue;
+                        CHECK(s * kFactorSliceRows + e % 32 < P.nown);
+                        b[s * kFactorSliceRows + e % 32].insert(d);
+                    }
+                CHECK(a == b && P.fpush_passes * fs * 32 <= h.fpush_max);
+            }
             for (int i = 0; i < P.nown; ++i) {
                 const int row = h.rows[P.row_off + i];
                 CHECK(row >= lo && row < lo + n);

@@ -142,20 +142,24 @@ def test_set_bodies_rejects_bad_input():
     assert rc == _lib.MFEM_BAD_ARG and b"line_search" in solver._lib.mfem_plan_last_error(solver._plan)
 
 
-@pytest.mark.parametrize("cells", [[(3, 2, 2), (30, 14, 12), (7, 6, 5), (9, 4, 4)],
-                                   [(48, 12, 12), (40, 14, 14), (4, 2, 2)]],
-                         ids=["clusters_1_to_16", "two_rows_a_thread"])
-def test_resident_bodies_agree_with_the_global_memory_pcg(cells):
+@pytest.mark.parametrize("cells,kw", [([(3, 2, 2), (30, 14, 12), (7, 6, 5), (9, 4, 4)], {}),
+                                      ([(48, 12, 12), (40, 14, 14), (4, 2, 2)], {}),
+                                      ([(3, 2, 2), (26, 11, 11), (7, 6, 5), (9, 4, 4), (14, 9, 8)],
+                                       dict(preconditioner="fsai")),
+                                      ([(40, 12, 12), (6, 4, 4)], dict(preconditioner="learned"))],
+                         ids=["clusters_1_to_16", "two_rows_a_thread", "fsai", "learned_streamed"])
+def test_resident_bodies_agree_with_the_global_memory_pcg(cells, kw):
     """Bodies on clusters of every size in one batch, up to bodies past 16 x
-    512 rows, against the global-memory PCG: both converge to 1e-6, positions
-    agree to 1e-5 of the largest as between schedules."""
+    512 rows (16 x 256 with a factor), against the global-memory PCG: both
+    converge to 1e-6, positions agree to 1e-5 of the largest as between
+    schedules."""
     bodies = [beams.build_beam(beams.BeamSpec(name=f"b{i}", cells=c, extent=tuple(0.05 * k for k in c),
                                               energy="arap" if i % 2 else "neohookean", E=(1e4, 1e6), nu=0.4,
                                               seed=20 + i)) for i, c in enumerate(cells)]
     batch = beams.concatenate(bodies)
     outs = []
-    for kw in ({}, dict(pcg_variant="global_memory")):
-        bs = BatchedSolver(batch, device=DEV, **kw)
+    for extra in ({}, dict(pcg_variant="global_memory")):
+        bs = BatchedSolver(batch, device=DEV, **kw, **extra)
         q, stats = run(bs, 2)
         assert all((s["status"] == _lib.MFEM_OK).all() for s in stats)
         outs.append(q)

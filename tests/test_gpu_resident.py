@@ -52,8 +52,7 @@ def test_solve_agrees_with_the_standard_form(cells, order):
     mesh = beams.build_beam("nh_beam", cells=cells)
     if order == "shuffled":
         mesh = shuffled(mesh)
-    sa, xa, lay = solve(mesh)
-    assert lay["variant"] == "single_reduction"
+    sa, xa, _ = solve(mesh)
     sb, xb, lay_b = solve(mesh, pcg_variant="standard" if order == "grid" else "gather")
     assert lay_b["variant"] in ("standard", "gather")
     assert sa["status"] == 0 and sb["status"] == 0, (sa, sb)
@@ -103,3 +102,49 @@ def test_nonfinite_input_is_reported(cells):
     mesh.q0[mesh.n // 2] = np.nan
     st, _, _ = solve(mesh)
     assert st["status"] == 3 and st["iterations"] == 0, st
+
+
+@pytest.mark.parametrize("cells", [(10, 6, 5), (16, 8, 7), (24, 13, 12), (34, 20, 17)],
+                         ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("order", ["grid", "shuffled"])
+@pytest.mark.parametrize("pc", ["fsai", "learned"])
+def test_factor_solve_agrees_with_the_global_memory_form(cells, order, pc):
+    """The resident factor PCG against the global-memory one (standard form)."""
+    mesh = beams.build_beam("nh_beam", cells=cells)
+    if order == "shuffled":
+        mesh = shuffled(mesh)
+    sa, xa, _ = solve(mesh, preconditioner=pc)
+    sb, xb, _ = solve(mesh, preconditioner=pc, pcg_variant="global_memory")
+    assert sa["status"] == 0 and sb["status"] == 0, (sa, sb)
+    assert abs(sa["iterations"] - sb["iterations"]) <= max(2, sb["iterations"] // 50), (sa, sb)
+    assert np.abs(xa - xb).max() <= 1e-4 * np.abs(xb).max()
+
+
+@pytest.mark.parametrize("precision", ["fp16", "bf16", "fp32_refined"])
+@pytest.mark.parametrize("pc", ["fsai", "learned"])
+def test_factor_refinement_reaches_its_tolerance(precision, pc):
+    """The refinement's inner solves on the resident factor PCG: the fp64
+    residual meets the tolerance, and the solution the fp32 solve's to 1e-4."""
+    mesh = beams.build_beam("nh_beam", cells=(24, 13, 12))
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=2, energy=mesh.spec.energy, line_search=False, preconditioner=pc,
+                            solver_precision=precision, outer_tolerance=1e-6, inner_tolerance=1e-2)
+    a, b = model.state(), model.state()
+    a.particle_q.copy_(torch.as_tensor(mesh.q0, device=DEV))
+    solver.step(a, b, None, None, mesh.spec.dt)
+    for st in solver.mixed_stats():
+        assert st["status"] == 0 and st["rel_residual"] <= 1e-6, st
+
+
+def test_autotune_keeps_serving_a_shuffled_factor_plan():
+    """A plan whose vertex order the windowed factor PCG cannot take is still
+    tuned: the resident solve competes with the global-memory schedules."""
+    mesh = shuffled(beams.build_beam("nh_beam", cells=(24, 13, 12)))
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=1, energy=mesh.spec.energy, line_search=False, preconditioner="fsai")
+    q = torch.as_tensor(mesh.q0, device=DEV)
+    assert solver.autotune(q, mesh.spec.dt) > 0.0
+    a, b = model.state(), model.state()
+    a.particle_q.copy_(q)
+    solver.step(a, b, None, None, mesh.spec.dt)
+    assert solver.solve_stats()[0]["status"] == 0

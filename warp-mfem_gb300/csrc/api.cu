@@ -4,6 +4,7 @@
 #include <atomic>
 #include <climits>
 #include <cmath>
+#include <memory>
 #include <cstring>
 #include <string>
 #include <type_traits>
@@ -54,6 +55,8 @@ struct mfem_plan {
     // block-Jacobi plans of a mesh that one cluster holds: its parts
     // (mfem_plan_create); cluster 0: none
     ResidentLayout rl{};
+    ResidentLayout rf{};  // the same with a factor preconditioner
+    bool rf_on = true;    // rf in use (mfem_plan_autotune_batch decides)
     LineSearchWork ls{};
     float stage_dt = 0.0f;     // dt of the last mfem_assemble (the line search's 1/dt^2)
     int stage_slot = 0;        // slot of the last mfem_global_solve
@@ -132,6 +135,8 @@ namespace {
 constexpr int kClusterRows = 400;
 // Rows up to which every solve of one mesh adds its sums in the ordered way.
 constexpr int kOrderedRows = 384;
+// Rows a CTA of a factor preconditioner's grid aims at while SMs are left.
+constexpr int kFactorGridRows = 64;
 
 struct DeviceGuard {
     int prev = -1;
@@ -254,6 +259,9 @@ bool valid_config(const mfem_config *cfg, std::string &err) {
     return false;
 }
 
+// The fp32 solve of a one-mesh plan runs on its resident factor layout.
+bool factor_resident(const mfem_plan *p) { return p->rf.cluster > 0 && p->rf_on && p->bw.n_bodies <= 1; }
+
 // A plan with the learned preconditioner needs its net before any assembly.
 bool net_ready(const mfem_plan *p) { return p->cfg.preconditioner != 3 || p->fv.ready; }
 
@@ -265,7 +273,11 @@ cudaError_t solve_bodies(mfem_plan *p, int slot, cudaStream_t s) {
     for (size_t i = 0; e == cudaSuccess && i < classes; ++i) {
         const auto &c = p->body_classes[i];
         if (c.stream) e = cudaStreamWaitEvent(c.stream, p->body_fork, 0);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && c.L.factor)
+            e = launch_resident_factor(p->bv, p->vv, c.L, c.tasks, p->bw.n_bodies, p->pw, p->bw, p->bw.stats, slot,
+                                       p->cfg.cg_tolerance, p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr,
+                                       c.stream ? c.stream : s);
+        else if (e == cudaSuccess)
             e = launch_resident(p->bv, p->vv, c.L, c.tasks, p->bw.n_bodies, p->pw, p->bw.stats, slot,
                                 p->cfg.cg_tolerance, p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr,
                                 c.stream ? c.stream : s);
@@ -282,8 +294,11 @@ cudaError_t global_solve(mfem_plan *p, int slot, cudaStream_t s) {
     if (p->ir.mode != 0)
         return launch_mixed_solve(p->bv, p->vv, p->ir, p->pw, p->bw,
                                   p->pl.variant == PcgLayout::kFactor ? p->pl : p->ir_pl,
-                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr, p->rl, p->pcg_ctas,
+                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr, p->rl, p->rf, p->pcg_ctas,
                                   slot, p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
+    if (factor_resident(p))
+        return launch_resident_factor(p->bv, p->vv, p->rf, 1, 1, p->pw, p->bw, p->bw.stats, slot, p->cfg.cg_tolerance,
+                                      p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr, s);
     if (p->pl.variant == PcgLayout::kFactor)
         return launch_pcg_factor(p->bv, p->vv, p->pw, p->bw, p->pl, p->pcg_ctas, slot, p->cfg.cg_tolerance,
                                  p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
@@ -424,6 +439,10 @@ cudaError_t upload_resident(std::vector<void *> &allocs, const ResidentHost &h, 
     put(&v.src, h.src);
     put(&v.col, h.col);
     put(&v.push, h.push);
+    put(&v.ftrip_ptr, h.ftrip_ptr);
+    put(&v.fsrc, h.fsrc);
+    put(&v.fcol, h.fcol);
+    put(&v.fpush, h.fpush);
     return e;
 }
 
@@ -453,16 +472,43 @@ cudaError_t plan_refinement(mfem_plan *p) {
     return cudaSuccess;
 }
 
-// The trips that a layout streams: a buffer of the plan's.
+// The trips that a layout streams: buffers of the plan's.
 cudaError_t alloc_stream(std::vector<void *> &allocs, size_t parts, ResidentLayout &L) {
-    if (L.stream_trips == 0) return cudaSuccess;
     void *raw = nullptr;
-    const cudaError_t e = cudaMalloc(&raw, parts * kPartWarps * (size_t)L.stream_trips * 1280);
-    if (e != cudaSuccess) return e;
-    allocs.push_back(raw);
-    L.v.stream = static_cast<float4 *>(raw);
+    cudaError_t e = cudaSuccess;
+    if (L.stream_trips > 0) {
+        e = cudaMalloc(&raw, parts * kPartWarps * (size_t)L.stream_trips * 1280);
+        if (e != cudaSuccess) return e;
+        allocs.push_back(raw);
+        L.v.stream = static_cast<float4 *>(raw);
+    }
+    if (L.factor && !(L.f_shared[0] && L.f_shared[1])) {
+        e = cudaMalloc(&raw, parts * (size_t)(L.f_trips[0] + L.f_trips[1]) * 640);
+        if (e != cudaSuccess) return e;
+        allocs.push_back(raw);
+        L.v.fstream = static_cast<uint4 *>(raw);
+    }
     return e;
 }
+
+// Row pointers of the lower (columns <= row) and upper block CSR of H's
+// pattern, and the factor's form for the partition.
+struct FactorPattern {
+    std::vector<int32_t> lrow, urow;
+    ResidentFactor form;
+    FactorPattern(const std::vector<int32_t> &row_ptr, const std::vector<int32_t> &col_idx, int mode, bool redundant) {
+        const int n = (int)row_ptr.size() - 1;
+        lrow.assign(n + 1, 0);
+        urow.assign(n + 1, 0);
+        for (int r = 0; r < n; ++r) {
+            const int32_t *c0 = col_idx.data() + row_ptr[r], *c1 = col_idx.data() + row_ptr[r + 1];
+            const int lower = (int)(std::upper_bound(c0, c1, r) - c0);
+            lrow[r + 1] = lrow[r] + lower;
+            urow[r + 1] = urow[r] + (int)(c1 - c0) - lower + 1;  // the diagonal in both
+        }
+        form = ResidentFactor{mode, lrow.data(), urow.data(), redundant};
+    }
+};
 
 // The resident PCG of one mesh: a cluster, or past what 16 CTAs hold on the
 // chip a grid.  A part takes at most 128 rows, one slice a warp, while the
@@ -508,6 +554,29 @@ cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q
         return e;
     }
     return cudaSuccess;
+}
+
+// The resident factor PCG of one mesh with preconditioner 2 or 3, where a
+// step's result does not turn on the PCG's rounding (plan_resident): a grid
+// whose CTAs recompute the passes on their halos.  (A cluster that exchanges
+// the passes' results instead took 6.1 us an iteration against 4.4 at 637
+// vertices and 7.9 against 4.6 at 2,673.)
+cudaError_t plan_resident_factor(mfem_plan *p, int max_ctas) {
+    if (p->cfg.line_search || p->n <= kOrderedRows) return cudaSuccess;
+    const int parts = std::min(std::min(max_ctas, kPartMaxGrid), (p->n + kFactorGridRows - 1) / kFactorGridRows);
+    if (p->n > parts * 2 * kPartWarps * kPartSliceRows) return cudaSuccess;
+    const FactorPattern fp(p->h_row_ptr, p->h_col_idx, p->cfg.preconditioner, true);
+    ResidentHost h;
+    resident_add_body(h, p->h_row_ptr.data(), p->h_col_idx.data(), p->h_rest.data(), 0, p->n, parts, 0, false, true,
+                      &fp.form);
+    bool fits = false;
+    ResidentLayout L;
+    cudaError_t e = resident_factor_layout(p->device, h, parts, true, L, fits);
+    if (e != cudaSuccess || !fits) return e;
+    e = upload_resident(p->allocs, h, L.v);
+    if (e == cudaSuccess) e = alloc_stream(p->allocs, h.parts.size(), L);
+    if (e == cudaSuccess) p->rf = L;
+    return e;
 }
 
 uint64_t count_kernel_nodes(cudaGraph_t g) {
@@ -886,6 +955,15 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
             mfem_plan_destroy(p);
             return fail(nullptr, rc, msg);
         }
+        if (cfg.preconditioner >= 2 && cfg.pcg_ctas == 0 &&
+            (cfg.pcg_variant == PcgLayout::kAuto || cfg.pcg_variant == PcgLayout::kFactor)) {
+            e = plan_resident_factor(p, max_ctas);
+            if (e != cudaSuccess) {
+                const int rc2 = cuda_fail(nullptr, e, "resident factor PCG");
+                mfem_plan_destroy(p);
+                return rc2;
+            }
+        }
     }
     *out = p;
     return MFEM_OK;
@@ -904,12 +982,18 @@ int mfem_plan_sizes(const mfem_plan *p, int32_t *n, int32_t *T, int64_t *nnzb) {
 int mfem_plan_pcg_layout(const mfem_plan *p, int32_t *variant, int32_t *ctas, int32_t *cache_matrix,
                          int64_t *smem_bytes) {
     if (!p) return MFEM_BAD_ARG;
-    // the resident PCG is the single-reduction iteration with H on the chip
+    // the form the vertex order allows, with the sizes of what runs: the
+    // resident PCG in place of any of them
     const bool resident = p->rl.cluster > 0 && p->bw.n_bodies == 0 && (p->ir.mode == 0 || p->ir.mode == kIrFp32);
-    if (variant) *variant = resident ? (int)PcgLayout::kSingleReduction : p->pl.variant;
+    if (variant) *variant = p->pl.variant;
     if (ctas) *ctas = resident ? p->rl.cluster : p->pcg_ctas;
     if (cache_matrix) *cache_matrix = resident ? p->rl.stream_trips == 0 : p->pl.cache_matrix;
     if (smem_bytes) *smem_bytes = (int64_t)(resident ? p->rl.smem : p->pl.smem);
+    if (p->pl.variant == PcgLayout::kFactor && factor_resident(p)) {
+        if (ctas) *ctas = p->rf.cluster;
+        if (cache_matrix) *cache_matrix = p->rf.stream_trips == 0;
+        if (smem_bytes) *smem_bytes = (int64_t)p->rf.smem;
+    }
     return MFEM_OK;
 }
 
@@ -1337,7 +1421,8 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     alloc(&w.scale, 2 * sizeof(float));
     // a plan on the persistent factor PCG runs its inner solves there, on a
     // copy of the 16-bit blocks padded to 20 bytes (4-byte aligned loads)
-    const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor) &&
+    const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
+                             p->rf.cluster > 0) &&
                             p->cfg.preconditioner >= 1;
     if (!refined32 && persistent) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
     // ... and the whole refinement in one launch there, with the iterate
@@ -1510,10 +1595,11 @@ void drop_body_classes(mfem_plan *p) {
     p->bodies_resident = false;
 }
 
-// Clusters for block-Jacobi bodies.  A body takes ceil(rows / cap) CTAs,
+// Clusters for a batch's bodies.  A body takes ceil(rows / cap) CTAs,
 // rounded up to a size of the list; the cap is the smallest of 128, 256 and
-// 384 rows (one to three slices a warp) whose clusters all run at once, or 384:
-// fewer rows a CTA shorten an iteration (1.4 us at 128, 0.45 more a further
+// 384 rows (one to three slices a warp; 256 with a factor preconditioner, whose
+// blocks take shared memory too) whose clusters all run at once, or the
+// largest: fewer rows a CTA shorten an iteration (1.4 us at 128, 0.45 more a further
 // slice), more rows raise the bodies in flight.  Nothing is set (and nothing
 // is wrong) when a body is too large for a cluster of 16.
 cudaError_t plan_bodies(mfem_plan *p, int n_bodies, const int32_t *voff) {
@@ -1521,7 +1607,11 @@ cudaError_t plan_bodies(mfem_plan *p, int n_bodies, const int32_t *voff) {
     int sms = 1;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device);
     std::vector<int> size(n_bodies);
-    for (int cap = 128; cap <= 384; cap += 128) {
+    const bool factor = p->cfg.preconditioner >= 2;
+    std::unique_ptr<FactorPattern> fp;
+    if (factor) fp.reset(new FactorPattern(p->h_row_ptr, p->h_col_idx, p->cfg.preconditioner, false));
+    const int most_rows = factor ? 256 : 384;
+    for (int cap = 128; cap <= most_rows; cap += 128) {
         int64_t ctas = 0;
         for (int b = 0; b < n_bodies; ++b) {
             const int need = (voff[b + 1] - voff[b] + cap - 1) / cap;
@@ -1546,11 +1636,12 @@ cudaError_t plan_bodies(mfem_plan *p, int n_bodies, const int32_t *voff) {
         std::stable_sort(members.begin(), members.end(),
                          [&](int a, int b) { return voff[a + 1] - voff[a] > voff[b + 1] - voff[b]; });
         ResidentHost h;
-        resident_add_bodies(h, p->h_row_ptr.data(), p->h_col_idx.data(), p->h_rest.data(), voff, members,
-                            kSizes[i]);
+        resident_add_bodies(h, p->h_row_ptr.data(), p->h_col_idx.data(), p->h_rest.data(), voff, members, kSizes[i],
+                            factor ? &fp->form : nullptr);
         mfem_plan::ResidentClass c;
         bool fits = false;
-        e = resident_layout(p->device, h, kSizes[i], false, c.L, fits);
+        e = factor ? resident_factor_layout(p->device, h, kSizes[i], false, c.L, fits)
+                   : resident_layout(p->device, h, kSizes[i], false, c.L, fits);
         if (e != cudaSuccess || !fits) return e;
         c.tasks = (int)members.size();
         e = upload_resident(p->batch_allocs, h, c.L.v);
@@ -1751,7 +1842,7 @@ int install_bodies(mfem_plan *p, int n_bodies, const int32_t *voff, const int32_
                            : apply_batch_layout(p, 256, 2048.0, INT_MAX);
     // pcg_variant 5 asks for the global-memory PCG; a one-body batch of a mesh
     // too large for the persistent PCGs has no gravity of its own
-    if (rc == MFEM_OK && gravity && p->cfg.preconditioner <= 1 && p->cfg.pcg_ctas == 0 &&
+    if (rc == MFEM_OK && gravity && p->cfg.pcg_ctas == 0 &&
         (p->cfg.pcg_variant == PcgLayout::kAuto || p->cfg.pcg_variant == PcgLayout::kSingleReduction)) {
         e = plan_bodies(p, n_bodies, voff);
         if (e != cudaSuccess) rc = cuda_fail(p, e, "resident bodies");
@@ -1994,11 +2085,16 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
     };
     // the resident clusters first, where the bodies have them; the schedules
     // of the global-memory PCG against them
-    bool resident = !p->body_classes.empty();
+    const bool one = p->body_classes.empty() && p->rf.cluster > 0 && p->bw.n_bodies <= 1;
+    bool resident = !p->body_classes.empty() || one;
+    auto use_resident = [&](bool on) {
+        if (one) p->rf_on = on;
+        else p->bodies_resident = on;
+    };
     if (resident) {
         float ms = 0.0f;
         int flag = 0;
-        p->bodies_resident = true;
+        use_resident(true);
         time_solve(ms, flag);
         if (e == cudaSuccess && flag) {
             e = rearm_barriers(p);
@@ -2006,7 +2102,7 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
         } else {
             best = ms;
         }
-        p->bodies_resident = false;
+        use_resident(false);
     }
     const int threads_opts[3] = {128, 256, 512};
     const double c0_opts[3] = {512.0, 2048.0, 8192.0};
@@ -2067,7 +2163,7 @@ int mfem_plan_autotune_batch(mfem_plan *p, const float *d_q, float dt, double *h
     if (e1) cudaEventDestroy(e1);
     if (x) cudaFree(x);
     if (dx0) cudaFree(dx0);
-    p->bodies_resident = resident;
+    use_resident(resident);
     if (e != cudaSuccess) return cuda_fail(p, e, "autotune");
     drop_graphs(p);
     const int rc = apply_batch_layout(p, best_t, best_m, best_g);

@@ -305,6 +305,7 @@ constexpr int kPartWarps = 16;
 constexpr int kPartThreads = 32 * kPartWarps;
 constexpr int kPartMaxCluster = 16;
 constexpr int kPartMaxGrid = 256;
+constexpr int kFactorSliceRows = 32;  // rows a warp takes at once in a factor pass, a lane a row
 constexpr int kPartMaxBlocks = 8;  // of a part, with ordered sums
 constexpr int kPartRegTrips = 4;    // trips of a warp's first slice whose blocks stay in registers
 
@@ -314,6 +315,12 @@ struct ResPart {
     int slice_off, nslices;  // trip_ptr[slice_off + s]: first trip of slice s
     int push_off, push_passes;  // push[push_off + (pass * nslices + slice) * 32 + lane]
     int block_lo, nblocks;   // the sums' blocks of rows that the part holds (ordered sums), else 0
+    // factor preconditioners: local rows (own rows, then the halo in its
+    // order) whose second-pass and first-pass results the part computes, and
+    // the slices of the first (0) and second (1) pass
+    int second_rows, first_rows;
+    int fslice_off[2], nfslices[2];  // ftrip_ptr[fslice_off[w] + s]
+    int fpush_off, fpush_passes;     // fpush[fpush_off + (pass * slices + slice) * 32 + lane], slices of own rows
 };
 
 // The parts of a plan's bodies as the host builds them (partition.cpp).
@@ -327,24 +334,43 @@ struct ResidentHost {
     int nown_max = 0, nhalo_max = 0, nlocal_max = 0, push_max = 0;
     int trips_max = 0, trips_max_reg = 0;  // most trips of a warp, in all and without its register trips
     int slice_trips_max = 0;
+    std::vector<int32_t> ftrip_ptr, fsrc;     // the factor passes, as trip_ptr, src and col
+    std::vector<uint16_t> fcol;
+    std::vector<int32_t> fpush;               // as push, for the passes' slices of 32 own rows
+    int fpush_max = 0;
+    int f_trips_max[2] = {0, 0};
     int blocks = 0;         // ordered sums: blocks of the body, row n v / blocks on in block v
     int block_max = 0;      // most blocks of a part
 };
+// A factor preconditioner's two passes on H's lower block pattern: mode 2
+// applies F^T F, 3 F F^T; lrow, urow are the row pointers of the plan's lower
+// and upper CSR.  redundant: a part also computes both passes for the foreign
+// rows that its own need (their halo is then three hops of the pattern wide),
+// else its own rows only, and the parts exchange both results.
+struct ResidentFactor {
+    int mode;
+    const int32_t *lrow, *urow;
+    bool redundant;
+};
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel = true);
+                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel = true,
+                       const ResidentFactor *factor = nullptr);
 // The same with the parts runs of `blocks` equal ranges of consecutive rows: for
 // the resident PCG's ordered sums.
 void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
                          bool push_lists);
 // The same for several bodies of `parts` parts each, the bodies in parallel.
 void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                         const int32_t *row_off, const std::vector<int> &bodies, int parts);
+                         const int32_t *row_off, const std::vector<int> &bodies, int parts,
+                         const ResidentFactor *factor = nullptr);
 
 struct ResidentViews {
     const ResPart *parts;
     const int4 *tasks;
     const int *rows, *halo, *trip_ptr, *src, *push;
-    const uint16_t *col;
+    const uint16_t *col, *fcol;
+    const int *ftrip_ptr, *fsrc, *fpush;
+    uint4 *fstream;  // factor trips that do not fit in shared memory
     float4 *stream;  // trips that fit neither registers nor shared memory
 };
 
@@ -353,11 +379,14 @@ struct ResidentLayout {
     int cluster = 0;       // parts of a body; 0: the plan has no resident layout
     bool grid = false;     // the parts meet in global memory (a cooperative grid), else in a cluster
     int own_slots = 1, row_slots = 1;  // own rows, and rows in all, that a thread keeps
-    int nown_max = 0, nhalo_max = 0, push_max = 0;
+    int nown_max = 0, nhalo_max = 0, push_max = 0, fpush_max = 0;
     int smem_trips = 0;    // trips a warp keeps in shared memory
     int stream_trips = 0;  // trips a warp streams from global memory
     int blocks = 0;        // ordered sums over so many blocks of rows; 0: sums over the parts
     int block_max = 0;
+    bool factor = false;   // a factor preconditioner's layout (pcg_resident_factor.cu)
+    int f_trips[2] = {0, 0};         // most trips of a part in the first and second pass
+    bool f_shared[2] = {false, false};  // that pass's blocks sit in shared memory
     size_t smem = 0;       // dynamic shared memory per CTA
     ResidentViews v{};
 };
@@ -485,6 +514,13 @@ cudaError_t launch_pcg_inner(const BsrViews &bv, const VertexViews &vv, const Ir
 cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const ResidentLayout &L, int n_tasks,
                             int n_bodies, const PcgWork &w, SolveStats *stats, int slot, float tol, int maxiter,
                             int use_precond, const IrWork *ir, cudaStream_t s);
+// The same with a factor preconditioner (mode 2 or 3, the factor in bw's BF16
+// forms), falling back to block-Jacobi on a breakdown.
+cudaError_t resident_factor_layout(int device, const ResidentHost &h, int cluster, bool grid, ResidentLayout &L,
+                                   bool &fits);
+cudaError_t launch_resident_factor(const BsrViews &bv, const VertexViews &vv, const ResidentLayout &L, int n_tasks,
+                                   int n_bodies, const PcgWork &w, const BatchViews &bw, SolveStats *stats, int slot,
+                                   float tol, int maxiter, int mode, const IrWork *ir, cudaStream_t s);
 cudaError_t pcg_max_ctas(int device, int *ctas);
 cudaError_t pcg_plan_layout(int device, PcgLayout &L, const int32_t *row_ptr, const int32_t *col_idx, int n,
                             int ctas, int variant, std::vector<int4> &cta_info, std::string &err);
@@ -510,10 +546,11 @@ cudaError_t launch_batched_pcg(const BsrViews &bv, const VertexViews &vv, const 
 int ir_residual_blocks(int n);
 // With fp32 blocks and block-Jacobi the inner solves run on the resident
 // layout rl where the plan has one (rl.cluster > 0), else on its
-// single-reduction layout (single, or null), one launch a correction.
+// single-reduction layout (single, or null), with a factor preconditioner on
+// the resident factor layout rf where it has one, one launch a correction.
 cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const IrWork &w, const PcgWork &pw,
                                const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single,
-                               const ResidentLayout &rl, int pcg_ctas, int slot, int maxiter, int use_precond,
+                               const ResidentLayout &rl, const ResidentLayout &rf, int pcg_ctas, int slot, int maxiter, int use_precond,
                                cudaStream_t s);
 // The whole mixed refinement in one launch of the persistent factor PCG
 // (needs IrWork's xf_hi / xf_lo): the warm start in vv.dx, the solution

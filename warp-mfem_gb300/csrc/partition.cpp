@@ -113,25 +113,66 @@ struct Bisector {
 
 // Adds the parts rows[bounds[p] .. bounds[p + 1]) of one body.
 void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int row_lo, int body,
-               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads);
+               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads,
+               const ResidentFactor *factor);
 
 // One part's arrays before they are joined.
 struct PartArrays {
     std::vector<int32_t> halo, trip_ptr, src;
     std::vector<uint16_t> col;
     int trips_max = 0, trips_max_reg = 0, slice_trips_max = 0;
+    int second_rows = 0, first_rows = 0, f_trips_max[2] = {0, 0};
+    std::vector<int32_t> ftrip_ptr[2], fsrc[2];
+    std::vector<uint16_t> fcol[2];
 };
+
+// Slices of ROWS rows, 32 / ROWS lanes a row; a trip is one block a
+// lane, padded lanes read no block (src -1).  row_blocks(i) gives local row
+// i's blocks: its first src, its columns and their number; local(c) a
+// column's local row.  warp_trips[w] gets the trips of warp w's slices.
+struct RowBlocks {
+    int32_t src;
+    const int32_t *cols;
+    int len;
+};
+template <int ROWS, class R, class L>
+void slice_rows(int nrows, const R &row_blocks, const L &local, std::vector<int32_t> &trip_ptr,
+                std::vector<int32_t> &src, std::vector<uint16_t> &col, std::vector<int> &slice_trips) {
+    constexpr int lanes = 32 / ROWS;
+    for (int r0 = 0; r0 < nrows; r0 += ROWS) {
+        const int nr = std::min(ROWS, nrows - r0);
+        RowBlocks rb[ROWS];
+        int trips = 0;
+        for (int r = 0; r < nr; ++r) {
+            rb[r] = row_blocks(r0 + r);
+            trips = std::max(trips, (rb[r].len + lanes - 1) / lanes);
+        }
+        trip_ptr.push_back((int32_t)(src.size() / 32));
+        slice_trips.push_back(trips);
+        const size_t base = src.size();
+        src.resize(base + (size_t)32 * trips, -1);
+        col.resize(base + (size_t)32 * trips, 0);
+        for (int r = 0; r < nr; ++r)
+            for (int e = 0; e < rb[r].len; ++e) {
+                const size_t at = base + (size_t)(e / lanes) * 32 + e % lanes * ROWS + r;
+                src[at] = rb[r].src + e;
+                col[at] = (uint16_t)local(rb[r].cols[e]);
+            }
+    }
+    trip_ptr.push_back((int32_t)(src.size() / 32));
+}
 
 }  // namespace
 
 void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel) {
+                       int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel,
+                       const ResidentFactor *factor) {
     const int n = row_hi - row_lo;
     const int threads = parallel ? thread_count(n) : 1;
     std::vector<int> rows(n), bounds(parts + 1, 0);
     for (int i = 0; i < n; ++i) rows[i] = row_lo + i;
     Bisector{rest_q}.split(rows, parts, bounds, threads);
-    add_parts(h, row_ptr, col_idx, row_lo, body, rows, bounds, push_lists, threads);
+    add_parts(h, row_ptr, col_idx, row_lo, body, rows, bounds, push_lists, threads, factor);
 }
 
 void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
@@ -140,7 +181,7 @@ void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t 
     for (int i = 0; i < n; ++i) rows[i] = i;
     const int first_part = (int)h.parts.size();
     for (int p = 1; p <= parts; ++p) bounds[p] = (int)((int64_t)n * ((int64_t)blocks * p / parts) / blocks);
-    add_parts(h, row_ptr, col_idx, 0, 0, rows, bounds, push_lists, thread_count(n));
+    add_parts(h, row_ptr, col_idx, 0, 0, rows, bounds, push_lists, thread_count(n), nullptr);
     h.blocks = blocks;
     for (int p = 0; p < parts; ++p) {
         ResPart &rp = h.parts[first_part + p];
@@ -153,7 +194,8 @@ void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t 
 namespace {
 
 void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int row_lo, int body,
-               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads) {
+               std::vector<int> &rows, const std::vector<int> &bounds, bool push_lists, int threads,
+               const ResidentFactor *factor) {
     const int n = (int)rows.size(), parts = (int)bounds.size() - 1;
     const int first_part = (int)h.parts.size();
     std::vector<int> part_of(n), local(n);
@@ -174,51 +216,74 @@ void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, 
     parallel_for(parts, threads, [&](int p) {
         PartArrays &m = made[p];
         const int lo = bounds[p], nown = bounds[p + 1] - lo;
-        std::vector<char> met(n, 0);
+        std::vector<char> met(n, 0);  // in the halo
         std::unique_ptr<int[]> halo_slot(new int[n]);  // set for the halo rows only
-        // the halo: ascending rows of other parts
-        for (int i = 0; i < nown; ++i)
-            for (int k = row_ptr[rows[lo + i]]; k < row_ptr[rows[lo + i] + 1]; ++k)
-                if (part_of[col_idx[k] - row_lo] != p && !met[col_idx[k] - row_lo]) {
-                    met[col_idx[k] - row_lo] = 1;
-                    m.halo.push_back(col_idx[k]);
-                }
-        std::sort(m.halo.begin(), m.halo.end());
-        for (size_t i = 0; i < m.halo.size(); ++i) halo_slot[m.halo[i] - row_lo] = (int)i;
-        // slices of kPartSliceRows rows, kPartLanes lanes a row; a trip is one
-        // block a lane, padded lanes read no block (src -1)
-        const int nslices = (nown + kPartSliceRows - 1) / kPartSliceRows;
-        int warp_trips[kPartWarps] = {0}, reg_trips[kPartWarps] = {0};
-        for (int s = 0; s < nslices; ++s) {
-            const int r0 = s * kPartSliceRows, nr = std::min(kPartSliceRows, nown - r0);
-            int trips = 0;
-            for (int r = 0; r < nr; ++r) {
-                const int row = rows[lo + r0 + r];
-                trips = std::max(trips, (row_ptr[row + 1] - row_ptr[row] + kPartLanes - 1) / kPartLanes);
-            }
-            m.trip_ptr.push_back((int32_t)(m.src.size() / 32));
-            warp_trips[s % kPartWarps] += trips;
-            if (s < kPartWarps) reg_trips[s] = std::min(trips, kPartRegTrips);
-            m.slice_trips_max = std::max(m.slice_trips_max, trips);
-            const size_t base = m.src.size();
-            m.src.resize(base + (size_t)32 * trips, -1);
-            m.col.resize(base + (size_t)32 * trips, 0);
-            for (int r = 0; r < nr; ++r) {
-                const int row = rows[lo + r0 + r], k0 = row_ptr[row], len = row_ptr[row + 1] - k0;
-                for (int e = 0; e < len; ++e) {
-                    const int c = col_idx[k0 + e];
-                    const size_t at = base + (size_t)(e / kPartLanes) * 32 + e % kPartLanes * kPartSliceRows + r;
-                    m.src[at] = k0 + e;
-                    m.col[at] = (uint16_t)(part_of[c - row_lo] == p
-                                               ? local[c - row_lo]
-                                               : nown + halo_slot[c - row_lo]);
+        // the halo: ascending rows of other parts that the columns of `span`
+        // reach, appended hop by hop for a redundant factor (the rows that the
+        // second pass, the first pass and the residual are needed on)
+        const auto hop = [&](int from, int to, int side) {
+            // local rows [from, to): every column, or the lower (-1) or upper (1) ones
+            const size_t first = m.halo.size();
+            for (int i = from; i < to; ++i) {
+                const int row = i < nown ? rows[lo + i] : m.halo[i - nown];
+                for (int k = row_ptr[row]; k < row_ptr[row + 1]; ++k) {
+                    const int c = col_idx[k];
+                    if ((side < 0 && c > row) || (side > 0 && c < row)) continue;
+                    if (part_of[c - row_lo] == p || met[c - row_lo]) continue;
+                    met[c - row_lo] = 1;
+                    m.halo.push_back(c);
                 }
             }
+            std::sort(m.halo.begin() + first, m.halo.end());
+            return nown + (int)m.halo.size();
+        };
+        const int reach = hop(0, nown, 0);
+        m.second_rows = m.first_rows = nown;
+        // the first pass's columns: lower for F^T F, upper for F F^T
+        const int side0 = factor && factor->mode == 2 ? -1 : 1;
+        if (factor && factor->redundant) {
+            m.second_rows = reach;
+            m.first_rows = hop(0, m.second_rows, -side0);
+            hop(0, m.first_rows, side0);
         }
-        m.trip_ptr.push_back((int32_t)(m.src.size() / 32));
-        for (int w = 0; w < kPartWarps; ++w) {
-            m.trips_max = std::max(m.trips_max, warp_trips[w]);
-            m.trips_max_reg = std::max(m.trips_max_reg, warp_trips[w] - reg_trips[w]);
+        for (size_t i = 0; i < m.halo.size(); ++i) halo_slot[m.halo[i] - row_lo] = (int)i;
+        const auto local_row = [&](int c) {
+            return part_of[c - row_lo] == p ? local[c - row_lo] : nown + halo_slot[c - row_lo];
+        };
+        const auto row_of = [&](int i) { return i < nown ? rows[lo + i] : m.halo[i - nown]; };
+        std::vector<int> slice_trips;
+        slice_rows<kPartSliceRows>(nown,
+                   [&](int i) {
+                       const int row = rows[lo + i];
+                       return RowBlocks{row_ptr[row], col_idx + row_ptr[row], row_ptr[row + 1] - row_ptr[row]};
+                   },
+                   local_row, m.trip_ptr, m.src, m.col, slice_trips);
+        const auto warp_most = [&](int skip) {
+            int warp[kPartWarps] = {0}, most = 0;
+            for (size_t s = 0; s < slice_trips.size(); ++s)
+                warp[s % kPartWarps] += s < kPartWarps ? std::max(0, slice_trips[s] - skip) : slice_trips[s];
+            for (int w : warp) most = std::max(most, w);
+            return most;
+        };
+        m.trips_max = warp_most(0);
+        m.trips_max_reg = warp_most(kPartRegTrips);
+        for (int t : slice_trips) m.slice_trips_max = std::max(m.slice_trips_max, t);
+        for (int w = 0; factor && w < 2; ++w) {
+            const bool lower = (w == 0) == (side0 < 0);
+            slice_trips.clear();
+            slice_rows<kFactorSliceRows>(w == 0 ? m.first_rows : m.second_rows,
+                       [&](int i) {
+                           // columns ascend: the lower form is a row's head, the
+                           // upper its tail, the diagonal in both
+                           const int row = row_of(i);
+                           const int32_t *c0 = col_idx + row_ptr[row], *c1 = col_idx + row_ptr[row + 1];
+                           const int32_t *d = std::lower_bound(c0, c1, row);
+                           return lower ? RowBlocks{factor->lrow[row], c0, (int)(d - c0) + 1}
+                                        : RowBlocks{factor->urow[row], d, (int)(c1 - d)};
+                       },
+                       local_row, m.ftrip_ptr[w], m.fsrc[w], m.fcol[w], slice_trips);
+            m.f_trips_max[w] = m.ftrip_ptr[w].back();
+            for (int t : slice_trips) m.slice_trips_max = std::max(m.slice_trips_max, t);
         }
     });
     h.rows.insert(h.rows.end(), rows.begin(), rows.end());
@@ -242,6 +307,17 @@ void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, 
         h.nown_max = std::max(h.nown_max, rp.nown);
         h.nhalo_max = std::max(h.nhalo_max, rp.nhalo);
         h.nlocal_max = std::max(h.nlocal_max, rp.nown + rp.nhalo);
+        rp.second_rows = m.second_rows;
+        rp.first_rows = m.first_rows;
+        for (int w = 0; factor && w < 2; ++w) {
+            const int32_t base = (int32_t)(h.fsrc.size() / 32);
+            rp.fslice_off[w] = (int)h.ftrip_ptr.size();
+            rp.nfslices[w] = (int)m.ftrip_ptr[w].size() - 1;
+            for (int32_t t : m.ftrip_ptr[w]) h.ftrip_ptr.push_back(base + t);
+            h.fsrc.insert(h.fsrc.end(), m.fsrc[w].begin(), m.fsrc[w].end());
+            h.fcol.insert(h.fcol.end(), m.fcol[w].begin(), m.fcol[w].end());
+            h.f_trips_max[w] = std::max(h.f_trips_max[w], m.f_trips_max[w]);
+        }
         h.parts.push_back(rp);
     }
     h.halo.resize(halos);
@@ -277,27 +353,44 @@ void add_parts(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, 
                        e % kPartLanes * kPartSliceRows + (i - lo) % kPartSliceRows] = dst[e];
         }
         h.push_max = std::max(h.push_max, rp.push_passes * rp.nslices * 32);
+        if (!factor) continue;
+        const int slices = (rp.nown + kFactorSliceRows - 1) / kFactorSliceRows;
+        rp.fpush_off = (int)h.fpush.size();
+        rp.fpush_passes = (int)most;
+        h.fpush.resize(h.fpush.size() + most * slices * 32, -1);
+        for (int i = lo; i < hi; ++i) {
+            const auto &dst = push[rows[i] - row_lo];
+            for (size_t e = 0; e < dst.size(); ++e)
+                h.fpush[rp.fpush_off + (e * slices + (i - lo) / kFactorSliceRows) * 32 + (i - lo) % kFactorSliceRows] =
+                    dst[e];
+        }
+        h.fpush_max = std::max(h.fpush_max, rp.fpush_passes * slices * 32);
     }
 }
 
 }  // namespace
 
 void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
-                         const int32_t *row_off, const std::vector<int> &bodies, int parts) {
+                         const int32_t *row_off, const std::vector<int> &bodies, int parts,
+                         const ResidentFactor *factor) {
     std::vector<ResidentHost> made(bodies.size());
     int rows = 0;
     for (int b : bodies) rows += row_off[b + 1] - row_off[b];
     parallel_for((int)bodies.size(), thread_count(rows), [&](int i) {
         const int b = bodies[i];
-        resident_add_body(made[i], row_ptr, col_idx, rest_q, row_off[b], row_off[b + 1], parts, b, parts > 1, false);
+        resident_add_body(made[i], row_ptr, col_idx, rest_q, row_off[b], row_off[b + 1], parts, b, parts > 1, false,
+                          factor);
     });
     for (const ResidentHost &m : made) {
         const int first = (int)h.parts.size(), trips = (int)(h.src.size() / 32);
+        const int ftrips = (int)(h.fsrc.size() / 32);
         for (ResPart rp : m.parts) {
             rp.row_off += (int)h.rows.size();
             rp.halo_off += (int)h.halo.size();
             rp.slice_off += (int)h.trip_ptr.size();
             rp.push_off += (int)h.push.size();
+            for (int &off : rp.fslice_off) off += (int)h.ftrip_ptr.size();
+            rp.fpush_off += (int)h.fpush.size();
             h.parts.push_back(rp);
         }
         for (int4 t : m.tasks) h.tasks.push_back(make_int4(first + t.x, t.y, t.z, t.w));
@@ -307,6 +400,12 @@ void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t 
         h.src.insert(h.src.end(), m.src.begin(), m.src.end());
         h.col.insert(h.col.end(), m.col.begin(), m.col.end());
         h.push.insert(h.push.end(), m.push.begin(), m.push.end());
+        h.fpush.insert(h.fpush.end(), m.fpush.begin(), m.fpush.end());
+        h.fpush_max = std::max(h.fpush_max, m.fpush_max);
+        for (int32_t t : m.ftrip_ptr) h.ftrip_ptr.push_back(ftrips + t);
+        h.fsrc.insert(h.fsrc.end(), m.fsrc.begin(), m.fsrc.end());
+        h.fcol.insert(h.fcol.end(), m.fcol.begin(), m.fcol.end());
+        for (int w = 0; w < 2; ++w) h.f_trips_max[w] = std::max(h.f_trips_max[w], m.f_trips_max[w]);
         h.nown_max = std::max(h.nown_max, m.nown_max);
         h.nhalo_max = std::max(h.nhalo_max, m.nhalo_max);
         h.nlocal_max = std::max(h.nlocal_max, m.nlocal_max);
