@@ -68,8 +68,7 @@ struct mfem_plan {
     // host copies kept to rebuild the assembly's contribution lists
     std::vector<int32_t> h_tets, h_row_ptr, h_col_idx, h_tet_slots;
     std::vector<float> h_rest;  // [n][3] rest positions (the resident PCG's parts)
-    const int32_t *base_chunk_ptr = nullptr, *base_code = nullptr, *base_slot = nullptr;
-    int base_chunks = 0;
+    AssemblyLists base_lists{};
     // mixed-precision global solve (mfem_plan_set_solver); mode 0 = the
     // reference's float32 PCG
     IrWork ir{};
@@ -210,8 +209,9 @@ bool buffer_ref(const mfem_plan *p, int which, BufferRef &ref) {
         case MFEM_BUF_H_LAMBDA: ref = {p->tv.H_l, T * 21 * 4}; return true;
         case MFEM_BUF_HESS_S_INV: ref = {p->tv.H_si, T * 21 * 4}; return true;
         case MFEM_BUF_G_LAMBDA: ref = {p->tv.g_l, T * 6 * 4}; return true;
-        case MFEM_BUF_ELEMENT_HESSIAN: ref = {p->tv.Ke, T * kKeFloats * 4}; return true;
-        case MFEM_BUF_ELEMENT_RHS: ref = {p->tv.fe, T * kFeFloats * 4}; return true;
+        // interleaved in the element records: copied through record_copy
+        case MFEM_BUF_ELEMENT_HESSIAN: ref = {nullptr, T * kKeFloats * 4}; return true;
+        case MFEM_BUF_ELEMENT_RHS: ref = {nullptr, T * kFeFloats * 4}; return true;
         case MFEM_BUF_ROW_PTR: ref = {(void *)p->bv.row_ptr, (n + 1) * 4}; return true;
         case MFEM_BUF_COL_IDX: ref = {(void *)p->bv.col_idx, nnzb * 4}; return true;
         case MFEM_BUF_TET_SLOTS: ref = {p->tet_slots, T * 16 * 4}; return true;
@@ -231,6 +231,20 @@ bool buffer_ref(const mfem_plan *p, int which, BufferRef &ref) {
         case MFEM_BUF_PRECOND_FACTOR: ref = {(void *)p->bw.Lval, (size_t)p->bw.nnzl * 9 * 4}; return true;
         default: return false;
     }
+}
+
+// The element blocks or right-hand sides as the plain arrays of the interface,
+// out of or into the records, through a stream-ordered scratch array.
+cudaError_t record_copy(const mfem_plan *p, int which, void *plain, size_t bytes, bool out, cudaStream_t s) {
+    const int per = which == MFEM_BUF_ELEMENT_HESSIAN ? kKeFloats : kFeFloats;
+    void *tmp = nullptr;
+    cudaError_t e = cudaMallocAsync(&tmp, bytes, s);
+    if (e != cudaSuccess) return e;
+    if (!out) e = cudaMemcpyAsync(tmp, plain, bytes, cudaMemcpyDefault, s);
+    if (e == cudaSuccess) e = launch_record_copy(p->tv, static_cast<float *>(tmp), per, out, s);
+    if (e == cudaSuccess && out) e = cudaMemcpyAsync(plain, tmp, bytes, cudaMemcpyDefault, s);
+    const cudaError_t f = cudaFreeAsync(tmp, s);
+    return e == cudaSuccess ? f : e;
 }
 
 bool valid_config(const mfem_config *cfg, std::string &err) {
@@ -702,7 +716,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     sym.tet_slots.resize((size_t)T * 16);
     if (!build_slot_map(n, T, h_tets, sym.row_ptr.data(), sym.col_idx.data(), sym.tet_slots.data(), err))
         return fail(nullptr, MFEM_BAD_ARG, err);
-    if (!build_contributions(n, T, h_tets, sym.row_ptr.data(), sym.tet_slots.data(), sym, err))
+    if (!build_contributions(n, T, sym.row_ptr.data(), sym.tet_slots.data(), sym, err))
         return fail(nullptr, MFEM_BAD_ARG, err);
 
     // (M + Q) diagonal: Hessian mass is identity on attached vertices and
@@ -732,11 +746,12 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     for (int a = 0; a < 3; ++a) p->gravity[a] = h_gravity[a];
 
     const size_t nT = T, nn = n, nz = (size_t)p->nnzb;
-    const int n_chunks = (int)sym.chunk_ptr.size() - 1;
     cudaError_t e = cudaSuccess;
     int4 *tets = nullptr;
     float *dminv = nullptr, *materials = nullptr, *mass = nullptr, *hd = nullptr, *pk = nullptr, *pt = nullptr;
-    int32_t *row_ptr = nullptr, *col_idx = nullptr, *chunk_ptr = nullptr, *ccode = nullptr, *cslot = nullptr;
+    int32_t *row_ptr = nullptr, *col_idx = nullptr, *ccode = nullptr;
+    int4 *chunk = nullptr;
+    int2 *pair = nullptr;
     float *rest = nullptr;
 #define ALLOC(ptr, count)                                  \
     if (e == cudaSuccess) e = dev_alloc(p, &(ptr), (count));
@@ -751,8 +766,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     ALLOC(p->tv.H_l, nT * 21);
     ALLOC(p->tv.H_si, nT * 21);
     ALLOC(p->tv.g_l, nT * 6);
-    ALLOC(p->tv.Ke, nT * kKeFloats);
-    ALLOC(p->tv.fe, nT * kFeFloats);
+    ALLOC(p->tv.Ke, nT * kKeRecord);
     ALLOC(p->tv.degenerate, nT);
     ALLOC(p->tv.n_degenerate, 1);
     ALLOC(p->tet_slots, nT * 16);
@@ -771,9 +785,9 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     ALLOC(row_ptr, nn + 1);
     ALLOC(col_idx, nz);
     ALLOC(p->bv.values, nz * 9);
-    ALLOC(chunk_ptr, (size_t)n_chunks + 1);
+    ALLOC(chunk, sym.chunk.size());
     ALLOC(ccode, sym.contrib_code.size());
-    ALLOC(cslot, sym.contrib_slot.size());
+    ALLOC(pair, sym.pair.size());
     ALLOC(p->pw.pub, 6 * n_pad * 3);  // also the resident PCG's [2][n] float4
     ALLOC(p->pw.partials, 2 * 256 * 4);
     ALLOC(p->pw.counter, 1);
@@ -886,9 +900,9 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     if (e == cudaSuccess) e = upload(p->inv_mass, h_inv_mass, nn);
     if (e == cudaSuccess) e = upload(row_ptr, sym.row_ptr.data(), nn + 1);
     if (e == cudaSuccess) e = upload(col_idx, sym.col_idx.data(), nz);
-    if (e == cudaSuccess) e = upload(chunk_ptr, sym.chunk_ptr.data(), (size_t)n_chunks + 1);
+    if (e == cudaSuccess) e = upload(chunk, sym.chunk.data(), sym.chunk.size());
     if (e == cudaSuccess) e = upload(ccode, sym.contrib_code.data(), sym.contrib_code.size());
-    if (e == cudaSuccess) e = upload(cslot, sym.contrib_slot.data(), sym.contrib_slot.size());
+    if (e == cudaSuccess) e = upload(pair, sym.pair.data(), sym.pair.size());
     if (e == cudaSuccess) e = cudaMemset(p->pw.partials, 0, 2 * 256 * 4 * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(p->pw.counter, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(p->pw.res_counter, 0, sizeof(unsigned long long));
@@ -922,14 +936,8 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     p->bv.nnzb = p->nnzb;
     p->bv.row_ptr = row_ptr;
     p->bv.col_idx = col_idx;
-    p->bv.n_chunks = n_chunks;
-    p->bv.chunk_ptr = chunk_ptr;
-    p->bv.contrib_code = ccode;
-    p->bv.contrib_slot = cslot;
-    p->base_chunk_ptr = chunk_ptr;
-    p->base_code = ccode;
-    p->base_slot = cslot;
-    p->base_chunks = n_chunks;
+    p->base_lists = {(int)sym.chunk.size(), chunk, ccode, pair};
+    p->bv.asm_lists = p->base_lists;
     p->h_tets.assign(h_tets, h_tets + (size_t)T * 4);
     p->h_rest.assign(h_rest_q, h_rest_q + nn * 3);
     p->h_row_ptr = sym.row_ptr;
@@ -1014,7 +1022,9 @@ int mfem_plan_copy_out(const mfem_plan *pc, int32_t which, void *dst, size_t byt
     if (bytes == 0) return MFEM_OK;
     if (!dst) return fail(p, MFEM_BAD_ARG, "dst is NULL");
     DeviceGuard g(p->device);
-    cudaError_t e = cudaMemcpyAsync(dst, ref.ptr, bytes, cudaMemcpyDefault, (cudaStream_t)stream);
+    cudaError_t e = which == MFEM_BUF_ELEMENT_HESSIAN || which == MFEM_BUF_ELEMENT_RHS
+                        ? record_copy(p, which, dst, bytes, true, (cudaStream_t)stream)
+                        : cudaMemcpyAsync(dst, ref.ptr, bytes, cudaMemcpyDefault, (cudaStream_t)stream);
     return e == cudaSuccess ? MFEM_OK : cuda_fail(p, e, "copy_out");
 }
 
@@ -1028,7 +1038,9 @@ int mfem_plan_copy_in(mfem_plan *p, int32_t which, const void *src, size_t bytes
     if (bytes == 0) return MFEM_OK;
     if (!src) return fail(p, MFEM_BAD_ARG, "src is NULL");
     DeviceGuard g(p->device);
-    cudaError_t e = cudaMemcpyAsync(ref.ptr, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream);
+    cudaError_t e = which == MFEM_BUF_ELEMENT_HESSIAN || which == MFEM_BUF_ELEMENT_RHS
+                        ? record_copy(p, which, const_cast<void *>(src), bytes, false, (cudaStream_t)stream)
+                        : cudaMemcpyAsync(ref.ptr, src, bytes, cudaMemcpyDefault, (cudaStream_t)stream);
     return e == cudaSuccess ? MFEM_OK : cuda_fail(p, e, "copy_in");
 }
 
@@ -1185,7 +1197,7 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
         return fail(p, MFEM_BAD_ARG, err);
     Symbolic sym;
     sym.col_idx = p->h_col_idx;
-    if (m > 0 && !build_contributions(p->n, p->T, p->h_tets.data(), p->h_row_ptr.data(), p->h_tet_slots.data(), sym,
+    if (m > 0 && !build_contributions(p->n, p->T, p->h_row_ptr.data(), p->h_tet_slots.data(), sym,
                                       err, m, tri_slots.data()))
         return fail(p, MFEM_BAD_ARG, err);
 
@@ -1200,10 +1212,7 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
     p->contact_allocs.clear();
     p->cv = ContactViews{};
     p->cv.tri_code_base = INT32_MAX;
-    p->bv.chunk_ptr = p->base_chunk_ptr;
-    p->bv.contrib_code = p->base_code;
-    p->bv.contrib_slot = p->base_slot;
-    p->bv.n_chunks = p->base_chunks;
+    p->bv.asm_lists = p->base_lists;
     p->n_bodies = 0;
     p->n_tris = 0;
     p->h_tris.clear();
@@ -1222,7 +1231,9 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
     };
     int *type = nullptr, *body = nullptr, *tris = nullptr, *vtp = nullptr, *vtc = nullptr;
     float *pose = nullptr, *scale = nullptr, *mu = nullptr, *body_q = nullptr;
-    int32_t *chunk_ptr = nullptr, *ccode = nullptr, *cslot = nullptr;
+    int32_t *ccode = nullptr;
+    int4 *chunk = nullptr;
+    int2 *pair = nullptr;
     ContactViews &cv = p->cv;
     alloc(&type, n_shapes);
     alloc(&pose, (size_t)n_shapes * 7);
@@ -1241,11 +1252,10 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
     alloc(&tris, (size_t)m * 3);
     alloc(&vtp, n + 1);
     alloc(&vtc, (size_t)m * 3);
-    const int n_chunks = m > 0 ? (int)sym.chunk_ptr.size() - 1 : 0;
     if (m > 0) {
-        alloc(&chunk_ptr, sym.chunk_ptr.size());
+        alloc(&chunk, sym.chunk.size());
         alloc(&ccode, sym.contrib_code.size());
-        alloc(&cslot, sym.contrib_slot.size());
+        alloc(&pair, sym.pair.size());
     }
     // the deferred local solve's partials cover max(vertices, tris); they
     // live as long as the plan
@@ -1264,9 +1274,9 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
     if (e == cudaSuccess && m > 0) e = upload(vtp, vt_ptr.data(), n + 1);
     else if (e == cudaSuccess) e = cudaMemset(vtp, 0, (n + 1) * sizeof(int));
     if (e == cudaSuccess && m > 0) e = upload(vtc, vt_code.data(), (size_t)m * 3);
-    if (e == cudaSuccess && m > 0) e = upload(chunk_ptr, sym.chunk_ptr.data(), sym.chunk_ptr.size());
+    if (e == cudaSuccess && m > 0) e = upload(chunk, sym.chunk.data(), sym.chunk.size());
     if (e == cudaSuccess && m > 0) e = upload(ccode, sym.contrib_code.data(), sym.contrib_code.size());
-    if (e == cudaSuccess && m > 0) e = upload(cslot, sym.contrib_slot.data(), sym.contrib_slot.size());
+    if (e == cudaSuccess && m > 0) e = upload(pair, sym.pair.data(), sym.pair.size());
     if (e == cudaSuccess) e = cudaMemset(cv.normal_lagged, 0, n * 3 * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(cv.force_lagged, 0, n * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(cv.shape_lagged, 0xff, n * sizeof(int));
@@ -1316,12 +1326,7 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
     cv.vt_ptr = vtp;
     cv.vt_code = vtc;
     cv.tri_code_base = m > 0 ? 16 * p->T : INT32_MAX;
-    if (m > 0) {
-        p->bv.chunk_ptr = chunk_ptr;
-        p->bv.contrib_code = ccode;
-        p->bv.contrib_slot = cslot;
-        p->bv.n_chunks = n_chunks;
-    }
+    if (m > 0) p->bv.asm_lists = {(int)sym.chunk.size(), chunk, ccode, pair};
     p->n_bodies = n_bodies;
     p->n_tris = m;
     p->h_tris.assign(h_tris, h_tris + (size_t)m * 3);

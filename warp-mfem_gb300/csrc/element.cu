@@ -27,53 +27,40 @@ __device__ __forceinline__ void load_vec3(const float *__restrict__ p, int i, fl
     v[2] = p[3 * i + 2];
 }
 
-// Element outputs staged per warp in shared memory, so that the tet-major
-// element blocks and rhs (which the assembly gathers per tet) leave in
-// 16-byte stores of consecutive tets instead of 90 scalar stores 360 bytes
-// apart.  Odd row strides keep the lanes' scalar writes free of bank
-// conflicts.
+// A warp stages its 32 tets' element records in shared memory, tet-major as
+// in global memory, and one bulk copy takes them there.  The staging writes
+// are 16 bytes a lane at a 416-byte stride (two lanes a bank group, so twice
+// the least number of cycles); the copy itself costs the warp nothing, where
+// 90 + 12 separate floats had to be picked up again through an index division
+// and four scalar loads for each 16-byte store.  331,200 tets: 138 -> 135 us,
+// and 126 us with four blocks an SM at 128 registers instead of three at 168
+// (160 bytes of spills a thread): latency of dependent arithmetic and fetching
+// 100 KB of straight-line code bound it, at 43% of the issue slots.
 constexpr int kElementWarps = kElementThreads / 32;
-constexpr int kKeStride = kKeFloats + 1;
-constexpr int kFeStride = kFeFloats + 1;
-constexpr int kElementSmem = kElementWarps * 32 * (kKeStride + kFeStride) * (int)sizeof(float);
+constexpr int kElementSmem = kElementWarps * 32 * kKeRecord * (int)sizeof(float);
 // grid of the fp64 pass: it loops over however many tets were listed
 constexpr int kElementFp64Blocks = 304;
 
-// Copies `count` floats of the warp's staged rows (row r = tet t0 + r, `per`
-// floats a row, stride `stride` in shared memory) to dst = the first tet's
-// output, 16 bytes a store where the destination allows.
-template <int per, int stride>
-__device__ __forceinline__ void warp_copy_out(const float *__restrict__ src, float *__restrict__ dst, int count,
-                                              int lane) {
-    const int n4 = count >> 2;
-    float4 *d4 = reinterpret_cast<float4 *>(dst);
-    for (int q = lane; q < n4; q += 32) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = 4 * q + u;
-            const int r = j / per;
-            v[u] = src[r * stride + (j - r * per)];
-        }
-        d4[q] = make_float4(v[0], v[1], v[2], v[3]);
-    }
-    for (int j = 4 * n4 + lane; j < count; j += 32) {
-        const int r = j / per;
-        dst[j] = src[r * stride + (j - r * per)];
-    }
+// One lane: `bytes` of shared memory (16-byte aligned, as are dst and bytes)
+// to global memory; returns when the source has been read.
+__device__ __forceinline__ void bulk_store(float *dst, const float *src, unsigned bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(src);
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(s), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
 // Everything one Newton iteration needs from tet t: the per-tet terms
 // (component-major, straight to global memory) and the element blocks and
-// rhs, written to ke [90] and fe [12] (shared-memory staging rows in the
-// element kernel, the tet's global rows in the fp64 pass).  FP64 takes the
+// rhs, written to the record rec (a shared-memory staging row in the element
+// kernel, the tet's global row in the fp64 pass).  FP64 takes the
 // polar decomposition and dS/dF in float64.  DIAG also writes H_s^-1 and
 // g_lambda, which the step does not read (the local solve and the rhs use
 // the cancellation-free form) but the stage diagnostics expose.  Returns
 // det F in float32.
 template <bool FP64, bool DIAG>
 __device__ __forceinline__ float element_tet(const float *__restrict__ x, int energy, const TetViews &tv, int t,
-                                             float *ke, float *fe) {
+                                             float *rec) {
     const int T = tv.n_tets;
     const int4 tt = tv.tets[t];
     float xv[4][3];
@@ -142,6 +129,9 @@ __device__ __forceinline__ float element_tet(const float *__restrict__ x, int en
         for (int j = 0; j < 6; ++j) acc += H_l[em::p21(i, j)] * c[j];
         w[i] = acc;
     }
+    float4 *const rec4 = reinterpret_cast<float4 *>(rec);
+    float tail[8];  // ninth entries of the off-diagonal blocks, in record order
+    tail[6] = tail[7] = 0.0f;
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
         float P[6][3];  // H_l G_l
@@ -154,16 +144,17 @@ __device__ __forceinline__ float element_tet(const float *__restrict__ x, int en
                 for (int j = 0; j < 6; ++j) acc += H_l[em::p21(i, j)] * G[j][3 * l + b];
                 P[i][b] = acc;
             }
+        float fe[3];
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
             float acc = 0.0f;
 #pragma unroll
             for (int i = 0; i < 6; ++i) acc += G[i][3 * l + b] * w[i];
-            fe[3 * l + b] = acc;
+            fe[b] = acc;
         }
 #pragma unroll
         for (int k = 0; k <= l; ++k) {
-            float *blk = ke + ke_block(k, l) * 9;
+            float blk[9];
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -173,32 +164,39 @@ __device__ __forceinline__ float element_tet(const float *__restrict__ x, int en
                     for (int i = 0; i < 6; ++i) acc += G[i][3 * k + a] * P[i][b];
                     blk[a * 3 + b] = acc;
                 }
+            const int head = ke_block(k, l) * (kKeHead / 4);
+            rec4[head] = make_float4(blk[0], blk[1], blk[2], blk[3]);
+            rec4[head + 1] = make_float4(blk[4], blk[5], blk[6], blk[7]);
+            if (k == l) rec4[kKeDiagTail / 4 + l] = make_float4(blk[8], fe[0], fe[1], fe[2]);
+            else tail[ke_off_tail(k, l) - kKeOffTail] = blk[8];
         }
     }
+    rec4[kKeOffTail / 4] = make_float4(tail[0], tail[1], tail[2], tail[3]);
+    rec4[kKeOffTail / 4 + 1] = make_float4(tail[4], tail[5], tail[6], tail[7]);
     return detF;
 }
 
 // One thread per tet, in float32; tets with det F < 1e-3 are listed for
 // element_fp64_kernel, which redoes them with the float64 polar path.
 template <bool DIAG>
-__global__ void __launch_bounds__(kElementThreads, 3)
+__global__ void __launch_bounds__(kElementThreads, 4)
     element_kernel(const float *__restrict__ x, int energy, TetViews tv) {
-    extern __shared__ __align__(16) float s_stage[];
+    extern __shared__ __align__(128) float s_stage[];
     const int T = tv.n_tets;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t0 = blockIdx.x * blockDim.x + warp * 32;  // the warp's first tet
     if (t0 >= T) return;                                 // warp-uniform
     const int t = t0 + lane;
-    float *const w_ke = s_stage + warp * 32 * kKeStride;                                   // [32][kKeStride]
-    float *const w_fe = s_stage + kElementWarps * 32 * kKeStride + warp * 32 * kFeStride;  // [32][kFeStride]
+    float *const w_rec = s_stage + warp * 32 * kKeRecord;  // [32][kKeRecord]
     if (t < T) {
-        const float detF = element_tet<false, DIAG>(x, energy, tv, t, w_ke + lane * kKeStride, w_fe + lane * kFeStride);
+        const float detF = element_tet<false, DIAG>(x, energy, tv, t, w_rec + lane * kKeRecord);
         if (!(detF >= em::kPolarFp64Det)) tv.degenerate[atomicAdd(tv.n_degenerate, 1u)] = t;
     }
+    // the staged records are visible to the bulk copy after this fence
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    const int nv = min(32, T - t0);
-    warp_copy_out<kKeFloats, kKeStride>(w_ke, tv.Ke + (size_t)t0 * kKeFloats, nv * kKeFloats, lane);
-    warp_copy_out<kFeFloats, kFeStride>(w_fe, tv.fe + (size_t)t0 * kFeFloats, nv * kFeFloats, lane);
+    if (lane == 0)
+        bulk_store(tv.Ke + (size_t)t0 * kKeRecord, w_rec, (unsigned)min(32, T - t0) * kKeRecord * (unsigned)sizeof(float));
 }
 
 // The listed near-degenerate or inverted tets again, with the polar
@@ -210,7 +208,7 @@ __global__ void __launch_bounds__(kElementThreads)
     const unsigned count = *tv.n_degenerate;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const int t = tv.degenerate[i];
-        element_tet<true, DIAG>(x, energy, tv, t, tv.Ke + (size_t)t * kKeFloats, tv.fe + (size_t)t * kFeFloats);
+        element_tet<true, DIAG>(x, energy, tv, t, tv.Ke + (size_t)t * kKeRecord);
     }
 }
 
@@ -421,6 +419,26 @@ __global__ void __launch_bounds__(kVertexThreads)
     for (int a = 0; a < 3; ++a) qd_out[3 * v + a] = (q_out[3 * v + a] - vv.x_start[3 * v + a]) / dt;
 }
 
+// The element blocks [T][10][3][3] (per = 90) or right-hand sides [T][12]
+// (per = 12) of the records, out to or in from a plain array.
+__device__ __forceinline__ int record_entry(int per, int j) {
+    if (per == kFeFloats) return kKeDiagTail + (j / 3) * 4 + 1 + j % 3;
+    const int b = j / 9, e = j - 9 * b;
+    if (e < kKeHead) return b * kKeHead + e;
+    const int k = (b >= 4) + (b >= 7) + (b >= 9), l = b - ke_block(k, k) + k;  // inverse of ke_block
+    return k == l ? kKeDiagTail + 4 * k : ke_off_tail(k, l);
+}
+
+template <bool OUT>
+__global__ void __launch_bounds__(kVertexThreads) record_copy_kernel(float *rec, float *plain, long long count, int per) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
+        const long long t = i / per;
+        float *const r = rec + t * kKeRecord + record_entry(per, (int)(i - t * per));
+        if (OUT) plain[i] = *r;
+        else *r = plain[i];
+    }
+}
+
 inline int blocks_for(int n, int threads) { return (n + threads - 1) / threads; }
 
 }  // namespace
@@ -437,6 +455,16 @@ cudaError_t launch_predict(const float *q_in, const float *qd_in, float *q_out, 
     if (vv.n == 0) return cudaSuccess;
     predict_kernel<<<blocks_for(vv.n, kVertexThreads), kVertexThreads, 0, s>>>(q_in, qd_in, q_out, gravity[0],
                                                                                gravity[1], gravity[2], dt, vv);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_record_copy(const TetViews &tv, float *plain, int per, bool out, cudaStream_t s) {
+    const long long count = (long long)tv.n_tets * per;
+    if (count == 0) return cudaSuccess;
+    const int blocks = (int)std::min<long long>((count + kVertexThreads - 1) / kVertexThreads, 8192);
+    if (out) record_copy_kernel<true><<<blocks, kVertexThreads, 0, s>>>(tv.Ke, plain, count, per);
+    else record_copy_kernel<false><<<blocks, kVertexThreads, 0, s>>>(tv.Ke, plain, count, per);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -18,11 +18,22 @@ namespace mfem {
 constexpr int kKeBlocks = 10;
 constexpr int kKeFloats = kKeBlocks * 9;
 constexpr int kFeFloats = 12;
+// A tet's element record as the assembly reads it: 32-byte sectors that hold
+// the first eight entries of each block (one 32-byte load a contribution),
+// then for each diagonal block its ninth entry with the vertex's three rhs
+// entries (one 16-byte load), then the ninth entries of the six others and
+// two floats of padding: 416 bytes, 13 sectors.
+constexpr int kKeHead = 8;
+constexpr int kKeDiagTail = kKeBlocks * kKeHead;  // 80
+constexpr int kKeOffTail = kKeDiagTail + 16;      // 96
+constexpr int kKeRecord = 104;
 
 __host__ __device__ __forceinline__ int ke_block(int k, int l) {
     // k <= l
     return k * 4 - (k * (k - 1)) / 2 + (l - k);
 }
+// place of block (k, l)'s ninth entry in the record, k < l
+__host__ __device__ __forceinline__ constexpr int ke_off_tail(int k, int l) { return kKeOffTail + l * (l - 1) / 2 + k; }
 
 // Packed upper triangle of a symmetric 6x6, row-major: (0,0)..(0,5),(1,1)..(5,5).
 __host__ __device__ __forceinline__ constexpr int sym6_index(int i, int j) {
@@ -53,8 +64,7 @@ struct TetViews {
     float *H_si;               // [21][T]
     float *g_l;                // [6][T]
     // element contributions gathered by the assembly, tet-major
-    float *Ke;                 // [T][90]
-    float *fe;                 // [T][12]
+    float *Ke;                 // [T][kKeRecord] blocks and rhs
     const unsigned char *energy_code;  // [T] per-tet energy (batched bodies), or null: the plan's
     // tets with det F < 1e-3, listed by the element kernel for its float64 pass
     int *degenerate;           // [T]
@@ -153,6 +163,22 @@ constexpr int kFactorLd = 10;
 constexpr int kFsaiMaxCols = 16;  // lower block columns a row may have for FSAI
 constexpr int kFsaiDim = 3 * kFsaiMaxCols;
 
+// What the assembly gathers.  Only the diagonal and upper slots are summed;
+// their transposes are the lower ones, bit for bit, since both would add the
+// same contributions in the same order.
+struct AssemblyLists {
+    int n_chunks;
+    // [n_chunks] a warp's work: contributions [x, y), whole slots; the first
+    // slot's pair z; bit i of w: lane i's contribution opens a slot
+    const int4 *chunk;
+    // e*16 + k*4 + l; 16 T + 9 tri + 3 i + j with contact tris; negative for
+    // the one empty contribution of a vertex without tets
+    const int *code;
+    // per summed slot: the slot, and the lower slot it is mirrored to or ~row
+    // on the diagonal
+    const int2 *pair;
+};
+
 struct BsrViews {
     int n;
     int64_t nnzb;
@@ -160,10 +186,7 @@ struct BsrViews {
     const int *col_idx;        // [nnzb]
     float *values;             // [nnzb][9]
     // contribution lists sorted by slot, packed into warp-sized chunks
-    int n_chunks;
-    const int *chunk_ptr;      // [n_chunks+1]
-    const int *contrib_code;   // e*16 + k*4 + l, or -(row+1) for an empty diagonal
-    const int *contrib_slot;   // slot of each contribution
+    AssemblyLists asm_lists;
 };
 
 struct PcgWork {
@@ -460,7 +483,9 @@ cudaError_t launch_refine(const RefineViews &rv, const ContactViews &cv, const R
 // Host-side symbolic analysis (symbolic.cpp).
 struct Symbolic {
     std::vector<int32_t> row_ptr, col_idx, tet_slots;
-    std::vector<int32_t> chunk_ptr, contrib_code, contrib_slot;
+    std::vector<int4> chunk;             // as AssemblyLists
+    std::vector<int32_t> contrib_code;
+    std::vector<int2> pair;
 };
 bool build_sparsity(int n, int T, const int32_t *tets, std::vector<int32_t> &row_ptr,
                     std::vector<int32_t> &col_idx, std::string &err);
@@ -471,7 +496,7 @@ bool build_slot_map(int n, int T, const int32_t *tets, const int32_t *row_ptr, c
 bool build_tri_slots(int n, int n_tris, const int32_t *tris, const int32_t *row_ptr, const int32_t *col_idx,
                      int32_t *tri_slots, std::vector<int32_t> &vt_ptr, std::vector<int32_t> &vt_code,
                      std::string &err);
-bool build_contributions(int n, int T, const int32_t *tets, const int32_t *row_ptr,
+bool build_contributions(int n, int T, const int32_t *row_ptr,
                          const int32_t *slots, Symbolic &sym, std::string &err, int n_tris = 0,
                          const int32_t *tri_slots = nullptr);
 
@@ -484,6 +509,9 @@ cudaError_t launch_predict(const float *q_in, const float *qd_in, float *q_out, 
 // g_lambda, which the step itself does not read.
 cudaError_t prepare_element_kernels();
 cudaError_t launch_element(const float *x, int energy, const TetViews &tv, bool diagnostics, cudaStream_t s);
+// the records' blocks (per = kKeFloats) or right-hand sides (per = kFeFloats)
+// to or from a plain device array [T][per]
+cudaError_t launch_record_copy(const TetViews &tv, float *plain, int per, bool out, cudaStream_t s);
 cudaError_t launch_assemble(const float *x, float dt, float singular_threshold, int use_precond,
                             const TetViews &tv, const VertexViews &vv, const BsrViews &bv, const ContactViews &cv,
                             cudaStream_t s);

@@ -7,9 +7,10 @@
 //
 //  * the vertex-adjacency sparsity of H, diagonal included, ascending columns;
 //  * the element -> slot map: the slot of block (tets[e][k], tets[e][l]);
-//  * the same map inverted and sorted by slot (then by tet), which the
-//    numeric assembly reduces with warp shuffles; whole slots are packed into
-//    warp-sized chunks so no slot is split between warps.
+//  * the same map inverted and sorted by slot (then by tet) for the diagonal
+//    and upper slots, which the numeric assembly reduces with warp shuffles
+//    and mirrors; whole slots are packed into warp-sized chunks so no slot is
+//    split between warps.
 #include <algorithm>
 #include <cstring>
 
@@ -167,21 +168,31 @@ bool build_tri_slots(int n, int n_tris, const int32_t *tris, const int32_t *row_
     return true;
 }
 
-bool build_contributions(int n, int T, const int32_t *tets, const int32_t *row_ptr, const int32_t *slots,
+bool build_contributions(int n, int T, const int32_t *row_ptr, const int32_t *slots,
                          Symbolic &sym, std::string &err, int n_tris, const int32_t *tri_slots) {
-    (void)tets;
     const int64_t nnzb = row_ptr[n];
     if ((int64_t)T * 16 + (int64_t)n_tris * 9 > (int64_t)INT32_MAX) {
         err = "too many tets and tris for 32-bit contribution codes";
         return false;
     }
-    std::vector<int32_t> count(nnzb + 1, 0);
-    for (int64_t i = 0; i < (int64_t)T * 16; ++i) count[slots[i] + 1]++;
-    for (int64_t i = 0; i < (int64_t)n_tris * 9; ++i) count[tri_slots[i] + 1]++;
+    // Contribution (k, l) of an element with slots S (N x N) is kept where
+    // slot (k, l) <= slot (l, k): rows ascend with the slots, so these are the
+    // diagonal and the upper triangle of H.
+    std::vector<int32_t> start(nnzb + 1, 0), mate(nnzb, 0);
+    auto count = [&](const int32_t *S, int N) {
+        for (int k = 0; k < N; ++k)
+            for (int l = 0; l < N; ++l) {
+                const int32_t s = S[k * N + l], m = S[l * N + k];
+                if (s > m) continue;
+                start[s + 1]++;
+                mate[s] = m;
+            }
+    };
+    for (int64_t e = 0; e < T; ++e) count(slots + 16 * e, 4);
+    for (int64_t t = 0; t < n_tris; ++t) count(tri_slots + 9 * t, 3);
     // a vertex without tets still owns its diagonal block (mass + attachment):
     // give it one empty contribution so the assembly visits it
-    std::vector<int32_t> isolated;  // vertices in no tet
-    std::vector<int32_t> isolated_slot;
+    std::vector<int32_t> isolated;  // diagonal slots of vertices in no tet
     for (int v = 0; v < n; ++v) {
         const int32_t *b = sym.col_idx.data() + row_ptr[v];
         const int32_t *e = sym.col_idx.data() + row_ptr[v + 1];
@@ -191,63 +202,54 @@ bool build_contributions(int n, int T, const int32_t *tets, const int32_t *row_p
             return false;
         }
         const int32_t ds = (int32_t)(p - sym.col_idx.data());
-        if (count[ds + 1] == 0) {
-            count[ds + 1] = 1;
-            isolated.push_back(v);
-            isolated_slot.push_back(ds);
+        mate[ds] = ~v;
+        if (start[ds + 1] == 0) {
+            start[ds + 1] = 1;
+            isolated.push_back(ds);
         }
     }
-    std::vector<int64_t> start(nnzb + 1, 0);
-    for (int64_t s = 0; s < nnzb; ++s) start[s + 1] = start[s] + count[s + 1];
-    const int64_t total = start[nnzb];
-    if (total > (int64_t)INT32_MAX) {
+    if ((int64_t)T * 16 + (int64_t)n_tris * 9 + (int64_t)isolated.size() > (int64_t)INT32_MAX) {
         err = "too many contributions";
         return false;
     }
-    sym.contrib_code.assign(total, 0);
-    sym.contrib_slot.assign(total, 0);
-    std::vector<int64_t> fill(start.begin(), start.end() - 1);
-    for (size_t i = 0; i < isolated.size(); ++i) {
-        const int32_t s = isolated_slot[i];
-        sym.contrib_code[fill[s]] = -(isolated[i] + 1);
-        sym.contrib_slot[fill[s]] = s;
-        fill[s]++;
+    for (int64_t s = 0; s < nnzb; ++s) start[s + 1] += start[s];
+    sym.contrib_code.resize(start[nnzb]);
+    std::vector<int32_t> fill(start.begin(), start.end() - 1);
+    for (int32_t s : isolated) sym.contrib_code[fill[s]++] = mate[s];
+    for (int64_t e = 0; e < T; ++e) {
+        const int32_t *S = slots + 16 * e;
+        for (int k = 0; k < 4; ++k)
+            for (int l = 0; l < 4; ++l)
+                if (S[k * 4 + l] <= S[l * 4 + k]) sym.contrib_code[fill[S[k * 4 + l]]++] = (int32_t)(e * 16 + k * 4 + l);
     }
-    for (int e = 0; e < T; ++e)
-        for (int kl = 0; kl < 16; ++kl) {
-            const int32_t s = slots[(int64_t)e * 16 + kl];
-            const int64_t pos = fill[s]++;
-            sym.contrib_code[pos] = e * 16 + kl;
-            sym.contrib_slot[pos] = s;
-        }
     // surface-tri contact blocks (i, j) after the tets of their slot, coded
     // 16 T + 9 tri + 3 i + j
-    for (int t = 0; t < n_tris; ++t)
-        for (int ij = 0; ij < 9; ++ij) {
-            const int32_t s = tri_slots[(int64_t)t * 9 + ij];
-            const int64_t pos = fill[s]++;
-            sym.contrib_code[pos] = 16 * T + 9 * t + ij;
-            sym.contrib_slot[pos] = s;
-        }
+    for (int64_t t = 0; t < n_tris; ++t) {
+        const int32_t *S = tri_slots + 9 * t;
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j)
+                if (S[i * 3 + j] <= S[j * 3 + i])
+                    sym.contrib_code[fill[S[i * 3 + j]]++] = (int32_t)(16 * (int64_t)T + 9 * t + i * 3 + j);
+    }
     // pack whole slots into chunks of <= 32 contributions (a longer slot gets
     // a chunk of its own)
-    sym.chunk_ptr.clear();
-    sym.chunk_ptr.push_back(0);
-    int64_t chunk_len = 0;
+    sym.chunk.clear();
+    sym.pair.clear();
+    int4 c = {0, 0, 0, 0};
+    auto close = [&] {
+        if (c.y > c.x) sym.chunk.push_back(c);
+        c = {c.y, c.y, (int32_t)sym.pair.size(), 0};
+    };
     for (int64_t s = 0; s < nnzb; ++s) {
-        const int64_t len = start[s + 1] - start[s];
+        const int32_t len = start[s + 1] - start[s];
         if (len == 0) continue;
-        if (chunk_len > 0 && chunk_len + len > 32) {
-            sym.chunk_ptr.push_back((int32_t)start[s]);
-            chunk_len = 0;
-        }
-        chunk_len += len;
-        if (chunk_len >= 32) {
-            sym.chunk_ptr.push_back((int32_t)start[s + 1]);
-            chunk_len = 0;
-        }
+        if (c.y - c.x + len > 32) close();
+        c.w |= (int32_t)(1u << (c.y - c.x));
+        c.y += len;
+        sym.pair.push_back(int2{(int32_t)s, mate[s]});
+        if (c.y - c.x >= 32) close();
     }
-    if (chunk_len > 0) sym.chunk_ptr.push_back((int32_t)total);
+    close();
     return true;
 }
 
