@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     float4 *halo_w = win + a.nown_max + a.nhalo_max;                        // [2][nhalo_max] pushed by the owners
     float4 *trips_s = halo_w + (SCOPE == kCluster ? 2 * a.nhalo_max : 0);   // [warps][smem_trips][80]
     float *minv_s = reinterpret_cast<float *>(trips_s + (size_t)kPartWarps * a.smem_trips * kTripFloats4);
-    int *push_s = reinterpret_cast<int *>(minv_s + (RS > 1 ? 9 * (a.nown_max + a.nhalo_max) : 0));
+    int *push_s = reinterpret_cast<int *>(minv_s + (RS > 1 ? 9 * max(0, a.nown_max + a.nhalo_max - kPartThreads) : 0));
     // ORDERED: r, u and w of the own rows, component by component
     float *const own_r = reinterpret_cast<float *>(push_s + a.push_max), *const own_u = own_r + 3 * a.nown_max,
                  *const own_w = own_u + 3 * a.nown_max;
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
 #pragma unroll
             for (int i = 0; i < 9; ++i) {
                 if (j == 0) minv[i] = m[i];
-                else minv_s[9 * l + i] = m[i];
+                else minv_s[9 * (l - kPartThreads) + i] = m[i];
             }
             if (!inner) {
 #pragma unroll
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 ntrips[o] |= (unsigned)(t1 - t0) << (8 * qq);
                 auto fetch = [&](int t, float h[9], int &c) {
                     const int src = a.v.src[(size_t)32 * t + lane];
-                    c = a.v.col[(size_t)32 * t + lane];
+                    c = trip_column(src, a.v.col[(size_t)32 * t + lane], lane);
                     if (src >= 0) {
                         load_block9(a.values, src, h);
                     } else {
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 for (int c = 0; c < 3; ++c) r[j][c] = v[c];
             }
             float z[3];
-            precond(j > 0 ? minv_s + 9 * l : minv, r[j], z, a.use_precond);
+            precond(j > 0 ? minv_s + 9 * (l - kPartThreads) : minv, r[j], z, a.use_precond);
             win[l] = make_float4(z[0], z[1], z[2], 0.0f);
             if (j < OS) {
 #pragma unroll
@@ -760,7 +760,7 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     const int trips = regs ? h.trips_max_reg : h.trips_max;
     const size_t most = (size_t)optin - fa.sharedSizeBytes;
     const size_t base = sizeof(float4) * ((size_t)h.nown_max + (!grid && cluster > 1 ? 3 : 1) * (size_t)h.nhalo_max) +
-                        (L.row_slots > 1 ? 9 * sizeof(float) * ((size_t)h.nown_max + h.nhalo_max) : 0) +
+                        (L.row_slots > 1 ? 9 * sizeof(float) * (size_t)std::max(0, h.nown_max + h.nhalo_max - kPartThreads) : 0) +
                         (!grid && cluster > 1 ? sizeof(int) * (size_t)h.push_max : 0) +
                         (L.blocks > 0 ? 9 * sizeof(float) * (size_t)h.nown_max : 0) + 16;
     const size_t per_trip = sizeof(float4) * kTripFloats4 * kPartWarps;

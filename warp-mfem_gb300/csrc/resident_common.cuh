@@ -79,6 +79,14 @@ __device__ __forceinline__ void block_mac(const float h[9], const float4 v, floa
     a[2] += h[6] * v.x + h[7] * v.y + h[8] * v.z;
 }
 
+// The window column of a lane of a trip: a lane without a block (src < 0)
+// reads, times zero, with another lane of its quarter warp, which costs no
+// bank conflict of its own.
+__device__ __forceinline__ int trip_column(int src, int c, int lane) {
+    const unsigned with = __ballot_sync(0xffffffffu, src >= 0) & (0xffu << (lane & 24));
+    return __shfl_sync(0xffffffffu, c, src >= 0 || with == 0 ? lane : __ffs(with) - 1);
+}
+
 // The warp's sums of v[0..2], each added in the order of a shuffle-down tree
 // (lane i takes lane i + 16, then + 8, ...): lanes 0, 16 and 8 return the sums
 // of v[0], v[1] and v[2].  Each exchange halves what a lane carries, so three
