@@ -56,6 +56,13 @@ constexpr int kIrThreads = 512;
 constexpr int kIrGroup = 4;  // lanes per block row in the product
 constexpr int kIrDepth = 4;  // blocks per lane and loop trip in the product
 constexpr int kResThreads = 256;
+// Lanes per block row of the residual.  The kernel is a chain of latencies
+// (product, block sums, ticket, the last block's totals and decision) on a
+// narrow fp64 pipe: at 9,126 rows 29 us with four lanes a row, one thread's sum
+// of the block partials and three components' fp64 work in one lane; 18 us with
+// eight lanes and the last block's threads sharing the partials; 15 us with a
+// lane a component and the state words read ahead.
+constexpr int kResGroup = 8;
 constexpr long long kIrWaitCycles = 8000000000ll;
 
 template <class T>
@@ -133,9 +140,9 @@ __global__ void __launch_bounds__(kResThreads)
     const size_t vec = (size_t)3 * vv.n;
     const float2 *xo = w.dx_pair + (size_t)par * vec;
     float2 *xn = w.dx_pair + (size_t)(par ^ 1) * vec;
-    const int g_lane = threadIdx.x & (kIrGroup - 1);
-    const unsigned gmask = ((1u << kIrGroup) - 1u) << (threadIdx.x & (32 - kIrGroup));
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) / kIrGroup;
+    const int g_lane = threadIdx.x & (kResGroup - 1);
+    const unsigned gmask = ((1u << kResGroup) - 1u) << (threadIdx.x & (32 - kResGroup));
+    const int row = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / kResGroup);
     // the iterate of row c: the warm start after a restart, else the last
     // iterate plus the pending inner correction
     auto iterate = [&](int c, int q) -> float2 {
@@ -146,69 +153,99 @@ __global__ void __launch_bounds__(kResThreads)
     double rr = 0.0, gg = 0.0;
     if (row < vv.n) {
         float2 acc[3] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-        for (int k = bv.row_ptr[row] + g_lane; k < bv.row_ptr[row + 1]; k += kIrGroup) {
-            const int c = bv.col_idx[k];
-            float2 xc[3];
+        // two blocks a lane at a time, their loads together
+        const int ke = bv.row_ptr[row + 1];
+        for (int k = bv.row_ptr[row] + g_lane; k < ke; k += 2 * kResGroup) {
+            const bool two = k + kResGroup < ke;
+            const int k1 = two ? k + kResGroup : k;
+            const int c0 = bv.col_idx[k], c1 = bv.col_idx[k1];
+            float2 x0[3], x1[3];
+            float h0[9], h1[9];
 #pragma unroll
-            for (int q = 0; q < 3; ++q) xc[q] = iterate(c, q);
-            const float *h = bv.values + (size_t)9 * k;
+            for (int i = 0; i < 9; ++i) {
+                h0[i] = bv.values[(size_t)9 * k + i];
+                h1[i] = two ? bv.values[(size_t)9 * k1 + i] : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                x0[q] = iterate(c0, q);
+                x1[q] = iterate(c1, q);
+            }
 #pragma unroll
             for (int a = 0; a < 3; ++a)
 #pragma unroll
-                for (int q = 0; q < 3; ++q) df_fma(acc[a], h[3 * a + q], xc[q]);
-        }
+                for (int q = 0; q < 3; ++q) df_fma(acc[a], h0[3 * a + q], x0[q]);
+            if (two) {
 #pragma unroll
-        for (int off = kIrGroup / 2; off > 0; off >>= 1)
+                for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int a = 0; a < 3; ++a) acc[a] = df_add(acc[a], df_shfl_xor(gmask, acc[a], off));
-        if (g_lane == 0) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float2 xr = iterate(row, a);
-                xn[3 * row + a] = xr;
-                w.dx_out[3 * row + a] = (double)xr.x + (double)xr.y;
-                vv.dx[3 * row + a] = __fadd_rn(xr.x, xr.y);
-                // r = g - (acc.hi + acc.lo), as a pair, then its double value
-                const float gq = vv.rhs[3 * row + a];
-                const double r = df_residual(gq, acc[a]);
-                w.res[3 * row + a] = (float)r;
-                rr += r * r;
-                gg += (double)gq * (double)gq;
+                    for (int q = 0; q < 3; ++q) df_fma(acc[a], h1[3 * a + q], x1[q]);
             }
         }
-    }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        rr += __shfl_down_sync(0xffffffffu, rr, off);
-        gg += __shfl_down_sync(0xffffffffu, gg, off);
+        for (int off = kResGroup / 2; off > 0; off >>= 1)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) acc[a] = df_add(acc[a], df_shfl_xor(gmask, acc[a], off));
+        // a lane a component: the fp64 pipe takes 16 cycles a warp instruction
+        // however few lanes it has
+        if (g_lane < 3) {
+            const float2 sum = g_lane == 0 ? acc[0] : g_lane == 1 ? acc[1] : acc[2];
+            const int i = 3 * row + g_lane;
+            const float2 xr = iterate(row, g_lane);
+            xn[i] = xr;
+            w.dx_out[i] = (double)xr.x + (double)xr.y;
+            vv.dx[i] = __fadd_rn(xr.x, xr.y);
+            // r = g - (sum.hi + sum.lo), as a pair, then its double value
+            const float gq = vv.rhs[i];
+            const double r = df_residual(gq, sum);
+            w.res[i] = (float)r;
+            rr = r * r;
+            gg = (double)gq * (double)gq;
+        }
     }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) {
-        s_red[0][wid] = rr;
-        s_red[1][wid] = gg;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a0 = 0.0, a1 = 0.0;
-        for (int k = 0; k < kResThreads / 32; ++k) {
-            a0 += s_red[0][k];
-            a1 += s_red[1][k];
+    // the block's sums of rr and gg, in thread 0
+    auto block_sums = [&] {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            rr += __shfl_down_sync(0xffffffffu, rr, off);
+            gg += __shfl_down_sync(0xffffffffu, gg, off);
         }
-        w.res_partials[2 * blockIdx.x + 0] = a0;
-        w.res_partials[2 * blockIdx.x + 1] = a1;
+        if (lane == 0) {
+            s_red[0][wid] = rr;
+            s_red[1][wid] = gg;
+        }
+        __syncthreads();
+        rr = gg = 0.0;
+        if (threadIdx.x == 0)
+            for (int k = 0; k < kResThreads / 32; ++k) {
+                rr += s_red[0][k];
+                gg += s_red[1][k];
+            }
+    };
+    block_sums();
+    if (threadIdx.x == 0) {
+        w.res_partials[2 * blockIdx.x + 0] = rr;
+        w.res_partials[2 * blockIdx.x + 1] = gg;
         __threadfence();
         s_last = atomicAdd(w.ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
-    // the last block: fixed-order totals and the decision
+    // the last block: the partials in a fixed order, by all its threads (one
+    // thread's chain of loads and fp64 adds took most of the kernel), and the
+    // decision
+    __threadfence();
+    const int outer = w.state[1], inner_its = w.state[2], error = w.state[5], full = w.state[6];
+    const double best = *w.best;
+    rr = gg = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kResThreads) {
+        rr += __ldcg(w.res_partials + 2 * b);
+        gg += __ldcg(w.res_partials + 2 * b + 1);
+    }
+    block_sums();
     if (threadIdx.x == 0) {
-        __threadfence();
-        double trr = 0.0, tgg = 0.0;
-        for (int b = 0; b < (int)gridDim.x; ++b) {
-            trr += __ldcg(w.res_partials + 2 * b);
-            tgg += __ldcg(w.res_partials + 2 * b + 1);
-        }
+        const double trr = rr, tgg = gg;
         const double rel = tgg > 0.0 ? sqrt(trr / tgg) : sqrt(trr);
         // the scale of the next inner right-hand side (unit norm: fp32 sums
         // of products of a tiny residual's entries would underflow)
@@ -217,17 +254,13 @@ __global__ void __launch_bounds__(kResThreads)
         const bool scaled = rn > 0.0 && isfinite(rn) && isfinite(inv);
         w.scale[0] = scaled ? inv : 1.0f;
         w.scale[1] = scaled ? (float)rn : 1.0f;
-        const int outer = w.state[1];
         int status = MFEM_OK;
         int done = 0;
-        const double best = *w.best;
-        w.state[7] = 0;
-        if (w.state[6] == 0 && isfinite(best) && !(rel <= 4.0 * best) && outer < w.outer_max) {
+        const bool again = full == 0 && isfinite(best) && !(rel <= 4.0 * best) && outer < w.outer_max;
+        if (again) {
             // diverging on the 16-bit H: restart from the warm start with
             // the fp32 H (the next inner PCG is skipped; the next residual
             // pass reads the warm start)
-            w.state[6] = 1;
-            w.state[7] = 1;
         } else if (!isfinite(rel)) {
             status = MFEM_NONFINITE;
             done = 1;
@@ -237,14 +270,17 @@ __global__ void __launch_bounds__(kResThreads)
             status = MFEM_MAXITER;
             done = 1;
         }
-        if (isfinite(rel) && rel < best && w.state[7] == 0) *w.best = rel;
+        if (isfinite(rel) && rel < best && !again) *w.best = rel;
         w.state[1] = outer + 1;
         w.state[3] = 0;
         w.state[4] = par ^ 1;
         w.state[0] = done;
-        if (w.state[5] == MFEM_OK) w.state[5] = status;
-        w.stats[slot] = IrStats{outer, w.state[2], w.state[5], w.state[6], rel};
-        pw.stats[slot] = SolveStats{w.state[2], w.state[5], (float)rel, 0.0f};
+        w.state[6] = again ? 1 : full;
+        w.state[7] = again;
+        const int result = error == MFEM_OK ? status : error;
+        w.state[5] = result;
+        w.stats[slot] = IrStats{outer, inner_its, result, again ? 1 : full, rel};
+        pw.stats[slot] = SolveStats{inner_its, result, (float)rel, 0.0f};
         *w.ticket = 0u;
     }
 }
@@ -670,7 +706,7 @@ cudaError_t ir_max_ctas(int device, int *ctas) {
     return cudaSuccess;
 }
 
-int ir_residual_blocks(int n) { return std::max(1, blocks_for(n * kIrGroup, kResThreads)); }
+int ir_residual_blocks(int n) { return std::max(1, (int)(((long long)n * kResGroup + kResThreads - 1) / kResThreads)); }
 
 cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const IrWork &w, const PcgWork &pw,
                                const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single,
