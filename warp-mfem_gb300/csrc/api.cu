@@ -433,30 +433,43 @@ void batch_schedule(const std::vector<int32_t> &nnzb, const std::vector<int32_t>
     ctas = capacity;
 }
 
-// Uploads a host partition; its arrays live in `allocs`.
+// Uploads a host partition in one allocation, which lives in `allocs`.
 cudaError_t upload_resident(std::vector<void *> &allocs, const ResidentHost &h, ResidentViews &v) {
-    cudaError_t e = cudaSuccess;
-    auto put = [&](auto **dst, const auto &src) {
-        if (e != cudaSuccess) return;
-        void *raw = nullptr;
-        e = cudaMalloc(&raw, std::max<size_t>(src.size() * sizeof(src[0]), 16));
-        if (e != cudaSuccess) return;
-        allocs.push_back(raw);
-        if (!src.empty()) e = cudaMemcpy(raw, src.data(), src.size() * sizeof(src[0]), cudaMemcpyHostToDevice);
-        *dst = static_cast<std::remove_reference_t<decltype(*dst)>>(raw);
+    std::vector<unsigned char> all;
+    void *raw = nullptr;
+    // twice: gather the arrays, 256-byte aligned; then set the views
+    auto arrays = [&](const auto &put) {
+        size_t at = 0;
+        auto one = [&](auto **dst, const auto &src) {
+            put(dst, src, at);
+            at += (src.size() * sizeof(src[0]) + 255) & ~(size_t)255;
+        };
+        one(&v.parts, h.parts);
+        one(&v.tasks, h.tasks);
+        one(&v.rows, h.rows);
+        one(&v.halo, h.halo);
+        one(&v.trip_ptr, h.trip_ptr);
+        one(&v.src, h.src);
+        one(&v.col, h.col);
+        one(&v.push, h.push);
+        one(&v.ftrip_ptr, h.ftrip_ptr);
+        one(&v.fsrc, h.fsrc);
+        one(&v.fcol, h.fcol);
+        one(&v.fpush, h.fpush);
+        return at;
     };
-    put(&v.parts, h.parts);
-    put(&v.tasks, h.tasks);
-    put(&v.rows, h.rows);
-    put(&v.halo, h.halo);
-    put(&v.trip_ptr, h.trip_ptr);
-    put(&v.src, h.src);
-    put(&v.col, h.col);
-    put(&v.push, h.push);
-    put(&v.ftrip_ptr, h.ftrip_ptr);
-    put(&v.fsrc, h.fsrc);
-    put(&v.fcol, h.fcol);
-    put(&v.fpush, h.fpush);
+    const size_t bytes = std::max<size_t>(arrays([](auto **, const auto &, size_t) {}), 256);
+    all.resize(bytes);
+    arrays([&](auto **, const auto &src, size_t at) {
+        if (!src.empty()) std::memcpy(all.data() + at, src.data(), src.size() * sizeof(src[0]));
+    });
+    cudaError_t e = cudaMalloc(&raw, bytes);
+    if (e != cudaSuccess) return e;
+    allocs.push_back(raw);
+    e = cudaMemcpy(raw, all.data(), bytes, cudaMemcpyHostToDevice);
+    arrays([&](auto **dst, const auto &, size_t at) {
+        *dst = reinterpret_cast<std::remove_reference_t<decltype(*dst)>>(static_cast<unsigned char *>(raw) + at);
+    });
     return e;
 }
 
@@ -653,7 +666,10 @@ int mfem_bsr_sparsity(int32_t n_particles, int32_t n_tets, const int32_t *h_tet_
                       int32_t *h_col_idx, int64_t *nnzb) {
     std::vector<int32_t> rp, ci;
     std::string err;
-    if (!build_sparsity(n_particles, n_tets, h_tet_indices, rp, ci, err)) return fail(nullptr, MFEM_BAD_ARG, err);
+    VertexTets vt;
+    if (!vertex_tets(n_particles, n_tets, h_tet_indices, vt, err) ||
+        !build_sparsity(n_particles, h_tet_indices, vt, rp, ci, err))
+        return fail(nullptr, MFEM_BAD_ARG, err);
     if (nnzb) *nnzb = (int64_t)ci.size();
     if (h_row_ptr) std::memcpy(h_row_ptr, rp.data(), rp.size() * sizeof(int32_t));
     if (h_col_idx && !ci.empty()) std::memcpy(h_col_idx, ci.data(), ci.size() * sizeof(int32_t));
@@ -664,7 +680,9 @@ int mfem_tet_slot_map(int32_t n_particles, int32_t n_tets, const int32_t *h_tet_
                       const int32_t *h_col_idx, int32_t *h_slots) {
     if (n_tets > 0 && (!h_row_ptr || !h_col_idx || !h_slots)) return fail(nullptr, MFEM_BAD_ARG, "NULL argument");
     std::string err;
-    if (!build_slot_map(n_particles, n_tets, h_tet_indices, h_row_ptr, h_col_idx, h_slots, err))
+    VertexTets vt;
+    if (!vertex_tets(n_particles, n_tets, h_tet_indices, vt, err) ||
+        !build_slot_map(n_particles, h_tet_indices, vt, h_row_ptr, h_col_idx, h_slots, err))
         return fail(nullptr, MFEM_BAD_ARG, err);
     return MFEM_OK;
 }
@@ -712,11 +730,13 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
             return fail(nullptr, MFEM_BAD_ARG, "particle_inv_mass must be finite and >= 0");
 
     Symbolic sym;
-    if (!build_sparsity(n, T, h_tets, sym.row_ptr, sym.col_idx, err)) return fail(nullptr, MFEM_BAD_ARG, err);
-    sym.tet_slots.resize((size_t)T * 16);
-    if (!build_slot_map(n, T, h_tets, sym.row_ptr.data(), sym.col_idx.data(), sym.tet_slots.data(), err))
+    VertexTets vt;
+    if (!vertex_tets(n, T, h_tets, vt, err) || !build_sparsity(n, h_tets, vt, sym.row_ptr, sym.col_idx, err))
         return fail(nullptr, MFEM_BAD_ARG, err);
-    if (!build_contributions(n, T, sym.row_ptr.data(), sym.tet_slots.data(), sym, err))
+    sym.tet_slots.resize((size_t)T * 16);
+    if (!build_slot_map(n, h_tets, vt, sym.row_ptr.data(), sym.col_idx.data(), sym.tet_slots.data(), err))
+        return fail(nullptr, MFEM_BAD_ARG, err);
+    if (!build_contributions(n, T, vt, sym.row_ptr.data(), sym.tet_slots.data(), sym, err))
         return fail(nullptr, MFEM_BAD_ARG, err);
 
     // (M + Q) diagonal: Hessian mass is identity on attached vertices and
@@ -1197,8 +1217,10 @@ int mfem_plan_set_contact(mfem_plan *p, const mfem_contact_config *cfg_in, int32
         return fail(p, MFEM_BAD_ARG, err);
     Symbolic sym;
     sym.col_idx = p->h_col_idx;
-    if (m > 0 && !build_contributions(p->n, p->T, p->h_row_ptr.data(), p->h_tet_slots.data(), sym,
-                                      err, m, tri_slots.data()))
+    VertexTets vt;
+    if (m > 0 && (!vertex_tets(p->n, p->T, p->h_tets.data(), vt, err) ||
+                  !build_contributions(p->n, p->T, vt, p->h_row_ptr.data(), p->h_tet_slots.data(), sym, err, m,
+                                       tri_slots.data())))
         return fail(p, MFEM_BAD_ARG, err);
 
     DeviceGuard g(p->device);

@@ -487,16 +487,23 @@ struct Symbolic {
     std::vector<int32_t> contrib_code;
     std::vector<int2> pair;
 };
-bool build_sparsity(int n, int T, const int32_t *tets, std::vector<int32_t> &row_ptr,
+// Tets of each vertex, ascending, as codes tet * 4 + corner; refuses tets
+// with a vertex out of range or repeated.
+struct VertexTets {
+    std::vector<int64_t> ptr;
+    std::vector<int32_t> code;
+};
+bool vertex_tets(int n, int T, const int32_t *tets, VertexTets &vt, std::string &err);
+bool build_sparsity(int n, const int32_t *tets, const VertexTets &vt, std::vector<int32_t> &row_ptr,
                     std::vector<int32_t> &col_idx, std::string &err);
-bool build_slot_map(int n, int T, const int32_t *tets, const int32_t *row_ptr, const int32_t *col_idx,
-                    int32_t *slots, std::string &err);
+bool build_slot_map(int n, const int32_t *tets, const VertexTets &vt, const int32_t *row_ptr,
+                    const int32_t *col_idx, int32_t *slots, std::string &err);
 // Slots of the 9 blocks (i, j) of each surface tri and the incident tri
 // corners (tri * 3 + corner) of each vertex.
 bool build_tri_slots(int n, int n_tris, const int32_t *tris, const int32_t *row_ptr, const int32_t *col_idx,
                      int32_t *tri_slots, std::vector<int32_t> &vt_ptr, std::vector<int32_t> &vt_code,
                      std::string &err);
-bool build_contributions(int n, int T, const int32_t *row_ptr,
+bool build_contributions(int n, int T, const VertexTets &vt, const int32_t *row_ptr,
                          const int32_t *slots, Symbolic &sym, std::string &err, int n_tris = 0,
                          const int32_t *tri_slots = nullptr);
 

@@ -8,55 +8,18 @@
 // parts, 124 rows a part, need 146 to 221 foreign rows against 310 for
 // contiguous row ranges of the x-major order (and nearly every row of the
 // mesh for a shuffled one).
+#include "host_parallel.h"
 #include "internal.h"
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdint>
-#include <exception>
 #include <memory>
-#include <mutex>
-#include <system_error>
-#include <thread>
 
 namespace mfem {
 namespace {
 
-constexpr int kMaxThreads = 8;
-constexpr int kThreadRows = 2048;  // a thread for every so many rows
-
-// Runs fn(i) for i in [0, count) on up to `threads` threads, this one
-// included; an exception of fn leaves here, as from a plain loop.
-template <class F>
-void parallel_for(int count, int threads, const F &fn) {
-    std::atomic<int> next{0};
-    std::exception_ptr failed;
-    std::mutex lock;
-    auto work = [&] {
-        try {
-            for (int i = next++; i < count; i = next++) fn(i);
-        } catch (...) {
-            std::lock_guard<std::mutex> hold(lock);
-            failed = std::current_exception();
-            next = count;
-        }
-    };
-    std::vector<std::thread> pool;
-    pool.reserve(std::max(0, std::min(threads, count) - 1));
-    try {
-        for (int t = 1; t < std::min(threads, count); ++t) pool.emplace_back(work);
-    } catch (const std::system_error &) {  // no more threads: the ones there are do it
-    }
-    work();
-    for (auto &t : pool) t.join();
-    if (failed) std::rethrow_exception(failed);
-}
-
-int thread_count(int rows) {
-    const int hw = (int)std::thread::hardware_concurrency();
-    return std::max(1, std::min(std::min(kMaxThreads, hw), rows / kThreadRows));
-}
+constexpr int kThreadRows = 768;  // 0.5 to 1 us of work a row
 
 struct Bisector {
     const float *q;  // [n][3]
@@ -289,7 +252,7 @@ void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *c
                        int row_lo, int row_hi, int parts, int body, bool push_lists, bool parallel,
                        const ResidentFactor *factor) {
     const int n = row_hi - row_lo;
-    const int threads = parallel ? thread_count(n) : 1;
+    const int threads = parallel ? thread_count(n, kThreadRows) : 1;
     std::vector<int> rows(n), bounds(parts + 1, 0);
     for (int i = 0; i < n; ++i) rows[i] = row_lo + i;
     Bisector{rest_q}.split(rows, parts, bounds, threads);
@@ -302,7 +265,7 @@ void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t 
     for (int i = 0; i < n; ++i) rows[i] = i;
     const int first_part = (int)h.parts.size();
     for (int p = 1; p <= parts; ++p) bounds[p] = (int)((int64_t)n * ((int64_t)blocks * p / parts) / blocks);
-    add_parts(h, row_ptr, col_idx, 0, 0, rows, bounds, push_lists, thread_count(n), nullptr, true);
+    add_parts(h, row_ptr, col_idx, 0, 0, rows, bounds, push_lists, thread_count(n, kThreadRows), nullptr, true);
     h.blocks = blocks;
     for (int p = 0; p < parts; ++p) {
         ResPart &rp = h.parts[first_part + p];
@@ -497,7 +460,7 @@ void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t 
     std::vector<ResidentHost> made(bodies.size());
     int rows = 0;
     for (int b : bodies) rows += row_off[b + 1] - row_off[b];
-    parallel_for((int)bodies.size(), thread_count(rows), [&](int i) {
+    parallel_for((int)bodies.size(), thread_count(rows, kThreadRows), [&](int i) {
         const int b = bodies[i];
         resident_add_body(made[i], row_ptr, col_idx, rest_q, row_off[b], row_off[b + 1], parts, b, parts > 1, false,
                           factor);

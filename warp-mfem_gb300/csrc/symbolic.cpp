@@ -14,9 +14,12 @@
 #include <algorithm>
 #include <cstring>
 
+#include "host_parallel.h"
 #include "internal.h"
 
 namespace mfem {
+
+constexpr int kThreadRows = 1024;  // 0.1 to 0.5 us of work a row in each pass
 
 static bool check_tets(int n, int T, const int32_t *tets, std::string &err) {
     if (n < 0 || T < 0) {
@@ -50,83 +53,99 @@ static bool check_tets(int n, int T, const int32_t *tets, std::string &err) {
     return true;
 }
 
-// Tets of each vertex, ascending, as codes tet * 4 + corner (a counting sort).
-static void vertex_tets(int n, int T, const int32_t *tets, std::vector<int64_t> &vptr, std::vector<int32_t> &vcode) {
-    vptr.assign((size_t)n + 1, 0);
-    for (int64_t i = 0; i < (int64_t)T * 4; ++i) vptr[tets[i] + 1]++;
-    for (int v = 0; v < n; ++v) vptr[v + 1] += vptr[v];
-    vcode.assign((size_t)T * 4, 0);
-    std::vector<int64_t> fill(vptr.begin(), vptr.end() - 1);
-    for (int64_t i = 0; i < (int64_t)T * 4; ++i) vcode[fill[tets[i]]++] = (int32_t)i;
-}
-
-bool build_sparsity(int n, int T, const int32_t *tets, std::vector<int32_t> &row_ptr, std::vector<int32_t> &col_idx,
-                    std::string &err) {
+bool vertex_tets(int n, int T, const int32_t *tets, VertexTets &vt, std::string &err) {
     if (!check_tets(n, T, tets, err)) return false;
-    // per row: the diagonal and the vertices of the row's tets, made unique
-    // with a stamp array and sorted (a few dozen columns a row)
-    std::vector<int64_t> vptr;
-    std::vector<int32_t> vcode;
-    vertex_tets(n, T, tets, vptr, vcode);
-    std::vector<int32_t> stamp((size_t)n, -1);
-    std::vector<int32_t> row;
-    row_ptr.assign((size_t)n + 1, 0);
-    col_idx.clear();
-    col_idx.reserve((size_t)T * 4 + (size_t)n);
-    for (int v = 0; v < n; ++v) {
-        row.clear();
-        stamp[v] = v;
-        row.push_back(v);
-        for (int64_t i = vptr[v]; i < vptr[v + 1]; ++i) {
-            const int32_t *t = tets + 4 * (int64_t)(vcode[i] >> 2);
-            for (int l = 0; l < 4; ++l)
-                if (stamp[t[l]] != v) {
-                    stamp[t[l]] = v;
-                    row.push_back(t[l]);
-                }
-        }
-        std::sort(row.begin(), row.end());
-        col_idx.insert(col_idx.end(), row.begin(), row.end());
-        if (col_idx.size() > (size_t)INT32_MAX) {
-            err = "sparsity exceeds 2^31 blocks";
-            return false;
-        }
-        row_ptr[v + 1] = (int32_t)col_idx.size();
-    }
+    vt.ptr.assign((size_t)n + 1, 0);
+    for (int64_t i = 0; i < (int64_t)T * 4; ++i) vt.ptr[tets[i] + 1]++;
+    for (int v = 0; v < n; ++v) vt.ptr[v + 1] += vt.ptr[v];
+    vt.code.resize((size_t)T * 4);
+    std::vector<int64_t> fill(vt.ptr.begin(), vt.ptr.end() - 1);
+    for (int64_t i = 0; i < (int64_t)T * 4; ++i) vt.code[fill[tets[i]]++] = (int32_t)i;
     return true;
 }
 
-bool build_slot_map(int n, int T, const int32_t *tets, const int32_t *row_ptr, const int32_t *col_idx, int32_t *slots,
-                    std::string &err) {
-    if (!check_tets(n, T, tets, err)) return false;
+bool build_sparsity(int n, const int32_t *tets, const VertexTets &vt, std::vector<int32_t> &row_ptr,
+                    std::vector<int32_t> &col_idx, std::string &err) {
+    const auto &vptr = vt.ptr;
+    const auto &vcode = vt.code;
+    // per row: the diagonal and the vertices of the row's tets, made unique
+    // with a stamp array and sorted (a few dozen columns a row)
+    row_ptr.assign((size_t)n + 1, 0);
+    const int threads = thread_count(n, kThreadRows);
+    std::vector<std::vector<int32_t>> cols(threads);
+    parallel_rows(n, threads, [&](int block, int first, int last) {
+        std::vector<int32_t> stamp((size_t)n, -1), row;
+        std::vector<int32_t> &out = cols[block];
+        out.reserve((size_t)((vptr[last] - vptr[first]) + (last - first)));
+        for (int v = first; v < last; ++v) {
+            row.clear();
+            stamp[v] = v;
+            row.push_back(v);
+            for (int64_t i = vptr[v]; i < vptr[v + 1]; ++i) {
+                const int32_t *t = tets + 4 * (int64_t)(vcode[i] >> 2);
+                for (int l = 0; l < 4; ++l)
+                    if (stamp[t[l]] != v) {
+                        stamp[t[l]] = v;
+                        row.push_back(t[l]);
+                    }
+            }
+            std::sort(row.begin(), row.end());
+            out.insert(out.end(), row.begin(), row.end());
+            row_ptr[v + 1] = (int32_t)row.size();
+        }
+    });
+    size_t total = 0;
+    for (const auto &c : cols) total += c.size();
+    if (total > (size_t)INT32_MAX) {
+        err = "sparsity exceeds 2^31 blocks";
+        return false;
+    }
+    for (int v = 0; v < n; ++v) row_ptr[v + 1] += row_ptr[v];
+    col_idx.resize(total);
+    parallel_rows(n, threads, [&](int block, int first, int) {
+        std::copy(cols[block].begin(), cols[block].end(), col_idx.begin() + row_ptr[first]);
+    });
+    return true;
+}
+
+bool build_slot_map(int n, const int32_t *tets, const VertexTets &vt, const int32_t *row_ptr, const int32_t *col_idx,
+                    int32_t *slots, std::string &err) {
+    const auto &vptr = vt.ptr;
+    const auto &vcode = vt.code;
     // per row: each column's slot through a stamped position array, then
     // the slots of the row's tet corners
-    std::vector<int64_t> vptr;
-    std::vector<int32_t> vcode;
-    vertex_tets(n, T, tets, vptr, vcode);
-    std::vector<int32_t> stamp((size_t)n, -1), pos((size_t)n, 0);
-    for (int v = 0; v < n; ++v) {
-        for (int32_t j = row_ptr[v]; j < row_ptr[v + 1]; ++j) {
-            const int32_t c = col_idx[j];
-            if (c < 0 || c >= n) {
-                err = "column index out of range in row " + std::to_string(v);
-                return false;
-            }
-            stamp[c] = v;
-            pos[c] = j;
-        }
-        for (int64_t i = vptr[v]; i < vptr[v + 1]; ++i) {
-            const int32_t e = vcode[i] >> 2, k = vcode[i] & 3;
-            const int32_t *t = tets + 4 * (int64_t)e;
-            for (int l = 0; l < 4; ++l) {
-                if (stamp[t[l]] != v) {
-                    err = "sparsity lacks block (" + std::to_string(v) + ", " + std::to_string(t[l]) + ")";
-                    return false;
+    const int threads = thread_count(n, kThreadRows);
+    std::vector<std::string> errs(threads);
+    parallel_rows(n, threads, [&](int block, int first, int last) {
+        std::vector<int32_t> stamp((size_t)n, -1), pos((size_t)n, 0);
+        for (int v = first; v < last; ++v) {
+            for (int32_t j = row_ptr[v]; j < row_ptr[v + 1]; ++j) {
+                const int32_t c = col_idx[j];
+                if (c < 0 || c >= n) {
+                    errs[block] = "column index out of range in row " + std::to_string(v);
+                    return;
                 }
-                slots[(int64_t)e * 16 + k * 4 + l] = pos[t[l]];
+                stamp[c] = v;
+                pos[c] = j;
+            }
+            for (int64_t i = vptr[v]; i < vptr[v + 1]; ++i) {
+                const int32_t e = vcode[i] >> 2, k = vcode[i] & 3;
+                const int32_t *t = tets + 4 * (int64_t)e;
+                for (int l = 0; l < 4; ++l) {
+                    if (stamp[t[l]] != v) {
+                        errs[block] = "sparsity lacks block (" + std::to_string(v) + ", " + std::to_string(t[l]) + ")";
+                        return;
+                    }
+                    slots[(int64_t)e * 16 + k * 4 + l] = pos[t[l]];
+                }
             }
         }
-    }
+    });
+    for (const std::string &e : errs)  // the first row's
+        if (!e.empty()) {
+            err = e;
+            return false;
+        }
     return true;
 }
 
@@ -168,7 +187,7 @@ bool build_tri_slots(int n, int n_tris, const int32_t *tris, const int32_t *row_
     return true;
 }
 
-bool build_contributions(int n, int T, const int32_t *row_ptr, const int32_t *slots,
+bool build_contributions(int n, int T, const VertexTets &vt, const int32_t *row_ptr, const int32_t *slots,
                          Symbolic &sym, std::string &err, int n_tris, const int32_t *tri_slots) {
     const int64_t nnzb = row_ptr[n];
     if ((int64_t)T * 16 + (int64_t)n_tris * 9 > (int64_t)INT32_MAX) {
@@ -177,23 +196,44 @@ bool build_contributions(int n, int T, const int32_t *row_ptr, const int32_t *sl
     }
     // Contribution (k, l) of an element with slots S (N x N) is kept where
     // slot (k, l) <= slot (l, k): rows ascend with the slots, so these are the
-    // diagonal and the upper triangle of H.
+    // diagonal and the upper triangle of H.  A tet's corners are distinct, so
+    // the contributions to a row's slots are those of the row's tets, one
+    // corner each: rows are independent.
+    const auto &vptr = vt.ptr;
+    const auto &vcode = vt.code;
+    const int threads = thread_count(n, kThreadRows);
     std::vector<int32_t> start(nnzb + 1, 0), mate(nnzb, 0);
-    auto count = [&](const int32_t *S, int N) {
-        for (int k = 0; k < N; ++k)
-            for (int l = 0; l < N; ++l) {
-                const int32_t s = S[k * N + l], m = S[l * N + k];
+    const auto row_contributions = [&](int v, const auto &keep) {
+        for (int64_t i = vptr[v]; i < vptr[v + 1]; ++i) {
+            const int64_t e = vcode[i] >> 2;
+            const int k = vcode[i] & 3;
+            const int32_t *S = slots + 16 * e;
+            for (int l = 0; l < 4; ++l)
+                if (S[k * 4 + l] <= S[l * 4 + k]) keep(S[k * 4 + l], S[l * 4 + k], (int32_t)(16 * e + 4 * k + l));
+        }
+    };
+    parallel_rows(n, threads, [&](int, int first, int last) {
+        for (int v = first; v < last; ++v)
+            row_contributions(v, [&](int32_t s, int32_t m, int32_t) {
+                start[s + 1]++;
+                mate[s] = s == m ? ~v : m;
+            });
+    });
+    for (int64_t t = 0; t < n_tris; ++t) {
+        const int32_t *S = tri_slots + 9 * t;
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) {
+                const int32_t s = S[i * 3 + j], m = S[j * 3 + i];
                 if (s > m) continue;
                 start[s + 1]++;
-                mate[s] = m;
+                if (s != m) mate[s] = m;
             }
-    };
-    for (int64_t e = 0; e < T; ++e) count(slots + 16 * e, 4);
-    for (int64_t t = 0; t < n_tris; ++t) count(tri_slots + 9 * t, 3);
+    }
     // a vertex without tets still owns its diagonal block (mass + attachment):
     // give it one empty contribution so the assembly visits it
     std::vector<int32_t> isolated;  // diagonal slots of vertices in no tet
     for (int v = 0; v < n; ++v) {
+        if (vptr[v] < vptr[v + 1]) continue;  // its tets' diagonal blocks are in the slot map
         const int32_t *b = sym.col_idx.data() + row_ptr[v];
         const int32_t *e = sym.col_idx.data() + row_ptr[v + 1];
         const int32_t *p = std::lower_bound(b, e, v);
@@ -216,12 +256,10 @@ bool build_contributions(int n, int T, const int32_t *row_ptr, const int32_t *sl
     sym.contrib_code.resize(start[nnzb]);
     std::vector<int32_t> fill(start.begin(), start.end() - 1);
     for (int32_t s : isolated) sym.contrib_code[fill[s]++] = mate[s];
-    for (int64_t e = 0; e < T; ++e) {
-        const int32_t *S = slots + 16 * e;
-        for (int k = 0; k < 4; ++k)
-            for (int l = 0; l < 4; ++l)
-                if (S[k * 4 + l] <= S[l * 4 + k]) sym.contrib_code[fill[S[k * 4 + l]]++] = (int32_t)(e * 16 + k * 4 + l);
-    }
+    parallel_rows(n, threads, [&](int, int first, int last) {
+        for (int v = first; v < last; ++v)
+            row_contributions(v, [&](int32_t s, int32_t, int32_t code) { sym.contrib_code[fill[s]++] = code; });
+    });
     // surface-tri contact blocks (i, j) after the tets of their slot, coded
     // 16 T + 9 tri + 3 i + j
     for (int64_t t = 0; t < n_tris; ++t) {
