@@ -38,6 +38,7 @@ __device__ __forceinline__ void load_vec3(const float *__restrict__ p, int i, fl
 // 100 KB of straight-line code bound it, at 43% of the issue slots.
 constexpr int kElementWarps = kElementThreads / 32;
 constexpr int kElementSmem = kElementWarps * 32 * kKeRecord * (int)sizeof(float);
+constexpr int kElementOneWave = 3 * 152;
 // grid of the fp64 pass: it loops over however many tets were listed
 constexpr int kElementFp64Blocks = 304;
 
@@ -178,8 +179,12 @@ __device__ __forceinline__ float element_tet(const float *__restrict__ x, int en
 
 // One thread per tet, in float32; tets with det F < 1e-3 are listed for
 // element_fp64_kernel, which redoes them with the float64 polar path.
-template <bool DIAG>
-__global__ void __launch_bounds__(kElementThreads, 4)
+// BLOCKS: resident blocks an SM.  Four at 128 registers hide more latency than
+// three at 168 (126 us against 135 at 331,200 tets), but their spills lengthen
+// the one wave of a small mesh (14.1 us against 13.5 at 324 tets): three up to
+// the meshes that three an SM hold at once.
+template <bool DIAG, int BLOCKS>
+__global__ void __launch_bounds__(kElementThreads, BLOCKS)
     element_kernel(const float *__restrict__ x, int energy, TetViews tv) {
     extern __shared__ __align__(128) float s_stage[];
     const int T = tv.n_tets;
@@ -276,31 +281,36 @@ __device__ __forceinline__ void local_tet(const TetViews &tv, const float *__res
     const int T = tv.n_tets;
     const int4 tt = tv.tets[t];
     const int vid[4] = {tt.x, tt.y, tt.z, tt.w};
-    float u[6];
+    // every load of the tet before the first use, in 127 registers (at 40 the
+    // loads come in batches, each a latency of its own): 576 -> 549 us for a
+    // step of 324 tets with the one-wave element kernel, 0.2 to 0.8% on meshes
+    // whose PCG takes most of the step
+    float u[6], G[72], Hl[21], gs[6], d[4][3];
+#pragma unroll
+    for (int i = 0; i < 72; ++i) G[i] = tv.G[(size_t)i * T + t];
+#pragma unroll
+    for (int i = 0; i < 21; ++i) Hl[i] = tv.H_l[(size_t)i * T + t];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         u[i] = tv.c[(size_t)i * T + t];
+        gs[i] = tv.g_s[(size_t)i * T + t];
         gdx[i] = 0.0f;
     }
     // u = c - G dx, block by block (kernels.py:266-268)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float d[3];
-        load_vec3(dx, vid[k], d);
+    for (int k = 0; k < 4; ++k) load_vec3(dx, vid[k], d[k]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-            const float *g = tv.G + (size_t)(i * 12 + 3 * k) * T + t;
-            const float gd = g[0] * d[0] + g[(size_t)T] * d[1] + g[(size_t)2 * T] * d[2];
+            const float *g = G + i * 12 + 3 * k;
+            const float gd = g[0] * d[k][0] + g[1] * d[k][1] + g[2] * d[k][2];
             u[i] -= gd;
             gdx[i] += gd;
         }
-    }
-    float Hl[21];
-#pragma unroll
-    for (int k = 0; k < 21; ++k) Hl[k] = tv.H_l[(size_t)k * T + t];
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-        float acc = em::inv_sym_w(i) * tv.g_s[(size_t)i * T + t];
+        float acc = em::inv_sym_w(i) * gs[i];
 #pragma unroll
         for (int j = 0; j < 6; ++j) acc += Hl[em::p21(i, j)] * u[j];
         nl[i] = -acc;
@@ -308,7 +318,7 @@ __device__ __forceinline__ void local_tet(const TetViews &tv, const float *__res
     }
 }
 
-__global__ void __launch_bounds__(kVertexThreads)
+__global__ void __launch_bounds__(kVertexThreads, 2)
     local_solve_kernel(float *x, TetViews tv, VertexViews vv, int tet_blocks) {
     if ((int)blockIdx.x >= tet_blocks) {
         const int v = (blockIdx.x - tet_blocks) * blockDim.x + threadIdx.x;
@@ -332,7 +342,7 @@ __global__ void __launch_bounds__(kVertexThreads)
 // stored, and each block writes its sums of the merit function at (x, s)
 // with the new lambda and of the slope (g_x - G^T lambda) . dx +
 // (g_s + SYM lambda) . ds (solver.py:803-869, 893-915).
-__global__ void __launch_bounds__(kVertexThreads)
+__global__ void __launch_bounds__(kVertexThreads, 2)
     local_solve_deferred_kernel(const float *__restrict__ x, int energy, float dt, double inv_dt2, TetViews tv,
                                 VertexViews vv, ContactViews cv, LineSearchWork w, int tet_blocks) {
     __shared__ double s_red[2][kVertexThreads / 32];
@@ -470,10 +480,9 @@ cudaError_t launch_record_copy(const TetViews &tv, float *plain, int per, bool o
 }
 
 cudaError_t prepare_element_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(element_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kElementSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(element_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kElementSmem);
+    cudaError_t e = cudaSuccess;
+    for (auto *k : {element_kernel<true, 3>, element_kernel<false, 3>, element_kernel<false, 4>})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kElementSmem);
     return e;
 }
 
@@ -484,10 +493,11 @@ cudaError_t launch_element(const float *x, int energy, const TetViews &tv, bool 
     if (e != cudaSuccess) return e;
     const int fix_blocks = std::min(blocks, kElementFp64Blocks);
     if (diagnostics) {
-        element_kernel<true><<<blocks, kElementThreads, kElementSmem, s>>>(x, energy, tv);
+        element_kernel<true, 3><<<blocks, kElementThreads, kElementSmem, s>>>(x, energy, tv);
         element_fp64_kernel<true><<<fix_blocks, kElementThreads, 0, s>>>(x, energy, tv);
     } else {
-        element_kernel<false><<<blocks, kElementThreads, kElementSmem, s>>>(x, energy, tv);
+        if (blocks <= kElementOneWave) element_kernel<false, 3><<<blocks, kElementThreads, kElementSmem, s>>>(x, energy, tv);
+        else element_kernel<false, 4><<<blocks, kElementThreads, kElementSmem, s>>>(x, energy, tv);
         element_fp64_kernel<false><<<fix_blocks, kElementThreads, 0, s>>>(x, energy, tv);
     }
     count_launches(2);
