@@ -34,7 +34,7 @@
 // GB300, us an iteration, a step's other kernels included, against the windowed
 // kernels of pcg.cu: 99 rows 1.1 (one CTA; 3.6), 425 to 1,225 rows 1.5 (clusters
 // of 4 to 16; 3.4), 2,673 rows 1.95 (3.65), 7,560 shuffled rows 3.0 (grid; 9.0),
-// 18,785 rows 3.3 (5.0), shuffled 3.5 (12.1), 140,481 rows 12.0 (20.6).
+// 18,785 rows 3.2 (5.0), shuffled 3.5 (12.1), 140,481 rows 9.6 (19.0).
 //
 // Blocks that fit neither registers nor shared memory (meshes past about
 // 55,000 rows) are copied once a solve into trips in global memory, which the
