@@ -148,3 +148,20 @@ def test_autotune_keeps_serving_a_shuffled_factor_plan():
     a.particle_q.copy_(q)
     solver.step(a, b, None, None, mesh.spec.dt)
     assert solver.solve_stats()[0]["status"] == 0
+
+
+@pytest.mark.parametrize("cells", [(10, 6, 5), (24, 13, 12), (34, 33, 16)], ids=["cluster", "4550", "grid"])
+@pytest.mark.parametrize("order", ["grid", "shuffled"])
+def test_block_jacobi_refinement_on_fp16_blocks_reaches_its_tolerance(cells, order):
+    """The inner solves on the resident PCG with widened FP16 blocks: the fp64 residual meets the tolerance."""
+    mesh = beams.build_beam("nh_beam", cells=cells)
+    if order == "shuffled":
+        mesh = shuffled(mesh)
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=2, energy=mesh.spec.energy, line_search=False,
+                            solver_precision="fp16", outer_tolerance=1e-6, inner_tolerance=1e-2)
+    a, b = model.state(), model.state()
+    a.particle_q.copy_(torch.as_tensor(mesh.q0, device=DEV))
+    solver.step(a, b, None, None, mesh.spec.dt)
+    for st in solver.mixed_stats():
+        assert st["status"] == 0 and st["rel_residual"] <= 1e-6, st

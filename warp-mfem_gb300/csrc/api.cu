@@ -1451,7 +1451,9 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
                              p->rf.cluster > 0) &&
                             p->cfg.preconditioner >= 1;
-    if (!refined32 && persistent) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
+    const bool resident =
+        w.mode == kIrFp16 && p->rl.cluster > 0 && p->rl.blocks == 0 && p->cfg.preconditioner == 1;
+    if (!refined32 && (persistent || resident)) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
     // ... and the whole refinement in one launch there, with the iterate
     // as hi / lo planes padded like the PCG's exchanged vectors
     if (persistent) {

@@ -722,10 +722,15 @@ cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const 
     ir_begin_kernel<<<blocks_for(3 * vv.n, 256), 256, 0, s>>>(vv, w);
     count_launches(fp32 ? 1 : 2);
     e = cudaGetLastError();
-    // block-Jacobi on the fp32 H: the resident or else the one-barrier
+    // block-Jacobi: the resident or else, on the fp32 H, the one-barrier
     // single-reduction PCG for the inner solves (one exchange an iteration
-    // against the factor kernel's two barriers), a launch per correction
-    const bool resident_inner = fp32 && use_precond == 1 && rl.cluster > 0;
+    // against the factor kernel's two barriers), a launch per correction.  The
+    // FP16 H keeps to the factor kernel where the resident PCG is the ordered
+    // one: there a step's result turns on the order of the sums.  So does the
+    // BF16 H everywhere: on ill-conditioned systems its refinement stalls at a
+    // level that depends on that order (3.1e-3 against 3.7e-3 on one).
+    const bool resident_inner =
+        use_precond == 1 && rl.cluster > 0 && (fp32 || (w.hq_words && !bf16 && rl.blocks == 0));
     // a factor preconditioner: the resident factor PCG where the plan has it
     const bool factor_inner = use_precond >= 2 && rf.cluster > 0 && (w.hq_words || fp32);
     const bool single_inner = fp32 && use_precond == 1 && single && single->variant == PcgLayout::kSingleReduction;

@@ -40,7 +40,8 @@
 // 55,000 rows) are copied once a solve into trips in global memory, which the
 // warps then read in coalesced 16-byte loads, four trips in flight.
 //
-// As an inner solve of the mixed-precision refinement (fp32 blocks) it starts
+// As an inner solve of the mixed-precision refinement (fp32 blocks, or the
+// 16-bit ones widened and scaled as they are loaded) it starts
 // from 0 on the residual scaled to unit norm and updates the refinement's
 // state words like the other inner solves (pcg.cu, pcg_factor.cu).
 //
@@ -72,18 +73,26 @@ struct ResArgs {
     // an inner solve of the refinement: its state words, (1 / ||r||, ||r||)
     int *ir_state;
     const float *ir_scale;
+    // its 16-bit blocks, null: the fp32 ones
+    const uint32_t *values_w;
+    const float *row_scale;
+    int lowp_kind;
 };
 
 // OS: own rows a thread keeps, RS: rows it keeps in all (the further ones
 // halo rows), KR: trips of a warp's first slice kept in registers, STREAM: some
 // trips do not fit in shared memory.
 //
+// LOWP: may load 16-bit blocks.  The large-mesh kernel has an instance without,
+// which takes 9.6 us an iteration at 140,481 rows where the other's allocation
+// of the same registers takes 10.0.
+//
 // ORDERED: the sums are added over the same blocks of consecutive rows, in the
 // same order, whatever CTAs the rows sit on, and the scalars are formed as in
 // the windowed single-reduction kernel (pcg.cu, which sums each CTA's range of
 // rows): such a solve has that kernel's iterates bit for bit.  A part is then a
 // run of whole blocks.
-template <Scope SCOPE, int OS, int RS, int KR, bool STREAM, bool ORDERED>
+template <Scope SCOPE, int OS, int RS, int KR, bool STREAM, bool ORDERED, bool LOWP = true>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int kBlocks = ORDERED && SCOPE != kGrid ? kPartMaxBlocks : 1;
@@ -106,10 +115,12 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool inner = a.ir_state != nullptr;
+    bool full = true;  // the fp32 blocks
     if (inner) {
         // nothing to do once the refinement has finished
         const volatile int *st = a.ir_state;
         if (st[0] != 0 || st[7] != 0) return;
+        full = !LOWP || a.values_w == nullptr || st[6] != 0;
     }
     int ncta = 1, rank = 0;
     if (SCOPE == kCluster) {
@@ -238,11 +249,17 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 if (sl >= part.nslices) break;
                 const int t0 = a.v.trip_ptr[part.slice_off + sl], t1 = a.v.trip_ptr[part.slice_off + sl + 1];
                 ntrips[o] |= (unsigned)(t1 - t0) << (8 * qq);
+                float scale = 1.0f;
+                if (LOWP && !full) {
+                    const int i = sl * kPartSliceRows + (lane & 7);
+                    if (i < part.nown) scale = __ldg(a.row_scale + a.v.rows[part.row_off + i]);
+                }
                 auto fetch = [&](int t, float h[9], int &c) {
                     const int src = a.v.src[(size_t)32 * t + lane];
                     c = trip_column(src, a.v.col[(size_t)32 * t + lane], lane);
                     if (src >= 0) {
-                        load_block9(a.values, src, h);
+                        if (LOWP) load_h(a.values, a.values_w, a.lowp_kind, full, src, scale, h);
+                        else load_block9(a.values, src, h);
                     } else {
 #pragma unroll
                         for (int i = 0; i < 9; ++i) h[i] = 0.0f;
@@ -658,10 +675,14 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     if (rank == 0 && tid == 0) {
         if (inner) {
             // a solve that stopped at the cap or stagnated still hands over
-            // its iterate
+            // its iterate; a 16-bit H that broke it restarts on the fp32 H
             a.ir_state[2] += it;
             a.ir_state[3] = 1;
-            if (d.status == MFEM_TIMEOUT || d.status == MFEM_NONFINITE) {
+            if (LOWP && d.status == MFEM_NONFINITE && a.values_w != nullptr && a.ir_state[6] == 0) {
+                a.ir_state[3] = 0;
+                a.ir_state[6] = 1;
+                a.ir_state[7] = 1;
+            } else if (d.status == MFEM_TIMEOUT || d.status == MFEM_NONFINITE) {
                 a.ir_state[5] = d.status;
                 a.ir_state[0] = 1;
             }
@@ -677,12 +698,13 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
 typedef void (*ResKernel)(ResArgs);
 
 template <bool STREAM>
-ResKernel pick_form(const ResidentLayout &L) {
+ResKernel pick_form(const ResidentLayout &L, bool lowp) {
     constexpr int KR = kPartRegTrips;
     if (L.grid) {
         if (L.own_slots == 2)
             return L.row_slots <= 3 ? pcg_resident_kernel<kGrid, 2, 3, 0, STREAM, false>
-                                    : pcg_resident_kernel<kGrid, 2, 4, 0, STREAM, false>;
+                   : lowp           ? pcg_resident_kernel<kGrid, 2, 4, 0, STREAM, false>
+                                    : pcg_resident_kernel<kGrid, 2, 4, 0, STREAM, false, false>;
         return L.row_slots <= 1   ? pcg_resident_kernel<kGrid, 1, 1, KR, STREAM, false>
                : L.row_slots <= 2 ? pcg_resident_kernel<kGrid, 1, 2, KR, STREAM, false>
                                   : pcg_resident_kernel<kGrid, 1, 4, 0, STREAM, false>;
@@ -703,9 +725,9 @@ ResKernel pick_ordered(const ResidentLayout &L) {
                             : pcg_resident_kernel<kCluster, 1, 2, KR, false, true>;
 }
 
-ResKernel pick(const ResidentLayout &L) {
+ResKernel pick(const ResidentLayout &L, bool lowp) {
     if (L.blocks > 0) return pick_ordered(L);
-    return L.stream_trips > 0 ? pick_form<true>(L) : pick_form<false>(L);
+    return L.stream_trips > 0 ? pick_form<true>(L, lowp) : pick_form<false>(L, lowp);
 }
 
 // Launch configuration of n_tasks bodies; attr holds two attributes.
@@ -754,7 +776,7 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
         L.own_slots = 2;  // the cluster form with more than two rows a thread
     }
     cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, pick(L));
+    e = cudaFuncGetAttributes(&fa, pick(L, false));
     if (e != cudaSuccess) return e;
     const bool regs = !(L.own_slots == 2 || L.row_slots > 2);  // pick()'s kernels with register trips
     const int trips = regs ? h.trips_max_reg : h.trips_max;
@@ -770,9 +792,11 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     L.smem = (base + per_trip * L.smem_trips + 15) & ~(size_t)15;
     if (L.smem > most || (L.blocks > 0 && L.stream_trips > 0)) return cudaSuccess;
     L.push_max = !grid && cluster > 1 ? h.push_max : 0;
-    const ResKernel k = pick(L);
+    const ResKernel k = pick(L, false);
     // the limit is the kernel's, not the plan's: every plan sets the same one
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e == cudaSuccess && pick(L, true) != k)
+        e = cudaFuncSetAttribute(pick(L, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e == cudaSuccess && !grid && cluster > 8)
         e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
@@ -817,9 +841,14 @@ cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const Res
     a.counter = w.res_counter;
     a.ir_state = ir ? ir->state : nullptr;
     a.ir_scale = ir ? ir->scale : nullptr;
+    if (ir) {
+        a.values_w = ir->mode == kIrFp32 ? nullptr : ir->hq_words;
+        a.row_scale = ir->row_scale;
+        a.lowp_kind = ir->mode == kIrBf16 ? 1 : 2;
+    }
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = launch_config(L, n_tasks, attr, s);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, pick(L), a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, pick(L, a.values_w != nullptr), a);
     count_launches(1);
     return e;
 }

@@ -64,37 +64,6 @@ struct FactorArgs {
     int lowp_kind;
 };
 
-__device__ __forceinline__ void bf16_pair(uint32_t w, float &a, float &b) {
-    a = __uint_as_float(w << 16);
-    b = __uint_as_float(w & 0xffff0000u);
-}
-
-// Block k of H for the product: fp32, or the widened 16-bit values times the
-// row's scale (the numbers an fp32 copy of the scaled blocks would hold).
-__device__ __forceinline__ void load_h(const FactorArgs &a, bool full, int k, float scale, float h[9]) {
-    if (full) {
-        load_block9(a.values, k, h);
-        return;
-    }
-    uint32_t u[5];
-    load_bf16_words(a.values_w, k, u);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) {
-        float lo, hi;
-        if (a.lowp_kind == 1) {
-            bf16_pair(u[i], lo, hi);
-        } else {
-            __half2 q;
-            memcpy(&q, &u[i], 4);
-            const float2 t = __half22float2(q);
-            lo = t.x;
-            hi = t.y;
-        }
-        h[2 * i] = lo * scale;
-        if (2 * i + 1 < 9) h[2 * i + 1] = hi * scale;
-    }
-}
-
 template <Scope SCOPE, int RS>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(FactorArgs a) {
     constexpr int KR = kPartRegTrips;
@@ -210,7 +179,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
                 const int src = a.v.src[(size_t)32 * t + lane];
                 c = place(a.v.col[(size_t)32 * t + lane]);
                 if (src >= 0) {
-                    load_h(a, full, src, scale, h);
+                    load_h(a.values, a.values_w, a.lowp_kind, full, src, scale, h);
                 } else {
 #pragma unroll
                     for (int e = 0; e < 9; ++e) h[e] = 0.0f;

@@ -3,6 +3,8 @@
 // the block products.  Header-only: each kernel file instantiates its own copy.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "block_loads.cuh"
 #include "grid_sync.cuh"
 #include "internal.h"
@@ -77,6 +79,39 @@ __device__ __forceinline__ void block_mac(const float h[9], const float4 v, floa
     a[0] += h[0] * v.x + h[1] * v.y + h[2] * v.z;
     a[1] += h[3] * v.x + h[4] * v.y + h[5] * v.z;
     a[2] += h[6] * v.x + h[7] * v.y + h[8] * v.z;
+}
+
+__device__ __forceinline__ void bf16_pair(uint32_t w, float &a, float &b) {
+    a = __uint_as_float(w << 16);
+    b = __uint_as_float(w & 0xffff0000u);
+}
+
+// Block k of H for the product: fp32, or the widened 16-bit values (five words
+// a block; kind 1: bfloat16, else half) times the row's scale, the numbers an
+// fp32 copy of the scaled blocks would hold.
+__device__ __forceinline__ void load_h(const float *values, const uint32_t *words, int kind, bool full, int k,
+                                       float scale, float h[9]) {
+    if (full) {
+        load_block9(values, k, h);
+        return;
+    }
+    uint32_t u[5];
+    load_bf16_words(words, k, u);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        float lo, hi;
+        if (kind == 1) {
+            bf16_pair(u[i], lo, hi);
+        } else {
+            __half2 q;
+            memcpy(&q, &u[i], 4);
+            const float2 t = __half22float2(q);
+            lo = t.x;
+            hi = t.y;
+        }
+        h[2 * i] = lo * scale;
+        if (2 * i + 1 < 9) h[2 * i + 1] = hi * scale;
+    }
 }
 
 // The window column of a lane of a trip: a lane without a block (src < 0)
