@@ -1,0 +1,44 @@
+"""Inner solves of the mixed refinement on meshes whose vertex order has no
+windowed PCG: the resident kernels stand in for the global-memory inner PCG
+there, and keep their dot products, partial sums and scalars in fp64 as it does.
+
+An inner tolerance of 1e-20 tells the two widths apart without measuring any
+rounding: the squared norms it is compared with are 1e-40, which float32 sums
+of products cannot hold (the recurrence breaks down on the way), and fp64 sums
+can.  Both forms run the same iteration on a well-conditioned system, so they
+meet the tolerance after as many iterations, to the 2 % that two forms of the
+recurrence are allowed elsewhere."""
+import pytest
+import torch
+
+from mfem_gb300 import Model, MixedFEMSolver, beams
+from test_gpu_resident import shuffled
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def inner_solve(mesh, **kw):
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=1, energy=mesh.spec.energy, line_search=False, inner_tolerance=1e-20,
+                            outer_tolerance=1e-14, outer_max_iterations=1, cg_max_iterations=5000, **kw)
+    q = torch.as_tensor(mesh.q0, device=DEV)
+    x = q.clone()
+    solver.predict(q, torch.zeros_like(q), mesh.spec.dt)
+    solver.update_system(x)
+    solver.assemble(x, mesh.spec.dt)
+    solver.global_solve(0)
+    return solver.mixed_stats()[0], solver.pcg_layout()
+
+
+@pytest.mark.parametrize("cells", [(16, 16, 16), (20, 20, 20), (26, 26, 24)], ids=lambda c: "x".join(map(str, c)))
+@pytest.mark.parametrize("pc", ["block_jacobi", "fsai"])
+@pytest.mark.parametrize("precision", ["fp16", "fp32_refined"])
+def test_inner_solve_reaches_a_tolerance_below_float32_sums(cells, pc, precision):
+    mesh = shuffled(beams.build_beam("cantilever", cells=cells))
+    a, _ = inner_solve(mesh, preconditioner=pc, solver_precision=precision)
+    b, lay = inner_solve(mesh, preconditioner=pc, solver_precision=precision, pcg_ctas=min(132, -(-mesh.n // 64)))
+    assert lay["variant"] in ("standard", "gather", "global_memory"), lay
+    assert b["inner_iterations"] < 5000, b
+    assert abs(a["inner_iterations"] - b["inner_iterations"]) <= max(2, b["inner_iterations"] // 50), (a, b)
+    assert a["rel_residual"] <= 2.0 * b["rel_residual"], (a, b)

@@ -1426,6 +1426,10 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     w.outer_max = cfg.outer_max_iterations;
     w.inner_tol = cfg.inner_tolerance;
     w.outer_tol = cfg.outer_tolerance;
+    // no windowed form of these inner solves (fp32 sums): the global-memory
+    // inner PCG's place, and its fp64 sums
+    w.wide = !(p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
+               (refined32 && p->pl.variant == PcgLayout::kSingleReduction));
     alloc(&w.lowp, refined32 ? 16 : nz * 9 * 2);
     alloc(&w.row_scale, (size_t)p->n * sizeof(float));
     alloc(&w.dx_pair, 2 * n3 * sizeof(float2));

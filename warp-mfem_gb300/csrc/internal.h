@@ -277,6 +277,8 @@ struct IrWork {
     int outer_max;
     float inner_tol;
     double outer_tol;
+    bool wide;                 // resident inner solves keep their dot products and scalars in fp64: those of
+                               // the plans whose inner solves would else run in the global-memory inner PCG
     void *lowp;                // [nnzb][9] bf16 / fp16, H / row scale
     float *row_scale;          // [n]
     float2 *dx_pair;           // [2][n][3] double-buffered solution, each value hi + lo of two floats
@@ -284,7 +286,7 @@ struct IrWork {
     float *e;                  // [n][3] inner correction
     float *res;                // [n][3] fp32 copy of the fp64 residual (inner rhs)
     float *z, *p0, *p1, *r, *Ap;  // inner PCG vectors [n][3]
-    double *partials;          // [2][256][4] fp64 partial sums of the inner PCG
+    double *partials;          // [2][256][4] fp64 partial sums of the inner PCG, resident or not
     unsigned long long *counter;  // inner PCG grid barrier, never reset
     double *res_partials;      // [residual blocks][2]
     unsigned *ticket;          // last-block detection of the residual kernel

@@ -727,8 +727,9 @@ cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const 
     // against the factor kernel's two barriers), a launch per correction.  The
     // FP16 H keeps to the factor kernel where the resident PCG is the ordered
     // one: there a step's result turns on the order of the sums.  So does the
-    // BF16 H everywhere: on ill-conditioned systems its refinement stalls at a
-    // level that depends on that order (3.1e-3 against 3.7e-3 on one).
+    // BF16 H with block-Jacobi: on ill-conditioned systems its refinement
+    // stalls at a level that depends on that order (3.1e-3 against 3.7e-3 on
+    // one).  With a factor preconditioner the resident form takes all three.
     const bool resident_inner =
         use_precond == 1 && rl.cluster > 0 && (fp32 || (w.hq_words && !bf16 && rl.blocks == 0));
     // a factor preconditioner: the resident factor PCG where the plan has it

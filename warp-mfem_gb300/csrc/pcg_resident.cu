@@ -43,7 +43,9 @@
 // As an inner solve of the mixed-precision refinement (fp32 blocks, or the
 // 16-bit ones widened and scaled as they are loaded) it starts
 // from 0 on the residual scaled to unit norm and updates the refinement's
-// state words like the other inner solves (pcg.cu, pcg_factor.cu).
+// state words like the other inner solves (pcg.cu, pcg_factor.cu); where it
+// stands in for the global-memory inner PCG (pcg_mixed.cu) its dot products,
+// partial sums and scalars are fp64 as that one's are.
 //
 // Every wait is bounded; after a timeout the kernel sets the sticky error
 // flag and every CTA leaves (a cluster's through one more barrier, which all
@@ -67,8 +69,9 @@ struct ResArgs {
     int maxiter, use_precond;
     int nown_max, nhalo_max, smem_trips, stream_trips, push_max;
     int blocks, block_warps;  // ordered sums: blocks of the body, warps of the longest one
-    // kGrid: published rows [2][n], partial sums [2][CTAs], barrier arrivals
-    float4 *pub, *partials;
+    // kGrid: published rows [2][n], partial sums [2][CTAs][4], barrier arrivals
+    float4 *pub;
+    void *partials;
     unsigned long long *counter;
     // an inner solve of the refinement: its state words, (1 / ||r||, ||r||)
     int *ir_state;
@@ -92,17 +95,23 @@ struct ResArgs {
 // the windowed single-reduction kernel (pcg.cu, which sums each CTA's range of
 // rows): such a solve has that kernel's iterates bit for bit.  A part is then a
 // run of whole blocks.
-template <Scope SCOPE, int OS, int RS, int KR, bool STREAM, bool ORDERED, bool LOWP = true>
+//
+// Sum: what dot products, partial sums and the recurrence's scalars are held
+// in; double for the inner solves that the global-memory inner PCG served.  A
+// chain of some fifty dependent fp64 operations an iteration: 7.0 us at 7,560
+// shuffled rows against 3.1 with fp32 sums (that form: 16.3).
+template <Scope SCOPE, int OS, int RS, int KR, bool STREAM, bool ORDERED, bool LOWP = true, class Sum = float>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int kBlocks = ORDERED && SCOPE != kGrid ? kPartMaxBlocks : 1;
+    constexpr bool kWide = sizeof(Sum) > sizeof(float);
     constexpr int kSums = SCOPE == kCluster ? kPartMaxCluster * kBlocks : 1;  // partial sums of a round
-    __shared__ float s_red[kBlocks][3][kPartWarps];
-    __shared__ __align__(16) float4 s_part[2][kSums];
+    __shared__ Sum s_red[kBlocks][3][kPartWarps];
+    __shared__ __align__(16) Sum s_part[2][kSums][4];
 
     __shared__ __align__(8) uint64_t s_mbar[2];
     __shared__ __align__(16) Verdict s_verdict;
-    __shared__ float s_norm[2];
+    __shared__ Sum s_norm[2];
     __shared__ int s_err;
     float4 *win = reinterpret_cast<float4 *>(smem);                         // u of own rows, then of halo rows
     float4 *halo_w = win + a.nown_max + a.nhalo_max;                        // [2][nhalo_max] pushed by the owners
@@ -143,8 +152,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         }
     }
     if (SCOPE == kGrid && warp == 0) target = grid_count(a.counter) / ncta * ncta;
-    for (int i = tid; SCOPE == kCluster && i < 2 * kSums; i += kPartThreads)
-        s_part[i / kSums][i % kSums] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = tid; SCOPE == kCluster && i < 2 * kSums * 4; i += kPartThreads) (&s_part[0][0][0])[i] = 0.0f;
     if (ORDERED) {
         for (int i = tid; i < kBlocks * 3 * kPartWarps; i += kPartThreads)
             s_red[i / (3 * kPartWarps)][i / kPartWarps % 3][i % kPartWarps] = 0.0f;
@@ -393,43 +401,44 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     // barrier hands them on; with the grid they go to halo_v.  CTA-uniform;
     // the verdict of a wait that gave up is a timeout.
     float halo_v[SCOPE == kGrid ? RS : 1][3];
-    auto exchange = [&](unsigned k, const float v[3], auto term, auto decide) -> Verdict {
+    auto exchange = [&](unsigned k, const Sum v[3], auto term, auto decide) -> Verdict {
         const int buf = k & 1;
         if (ORDERED) {
             __syncthreads();  // own_r, own_u, own_w
 #pragma unroll
             for (int q = 0; q < kTasks; ++q) {
                 if (task_dst[q] < 0) break;
-                float acc[3] = {0.0f, 0.0f, 0.0f};
+                Sum acc[3] = {0.0f, 0.0f, 0.0f};
                 if (task_i[q] < task_end[q]) term(task_i[q], acc);
                 if (SCOPE == kGrid)  // blocks of more than 170 rows
                     for (int i = task_i[q] + kPartThreads; i < task_end[q]; i += kPartThreads) term(i, acc);
-                const float k3 = warp_sum3(acc, lane);
+                const Sum k3 = warp_sum3(acc, lane);
                 if ((lane & 7) == 0 && lane < 24)
                     (&s_red[0][0][0])[task_dst[q] + kPartWarps * (lane == 0 ? 0 : lane == 16 ? 1 : 2)] = k3;
             }
         } else {
-            const float k3 = warp_sum3(v, lane);
+            // (fp64: a warp without rows spares the SM's fp64 pipe)
+            const Sum k3 = kWide && first_trips == 0 ? (Sum)0.0f : warp_sum3(v, lane);
             if ((lane & 7) == 0 && lane < 24) s_red[0][lane == 0 ? 0 : lane == 16 ? 1 : 2][warp] = k3;
         }
         __syncthreads();
-        float sum[3];
+        Sum sum[3];
         const int g = min(lane >> 3, 2), i = lane & 7;
         bool ok = true;
         if (SCOPE == kCluster && tid == 0)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_mbar[buf])),
-                         "r"(16u * (uint32_t)((ORDERED ? a.blocks : ncta) + part.nhalo))
+                         "r"((uint32_t)(4 * sizeof(Sum)) * (uint32_t)(ORDERED ? a.blocks : ncta) + 16u * (uint32_t)part.nhalo)
                          : "memory");
         if (warp < (ORDERED ? part.nblocks : 1)) {
             // a block's sum, by a warp of its own
             const int b = ORDERED ? warp : 0;
             group_sum3(s_red[b][g][i] + s_red[b][g][i + 8], sum);
             if (SCOPE == kCluster && lane < ncta)
-                push16(&s_part[buf][ORDERED ? part.block_lo + b : rank], &s_mbar[buf], lane, sum[0], sum[1], sum[2]);
+                push_sums(s_part[buf][ORDERED ? part.block_lo + b : rank], &s_mbar[buf], lane, sum);
         }
         if (warp == 0) {
             if (SCOPE == kOne && ORDERED && part.nblocks > 1) {
-                float second[3];
+                Sum second[3];
                 group_sum3(s_red[kBlocks > 1 ? 1 : 0][g][i] + s_red[kBlocks > 1 ? 1 : 0][g][i + 8], second);
 #pragma unroll
                 for (int c = 0; c < 3; ++c) sum[c] += second[c];
@@ -437,25 +446,25 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
             if (SCOPE == kCluster) {
                 ok = __all_sync(0xffffffffu, wait_phase(&s_mbar[buf], (k >> 1) & 1u));
                 if (ORDERED) {
-                    float t[3] = {0.0f, 0.0f, 0.0f};
+                    Sum t[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
                     for (int b = 0; b < kSums; b += 32)  // zero past the last block
                         if (b < a.blocks) {
-                            const float4 q = s_part[buf][b + lane < kSums ? b + lane : 0];
-                            t[0] += q.x;
-                            t[1] += q.y;
-                            t[2] += q.z;
+                            const Sum *q = s_part[buf][b + lane < kSums ? b + lane : 0];
+                            t[0] += q[0];
+                            t[1] += q[1];
+                            t[2] += q[2];
                         }
                     spread_sum3(warp_sum3(t, lane), sum);
                 } else {
-                    const float *t = reinterpret_cast<const float *>(s_part[buf]) + g;
+                    const Sum *t = s_part[buf][0] + g;
                     group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
                 }
             }
             if (SCOPE == kGrid) {
                 target += ncta;
                 if (lane == 0) {
-                    a.partials[buf * ncta + rank] = make_float4(sum[0], sum[1], sum[2], 0.0f);
+                    put_sums(static_cast<Sum *>(a.partials), buf * ncta + rank, sum);
                     // every earlier store of this CTA is released before the
                     // counter moves
                     grid_arrive(a.counter);
@@ -483,14 +492,11 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 halo_v[j][2] = t.z;
             }
             if (warp == 0) {
-                float t[3] = {0.0f, 0.0f, 0.0f};
+                Sum t[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
                 for (int b = 0; b < kPartMaxGrid / 32; ++b) {
                     const int c = lane + 32 * b;
-                    const float4 q = c < ncta ? __ldcg(a.partials + buf * ncta + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    t[0] += q.x;
-                    t[1] += q.y;
-                    t[2] += q.z;
+                    add_sums(static_cast<const Sum *>(a.partials), buf * ncta + c, c < ncta, t);
                 }
                 spread_sum3(warp_sum3(t, lane), sum);
             }
@@ -560,31 +566,23 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         }
     };
     // partial sums of gamma, delta and (r, r) over the own rows
-    auto dots = [&](float (&sum)[3]) {
+    auto dots = [&](Sum (&sum)[3]) {
         if (ORDERED) return;
         sum[0] = sum[1] = sum[2] = 0.0f;
 #pragma unroll
-        for (int o = 0; o < OS; ++o)
-            if (own[o]) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    sum[0] = __fmaf_rn(r[o][c], u[o][c], sum[0]);
-                    sum[1] = __fmaf_rn(w[o][c], u[o][c], sum[1]);
-                    sum[2] = __fmaf_rn(r[o][c], r[o][c], sum[2]);
-                }
-            }
+        for (int o = 0; o < OS; ++o) add_rows(r[o], u[o], w[o], own[o], lane, sum);
     };
 
-    auto term = [&](int i, float acc[3]) {  // ORDERED: the same of component i
+    auto term = [&](int i, Sum acc[3]) {  // ORDERED: the same of component i
         const float rc = own_r[i], uc = own_u[i];
-        acc[0] = __fmaf_rn(rc, uc, acc[0]);
-        acc[1] = __fmaf_rn(own_w[i], uc, acc[1]);
-        acc[2] = __fmaf_rn(rc, rc, acc[2]);
+        add_product(rc, uc, acc[0]);
+        add_product(own_w[i], uc, acc[1]);
+        add_product(rc, rc, acc[2]);
     };
 
     // ---- r0 = g - H x0 (x0 = 0 for an inner solve), exchanged in round 0
     const float bscale = inner ? a.ir_scale[0] : 1.0f;
-    float sum[3] = {0.0f, 0.0f, 0.0f};
+    Sum sum[3] = {0.0f, 0.0f, 0.0f};
     product(inner, [&](int q, float acc[3]) {
         const int i = (warp + kPartWarps * q) * kPartSliceRows + (lane & 7);
         if (i < part.nown) {
@@ -601,19 +599,19 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float g = __ldg(a.b + (size_t)3 * row_id[o] + c) * bscale;
-                sum[0] = __fmaf_rn(g, g, sum[0]);
+                add_product(g, g, sum[0]);
                 if (ORDERED) own_r[3 * (row_id[o] - row0) + c] = g;
             }
         }
     // the recurrence's scalars, kept by thread 0 (||g||^2 and (r, r) in s_norm)
-    float thr2 = 0.0f, gamma = 0.0f, alpha = 0.0f;
+    Sum thr2 = 0.0f, gamma = 0.0f, alpha = 0.0f;  // fp64: alpha holds the last denominator
     int it = 0;
     unsigned round = 0;
-    auto rhs_term = [&](int i, float acc[3]) { acc[0] = __fmaf_rn(own_r[i], own_r[i], acc[0]); };
-    Verdict d = exchange(round, sum, rhs_term, [&](const float t[3]) {
+    auto rhs_term = [&](int i, Sum acc[3]) { add_product(own_r[i], own_r[i], acc[0]); };
+    Verdict d = exchange(round, sum, rhs_term, [&](const Sum t[3]) {
         s_norm[0] = t[0];
         s_norm[1] = 0.0f;
-        thr2 = a.tol * a.tol * t[0];
+        thr2 = (Sum)a.tol * a.tol * t[0];
         return Verdict{0.0f, 0.0f, 0, MFEM_OK};
     });
     if (!d.done) {
@@ -626,11 +624,12 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         product(false, push_w);
         if (SCOPE == kGrid) publish(round + 1);
         dots(sum);
-        d = exchange(++round, sum, term, [&](const float t[3]) {
+        d = exchange(++round, sum, term, [&](const Sum t[3]) {
             gamma = t[0];
-            const float rr = t[2];
+            const Sum rr = t[2];
             s_norm[1] = rr;
-            alpha = t[1] > 0.0f ? gamma / t[1] : 0.0f;
+            const Sum first = t[1] > 0.0f ? gamma / t[1] : 0.0f;
+            alpha = kWide ? t[1] : first;
             int status = MFEM_OK;
             if (!isfinite(gamma) || !isfinite(t[1]) || !isfinite(rr) || !isfinite(s_norm[0])) status = MFEM_NONFINITE;
             else if (!(t[1] > 0.0f) && rr > 0.0f) status = MFEM_STAGNATION;
@@ -639,7 +638,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 done = 1;
                 status = MFEM_MAXITER;
             }
-            return Verdict{alpha, 0.0f, done, status};
+            return Verdict{(float)first, 0.0f, done, status};
         });
         while (!d.done) {
             show_u(round, true, d.alpha, d.beta, it == 0);
@@ -648,18 +647,22 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
             if (SCOPE == kGrid) publish(round + 1);
             dots(sum);
             ++it;
-            d = exchange(++round, sum, term, [&](const float t[3]) {
-                const float rr = t[2];
+            d = exchange(++round, sum, term, [&](const Sum t[3]) {
+                const Sum rr = t[2];
                 s_norm[1] = rr;
                 if (!isfinite(t[0]) || !isfinite(t[1]) || !isfinite(rr)) return Verdict{0.0f, 0.0f, 1, MFEM_NONFINITE};
                 if (rr <= thr2) return Verdict{0.0f, 0.0f, 1, MFEM_OK};
-                const float beta = t[0] / gamma;
-                // the ratio in flight with beta, or in the windowed kernel's order
-                const float denom = ORDERED ? t[1] - beta * t[0] / alpha : t[1] - beta * (t[0] / alpha);
+                const Sum beta = t[0] / gamma;
+                // the ratio in flight with beta, or in the windowed kernel's order, or
+                // (a slow fp64 division less) from the last denominator gamma / alpha
+                const Sum denom = kWide     ? t[1] - beta * beta * alpha
+                                  : ORDERED ? t[1] - beta * t[0] / alpha
+                                            : t[1] - beta * (t[0] / alpha);
                 if (!(denom > 0.0f)) return Verdict{0.0f, 0.0f, 1, MFEM_STAGNATION};
-                alpha = t[0] / denom;
+                const Sum next = t[0] / denom;
+                alpha = kWide ? denom : next;
                 gamma = t[0];
-                return Verdict{alpha, beta, it >= a.maxiter, it >= a.maxiter ? MFEM_MAXITER : MFEM_OK};
+                return Verdict{(float)next, (float)beta, it >= a.maxiter, it >= a.maxiter ? MFEM_MAXITER : MFEM_OK};
             });
         }
     }
@@ -687,7 +690,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
                 a.ir_state[0] = 1;
             }
         } else {
-            const float bb = s_norm[0], rr = s_norm[1];
+            const float bb = (float)s_norm[0], rr = (float)s_norm[1];
             const float rel = d.status == MFEM_TIMEOUT ? 0.0f : bb > 0.0f ? sqrtf(rr / bb) : sqrtf(rr);
             a.stats[(size_t)a.slot * a.bodies + task.z] = SolveStats{it, d.status, rel, 0.0f};
         }
@@ -725,12 +728,29 @@ ResKernel pick_ordered(const ResidentLayout &L) {
                             : pcg_resident_kernel<kCluster, 1, 2, KR, false, true>;
 }
 
-ResKernel pick(const ResidentLayout &L, bool lowp) {
+// With fp64 sums, for the mixed refinement's inner solves: slots and register
+// trips as pick_form's, one instance for meshes with and without streamed trips.
+ResKernel pick_wide(const ResidentLayout &L) {
+    constexpr int KR = kPartRegTrips;
+    if (L.grid) {
+        if (L.own_slots == 2) return pcg_resident_kernel<kGrid, 2, 4, 0, true, false, true, double>;
+        return L.row_slots <= 1   ? pcg_resident_kernel<kGrid, 1, 1, KR, true, false, true, double>
+               : L.row_slots <= 2 ? pcg_resident_kernel<kGrid, 1, 2, KR, true, false, true, double>
+                                  : pcg_resident_kernel<kGrid, 1, 4, 0, true, false, true, double>;
+    }
+    if (L.cluster <= 1) return pcg_resident_kernel<kOne, 1, 1, KR, true, false, true, double>;
+    if (L.own_slots == 2) return pcg_resident_kernel<kCluster, 2, 4, 0, true, false, true, double>;
+    return L.row_slots <= 1 ? pcg_resident_kernel<kCluster, 1, 1, KR, true, false, true, double>
+                            : pcg_resident_kernel<kCluster, 1, 2, KR, true, false, true, double>;
+}
+
+ResKernel pick(const ResidentLayout &L, bool lowp, bool wide = false) {
     if (L.blocks > 0) return pick_ordered(L);
+    if (wide) return pick_wide(L);
     return L.stream_trips > 0 ? pick_form<true>(L, lowp) : pick_form<false>(L, lowp);
 }
 
-// Launch configuration of n_tasks bodies; attr holds two attributes.
+// Launch configuration of n_tasks bodies; attr holds its attribute.
 cudaLaunchConfig_t launch_config(const ResidentLayout &L, int n_tasks, cudaLaunchAttribute attr[1], cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_tasks * L.cluster));
@@ -780,7 +800,13 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     if (e != cudaSuccess) return e;
     const bool regs = !(L.own_slots == 2 || L.row_slots > 2);  // pick()'s kernels with register trips
     const int trips = regs ? h.trips_max_reg : h.trips_max;
-    const size_t most = (size_t)optin - fa.sharedSizeBytes;
+    size_t fixed = fa.sharedSizeBytes;
+    if (L.blocks == 0) {  // the same layout serves the fp64 sums
+        e = cudaFuncGetAttributes(&fa, pick_wide(L));
+        if (e != cudaSuccess) return e;
+        fixed = std::max(fixed, fa.sharedSizeBytes);
+    }
+    const size_t most = (size_t)optin - fixed;
     const size_t base = sizeof(float4) * ((size_t)h.nown_max + (!grid && cluster > 1 ? 3 : 1) * (size_t)h.nhalo_max) +
                         (L.row_slots > 1 ? 9 * sizeof(float) * (size_t)std::max(0, h.nown_max + h.nhalo_max - kPartThreads) : 0) +
                         (!grid && cluster > 1 ? sizeof(int) * (size_t)h.push_max : 0) +
@@ -794,11 +820,11 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     L.push_max = !grid && cluster > 1 ? h.push_max : 0;
     const ResKernel k = pick(L, false);
     // the limit is the kernel's, not the plan's: every plan sets the same one
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e == cudaSuccess && pick(L, true) != k)
-        e = cudaFuncSetAttribute(pick(L, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    if (e == cudaSuccess && !grid && cluster > 8)
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (const ResKernel f : {k, pick(L, true), pick(L, true, true)}) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e == cudaSuccess && !grid && cluster > 8)
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
     if (e != cudaSuccess) return e;
     fits = true;
     if (!grid && cluster > 1) {
@@ -837,7 +863,8 @@ cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const Res
     const int block_rows = L.blocks > 0 ? (bv.n + L.blocks - 1) / L.blocks : 0;
     a.block_warps = std::min(kPartWarps, (3 * block_rows + 31) / 32);
     a.pub = reinterpret_cast<float4 *>(w.pub);
-    a.partials = reinterpret_cast<float4 *>(w.partials);
+    const bool wide = ir && ir->wide && L.blocks == 0;
+    a.partials = wide ? static_cast<void *>(ir->partials) : w.partials;
     a.counter = w.res_counter;
     a.ir_state = ir ? ir->state : nullptr;
     a.ir_scale = ir ? ir->scale : nullptr;
@@ -848,7 +875,7 @@ cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const Res
     }
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = launch_config(L, n_tasks, attr, s);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, pick(L, a.values_w != nullptr), a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, pick(L, a.values_w != nullptr, wide), a);
     count_launches(1);
     return e;
 }

@@ -28,7 +28,10 @@
 //
 // A breakdown (non-finite values or a denominator <= 0) starts the solve again
 // with block-Jacobi, inside the launch.  As an inner solve of the refinement H
-// is read from the 16-bit blocks until the refinement has switched to fp32.
+// is read from the 16-bit blocks until the refinement has switched to fp32, and
+// where it stands in for the global-memory inner PCG (pcg_mixed.cu) its dot
+// products, partial sums and scalars are fp64 as that one's are (FSAI at 7,560
+// shuffled rows: 10.9 us an iteration, with fp32 sums 7.1, that form 27.9).
 #include "resident_common.cuh"
 
 #include <algorithm>
@@ -52,8 +55,9 @@ struct FactorArgs {
     const uint32_t *fwords[2];  // the passes' BF16 blocks, five words each
     int nown_max, nhalo_max, push_max, fpush_max, smem_trips, stream_trips;
     int f_trips[2], f_shared[2];
-    // kGrid: published rows [2][n], partial sums [2][CTAs], barrier arrivals
-    float4 *pub, *partials;
+    // kGrid: published rows [2][n], partial sums [2][CTAs][4], barrier arrivals
+    float4 *pub;
+    void *partials;
     unsigned long long *counter;
     // an inner solve of the refinement: its state words, (1 / ||r||, ||r||), and
     // H's 16-bit blocks (kind 1 BF16, 2 FP16; null: fp32) with row scales
@@ -64,15 +68,17 @@ struct FactorArgs {
     int lowp_kind;
 };
 
-template <Scope SCOPE, int RS>
+// Sum: what dot products, partial sums and the scalars are held in.
+template <Scope SCOPE, int RS, class Sum = float>
 __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(FactorArgs a) {
     constexpr int KR = kPartRegTrips;
+    constexpr bool kWide = sizeof(Sum) > sizeof(float);
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float s_red[3][kPartWarps];
-    __shared__ __align__(16) float4 s_part[2][kPartMaxCluster];
+    __shared__ Sum s_red[3][kPartWarps];
+    __shared__ __align__(16) Sum s_part[2][kPartMaxCluster][4];
     __shared__ __align__(8) uint64_t s_mbar[4];  // rounds (two), y, u
     __shared__ __align__(16) Verdict s_verdict;
-    __shared__ float s_norm[2];
+    __shared__ Sum s_norm[2];
     __shared__ int s_err, s_ok[2];
     __shared__ int s_ftrips[2][kMaxFSlices];  // (first trip << 8 | trips) of each slice of a pass
     const int nall = a.nown_max + a.nhalo_max;
@@ -116,7 +122,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
         }
     }
     if (SCOPE == kGrid && warp == 0) target = grid_count(a.counter) / ncta * ncta;
-    if (SCOPE == kCluster && tid < 2 * kPartMaxCluster) s_part[0][tid] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (SCOPE == kCluster && tid < 2 * kPartMaxCluster * 4) (&s_part[0][0][0])[tid] = 0.0f;
     __syncthreads();
     int err = s_err;
     if (SCOPE == kCluster) {
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
         for (int e = 0; e < part.push_passes; ++e, d += part.nslices * 32)
             if (*d >= 0) push16(dst + (*d & 0xffff), mbar, *d >> 16, v[0], v[1], v[2]);
     };
-    auto expect = [&](uint64_t *mbar, int values) {
+    auto expect = [&](uint64_t *mbar, int values) {  // of 16 bytes
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)),
                      "r"(16u * (uint32_t)values)
                      : "memory");
@@ -346,27 +352,28 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
     // Round k: the sums of v[] over the body's own rows, on which warp 0 alone
     // decides, and w of the halo rows (pcg_resident.cu's exchange).
     float halo_v[SCOPE == kGrid ? RS : 1][3];
-    auto exchange = [&](unsigned k, const float v[3], auto decide) -> Verdict {
+    auto exchange = [&](unsigned k, const Sum v[3], auto decide) -> Verdict {
         const int buf = k & 1;
-        const float k3 = warp_sum3(v, lane);
+        // (fp64: a warp without rows spares the SM's fp64 pipe)
+        const Sum k3 = kWide && ntrips == 0 ? (Sum)0.0f : warp_sum3(v, lane);
         if ((lane & 7) == 0 && lane < 24) s_red[lane == 0 ? 0 : lane == 16 ? 1 : 2][warp] = k3;
         __syncthreads();
-        float sum[3];
+        Sum sum[3];
         const int g = min(lane >> 3, 2), i = lane & 7;
         bool ok = true;
         if (warp == 0) {
-            if (SCOPE == kCluster && lane == 0) expect(&s_mbar[buf], ncta + part.nhalo);
+            if (SCOPE == kCluster && lane == 0) expect(&s_mbar[buf], (int)(sizeof(Sum) / 4) * ncta + part.nhalo);
             group_sum3(s_red[g][i] + s_red[g][i + 8], sum);
             if (SCOPE == kCluster) {
-                if (lane < ncta) push16(&s_part[buf][rank], &s_mbar[buf], lane, sum[0], sum[1], sum[2]);
+                if (lane < ncta) push_sums(s_part[buf][rank], &s_mbar[buf], lane, sum);
                 ok = __all_sync(0xffffffffu, wait_phase(&s_mbar[buf], (k >> 1) & 1u));
-                const float *t = reinterpret_cast<const float *>(s_part[buf]) + g;
+                const Sum *t = s_part[buf][0] + g;
                 group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
             }
             if (SCOPE == kGrid) {
                 target += ncta;
                 if (lane == 0) {
-                    a.partials[buf * ncta + rank] = make_float4(sum[0], sum[1], sum[2], 0.0f);
+                    put_sums(static_cast<Sum *>(a.partials), buf * ncta + rank, sum);
                     grid_arrive(a.counter);
                     const long long t0 = clock64();
                     unsigned spins = 0;
@@ -392,14 +399,11 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
                 halo_v[j][2] = t.z;
             }
             if (warp == 0) {
-                float t[3] = {0.0f, 0.0f, 0.0f};
+                Sum t[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
                 for (int b = 0; b < kPartMaxGrid / 32; ++b) {
                     const int c = lane + 32 * b;
-                    const float4 q = c < ncta ? __ldcg(a.partials + buf * ncta + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    t[0] += q.x;
-                    t[1] += q.y;
-                    t[2] += q.z;
+                    add_sums(static_cast<const Sum *>(a.partials), buf * ncta + c, c < ncta, t);
                 }
                 spread_sum3(warp_sum3(t, lane), sum);
             }
@@ -516,16 +520,9 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
         }
         return true;
     };
-    auto dots = [&](float (&sum)[3]) {
+    auto dots = [&](Sum (&sum)[3]) {
         sum[0] = sum[1] = sum[2] = 0.0f;
-        if (own) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                sum[0] = __fmaf_rn(r[0][c], u[c], sum[0]);
-                sum[1] = __fmaf_rn(w[c], u[c], sum[1]);
-                sum[2] = __fmaf_rn(r[0][c], r[0][c], sum[2]);
-            }
-        }
+        add_rows(r[0], u, w, own, lane, sum);
     };
 
     const float bscale = inner ? a.ir_scale[0] : 1.0f;
@@ -564,20 +561,20 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
             if (SCOPE == kCluster) push_row(halo_w + (round & 1) * a.nhalo_max, &s_mbar[round & 1], q, acc);
         });
         publish(round);
-        float sum[3] = {0.0f, 0.0f, 0.0f};
+        Sum sum[3] = {0.0f, 0.0f, 0.0f};
         if (own) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const float g = __ldg(a.b + (size_t)3 * row_id[0] + c) * bscale;
-                sum[0] = __fmaf_rn(g, g, sum[0]);
+                add_product(g, g, sum[0]);
             }
         }
         // the recurrence's scalars, kept by thread 0 (||g||^2 and (r, r) in s_norm)
-        float thr2 = 0.0f, gamma = 0.0f, alpha = 0.0f;
-        d = exchange(round, sum, [&](const float t[3]) {
+        Sum thr2 = 0.0f, gamma = 0.0f, alpha = 0.0f;  // fp64: alpha holds the last denominator
+        d = exchange(round, sum, [&](const Sum t[3]) {
             s_norm[0] = t[0];
             s_norm[1] = 0.0f;
-            thr2 = a.tol * a.tol * t[0];
+            thr2 = (Sum)a.tol * a.tol * t[0];
             return Verdict{0.0f, 0.0f, 0, MFEM_OK};
         });
         const Verdict lost{0.0f, 0.0f, 1, MFEM_TIMEOUT};
@@ -590,11 +587,12 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
             product(false, push_w);
             publish(round + 1);
             dots(sum);
-            d = exchange(++round, sum, [&](const float t[3]) {
+            d = exchange(++round, sum, [&](const Sum t[3]) {
                 gamma = t[0];
-                const float rr = t[2];
+                const Sum rr = t[2];
                 s_norm[1] = rr;
-                alpha = t[1] > 0.0f ? gamma / t[1] : 0.0f;
+                const Sum first = t[1] > 0.0f ? gamma / t[1] : 0.0f;
+                alpha = kWide ? t[1] : first;
                 int status = MFEM_OK;
                 if (!isfinite(gamma) || !isfinite(t[1]) || !isfinite(rr) || !isfinite(s_norm[0])) status = MFEM_NONFINITE;
                 else if (!(t[1] > 0.0f) && rr > 0.0f) status = MFEM_STAGNATION;
@@ -605,7 +603,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
                     done = 1;
                     status = MFEM_MAXITER;
                 }
-                return Verdict{alpha, 0.0f, done, status};
+                return Verdict{(float)first, 0.0f, done, status};
             });
         }
         while (!d.done) {
@@ -617,17 +615,20 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
             publish(round + 1);
             dots(sum);
             ++it;
-            d = exchange(++round, sum, [&](const float t[3]) {
-                const float rr = t[2];
+            d = exchange(++round, sum, [&](const Sum t[3]) {
+                const Sum rr = t[2];
                 s_norm[1] = rr;
                 if (!isfinite(t[0]) || !isfinite(t[1]) || !isfinite(rr)) return Verdict{0.0f, 0.0f, 1, MFEM_NONFINITE};
                 if (rr <= thr2) return Verdict{0.0f, 0.0f, 1, MFEM_OK};
-                const float beta = t[0] / gamma;
-                const float denom = t[1] - beta * (t[0] / alpha);  // the ratio in flight with beta
+                const Sum beta = t[0] / gamma;
+                // the ratio in flight with beta, or (a slow fp64 division less) from
+                // the last denominator gamma / alpha
+                const Sum denom = kWide ? t[1] - beta * beta * alpha : t[1] - beta * (t[0] / alpha);
                 if (!(denom > 0.0f)) return Verdict{0.0f, 0.0f, 1, MFEM_STAGNATION};
-                alpha = t[0] / denom;
+                const Sum next = t[0] / denom;
+                alpha = kWide ? denom : next;
                 gamma = t[0];
-                return Verdict{alpha, beta, it >= a.maxiter, it >= a.maxiter ? MFEM_MAXITER : MFEM_OK};
+                return Verdict{(float)next, (float)beta, it >= a.maxiter, it >= a.maxiter ? MFEM_MAXITER : MFEM_OK};
             });
         }
         ++round;  // the next attempt's first
@@ -660,7 +661,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
                 a.ir_state[0] = 1;
             }
         } else {
-            const float bb = s_norm[0], rr = s_norm[1];
+            const float bb = (float)s_norm[0], rr = (float)s_norm[1];
             const float rel = d.status == MFEM_TIMEOUT ? 0.0f : bb > 0.0f ? sqrtf(rr / bb) : sqrtf(rr);
             a.stats[(size_t)a.slot * a.bodies + task.z] = SolveStats{it_done + it, d.status, rel, 0.0f};
         }
@@ -669,6 +670,12 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
 }
 
 typedef void (*FacKernel)(FactorArgs);
+
+// With fp64 sums, for the mixed refinement's inner solves (grids only).
+FacKernel pick_wide(const ResidentLayout &L) {
+    return L.row_slots <= 2 ? pcg_resident_factor_kernel<kGrid, 2, double>
+                            : pcg_resident_factor_kernel<kGrid, 3, double>;
+}
 
 FacKernel pick(const ResidentLayout &L) {
     if (L.grid) return L.row_slots <= 2 ? pcg_resident_factor_kernel<kGrid, 2> : pcg_resident_factor_kernel<kGrid, 3>;
@@ -720,7 +727,13 @@ cudaError_t resident_factor_layout(int device, const ResidentHost &h, int cluste
     cudaFuncAttributes fa;
     e = cudaFuncGetAttributes(&fa, k);
     if (e != cudaSuccess) return e;
-    const size_t most = (size_t)optin - fa.sharedSizeBytes;
+    size_t fixed = fa.sharedSizeBytes;
+    if (grid) {  // the same layout serves the fp64 sums
+        e = cudaFuncGetAttributes(&fa, pick_wide(L));
+        if (e != cudaSuccess) return e;
+        fixed = std::max(fixed, fa.sharedSizeBytes);
+    }
+    const size_t most = (size_t)optin - fixed;
     L.push_max = !grid && cluster > 1 ? h.push_max : 0;
     L.fpush_max = !grid && cluster > 1 ? h.fpush_max : 0;
     size_t left = sizeof(float4) * (3 * ((size_t)h.nown_max + h.nhalo_max) + (L.push_max ? 2 * (size_t)h.nhalo_max : 0)) +
@@ -744,6 +757,8 @@ cudaError_t resident_factor_layout(int device, const ResidentHost &h, int cluste
     if (L.smem > most) return cudaSuccess;
     // the limit is the kernel's, not the plan's: every plan sets the same one
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e == cudaSuccess && grid)
+        e = cudaFuncSetAttribute(pick_wide(L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e == cudaSuccess && !grid && cluster > 8)
         e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
@@ -788,7 +803,8 @@ cudaError_t launch_resident_factor(const BsrViews &bv, const VertexViews &vv, co
         a.f_shared[i] = L.f_shared[i] ? 1 : 0;
     }
     a.pub = reinterpret_cast<float4 *>(w.pub);
-    a.partials = reinterpret_cast<float4 *>(w.partials);
+    const bool wide = ir && ir->wide && L.grid;
+    a.partials = wide ? static_cast<void *>(ir->partials) : w.partials;
     a.counter = w.res_counter;
     if (ir) {
         a.ir_state = ir->state;
@@ -799,7 +815,7 @@ cudaError_t launch_resident_factor(const BsrViews &bv, const VertexViews &vv, co
     }
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = launch_config(L, n_tasks, attr, s);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, pick(L), a);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, wide ? pick_wide(L) : pick(L), a);
     count_launches(1);
     return e;
 }

@@ -28,10 +28,11 @@ __device__ __forceinline__ uint32_t remote_addr(const void *p, int rank) {
 }
 
 // 16 bytes into CTA `rank`'s shared memory, counted by its mbarrier.
-__device__ __forceinline__ void push16(const void *dst, const void *mbar, int rank, float a, float b, float c) {
+__device__ __forceinline__ void push16(const void *dst, const void *mbar, int rank, float a, float b, float c,
+                                       float d = 0.0f) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
                      remote_addr(dst, rank)),
-                 "f"(a), "f"(b), "f"(c), "f"(0.0f), "r"(remote_addr(mbar, rank))
+                 "f"(a), "f"(b), "f"(c), "f"(d), "r"(remote_addr(mbar, rank))
                  : "memory");
 }
 
@@ -127,17 +128,19 @@ __device__ __forceinline__ int trip_column(int src, int c, int lane) {
 // of v[0], v[1] and v[2].  Each exchange halves what a lane carries, so three
 // sums take six shuffles (a block's 16 warps otherwise spend most of a
 // reduction issuing shuffles).
-__device__ __forceinline__ float warp_sum3(const float v[3], int lane) {
+template <class Sum>
+__device__ __forceinline__ Sum warp_sum3(const Sum v[3], int lane) {
     const bool b0 = lane & 16, b1 = lane & 8;
-    float k0 = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 16);
-    float k1 = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
-    float k = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 8);
+    Sum k0 = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], 16);
+    Sum k1 = v[2] + __shfl_xor_sync(0xffffffffu, v[2], 16);
+    Sum k = (b1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b1 ? k0 : k1, 8);
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(0xffffffffu, k, off);
     return k;
 }
 
-__device__ __forceinline__ void spread_sum3(float k, float sum[3]) {
+template <class Sum>
+__device__ __forceinline__ void spread_sum3(Sum k, Sum sum[3]) {
     sum[0] = __shfl_sync(0xffffffffu, k, 0);
     sum[1] = __shfl_sync(0xffffffffu, k, 16);
     sum[2] = __shfl_sync(0xffffffffu, k, 8);
@@ -145,11 +148,98 @@ __device__ __forceinline__ void spread_sum3(float k, float sum[3]) {
 
 // Adds two values a lane over lanes 8g .. 8g + 7 and hands group g's sum to
 // every lane as sum[g].
-__device__ __forceinline__ void group_sum3(float k, float sum[3]) {
+template <class Sum>
+__device__ __forceinline__ void group_sum3(Sum k, Sum sum[3]) {
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(0xffffffffu, k, off);
 #pragma unroll
     for (int i = 0; i < 3; ++i) sum[i] = __shfl_sync(0xffffffffu, k, 8 * i);
+}
+
+// A CTA's three partial sums (16 bytes, or 32 in fp64) into CTA `rank`'s
+// shared memory.
+__device__ __forceinline__ void push_sums(const void *dst, const void *mbar, int rank, const float s[3]) {
+    push16(dst, mbar, rank, s[0], s[1], s[2]);
+}
+__device__ __forceinline__ void push_sums(const double *dst, const void *mbar, int rank, const double s[3]) {
+    push16(dst, mbar, rank, __int_as_float(__double2loint(s[0])), __int_as_float(__double2hiint(s[0])),
+           __int_as_float(__double2loint(s[1])), __int_as_float(__double2hiint(s[1])));
+    push16(dst + 2, mbar, rank, __int_as_float(__double2loint(s[2])), __int_as_float(__double2hiint(s[2])), 0.0f);
+}
+
+// CTA c's partial sums in a grid's array of them, four numbers a CTA; add_sums
+// adds those of a CTA that is in the grid.
+__device__ __forceinline__ void put_sums(float *partials, int c, const float s[3]) {
+    reinterpret_cast<float4 *>(partials)[c] = make_float4(s[0], s[1], s[2], 0.0f);
+}
+__device__ __forceinline__ void put_sums(double *partials, int c, const double s[3]) {
+    double2 *d = reinterpret_cast<double2 *>(partials) + 2 * c;
+    d[0] = make_double2(s[0], s[1]);
+    d[1] = make_double2(s[2], 0.0);
+}
+__device__ __forceinline__ void add_sums(const float *partials, int c, bool in, float t[3]) {
+    const float4 q = in ? __ldcg(reinterpret_cast<const float4 *>(partials) + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    t[0] += q.x;
+    t[1] += q.y;
+    t[2] += q.z;
+}
+__device__ __forceinline__ void add_sums(const double *partials, int c, bool in, double t[3]) {
+    if (!in) return;
+    const double2 *d = reinterpret_cast<const double2 *>(partials) + 2 * c;
+    const double2 a = __ldcg(d), b = __ldcg(d + 1);
+    t[0] += a.x;
+    t[1] += a.y;
+    t[2] += b.x;
+}
+
+__device__ __forceinline__ void add_product(float a, float b, float &sum) { sum = __fmaf_rn(a, b, sum); }
+__device__ __forceinline__ void add_product(float a, float b, double &sum) { sum = fma((double)a, (double)b, sum); }
+
+// A warp's products of r.u, w.u and r.r over the rows its lanes own (`own`),
+// added to sum[].  fp32: a lane its own row.  fp64: an SM starts a warp's fp64
+// instruction every 16 cycles, full or not, and with up to 128 rows a CTA
+// only eight lanes of a warp own one; so for one or two groups of eight the
+// components are dealt out, one a lane, and the warp issues 6 or 12 of them
+// instead of 18 (7,560 rows: 8.4 -> 7.0 us an iteration).
+__device__ __forceinline__ void add_rows(const float r[3], const float u[3], const float w[3], bool own, int,
+                                         float sum[3]) {
+    if (!own) return;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        add_product(r[c], u[c], sum[0]);
+        add_product(w[c], u[c], sum[1]);
+        add_product(r[c], r[c], sum[2]);
+    }
+}
+__device__ __forceinline__ void add_rows(const float r[3], const float u[3], const float w[3], bool own, int lane,
+                                         double sum[3]) {
+    const unsigned owners = __ballot_sync(0xffffffffu, own);
+    if (owners & 0xffff0000u) {
+        if (!own) return;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            add_product(r[c], u[c], sum[0]);
+            add_product(w[c], u[c], sum[1]);
+            add_product(r[c], r[c], sum[2]);
+        }
+        return;
+    }
+    const int c = lane % 3;
+    for (int from = lane / 3; owners >> (from - lane / 3); from += 8) {
+        float v[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float *x = i == 0 ? r : i == 1 ? u : w;
+            const float x0 = __shfl_sync(0xffffffffu, x[0], from), x1 = __shfl_sync(0xffffffffu, x[1], from),
+                        x2 = __shfl_sync(0xffffffffu, x[2], from);
+            v[i] = c == 0 ? x0 : c == 1 ? x1 : x2;
+        }
+        if (lane < 24 && ((owners >> from) & 1u)) {
+            add_product(v[0], v[1], sum[0]);
+            add_product(v[2], v[1], sum[1]);
+            add_product(v[0], v[0], sum[2]);
+        }
+    }
 }
 
 // What warp 0 decides after a reduction, for the whole CTA.
