@@ -332,6 +332,7 @@ constexpr int kPartMaxCluster = 16;
 constexpr int kPartMaxGrid = 256;
 constexpr int kFactorSliceRows = 32;  // rows a warp takes at once in a factor pass, a lane a row
 constexpr int kPartMaxBlocks = 8;  // of a part, with ordered sums
+constexpr int kPartTasks = 3;      // runs of 32 components that a warp of a cluster sums, with ordered sums
 constexpr int kPartRegTrips = 4;    // trips of a warp's first slice whose blocks stay in registers
 
 struct ResPart {
@@ -384,6 +385,15 @@ void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *c
 // the resident PCG's ordered sums.
 void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
                          bool push_lists);
+// Warps that add a block's components, 32 each.
+inline int ordered_block_warps(int n, int blocks) {
+    const int rows = (n + blocks - 1) / blocks;
+    return 3 * rows >= 32 * kPartWarps ? kPartWarps : (3 * rows + 31) / 32;
+}
+// The kernel's ordered sums reach every component of every part: on a grid a
+// part is one block, which its warps stride over; in a cluster a warp adds
+// kPartTasks runs, in one CTA one, and no warp a second run of its block.
+bool ordered_sums_fit(const ResidentHost &h, int cluster, bool grid);
 // The same for several bodies of `parts` parts each, the bodies in parallel.
 void resident_add_bodies(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, const float *rest_q,
                          const int32_t *row_off, const std::vector<int> &bodies, int parts,
@@ -408,7 +418,6 @@ struct ResidentLayout {
     int smem_trips = 0;    // trips a warp keeps in shared memory
     int stream_trips = 0;  // trips a warp streams from global memory
     int blocks = 0;        // ordered sums over so many blocks of rows; 0: sums over the parts
-    int block_max = 0;
     bool factor = false;   // a factor preconditioner's layout (pcg_resident_factor.cu)
     int f_trips[2] = {0, 0};         // most trips of a part in the first and second pass
     bool f_shared[2] = {false, false};  // that pass's blocks sit in shared memory

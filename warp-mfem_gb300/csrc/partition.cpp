@@ -259,6 +259,13 @@ void resident_add_body(ResidentHost &h, const int32_t *row_ptr, const int32_t *c
     add_parts(h, row_ptr, col_idx, row_lo, body, rows, bounds, push_lists, threads, factor, false);
 }
 
+bool ordered_sums_fit(const ResidentHost &h, int cluster, bool grid) {
+    if (grid) return h.block_max <= 1;
+    const int n = h.tasks[0].w, tasks = cluster > 1 ? kPartTasks : 1;
+    return h.block_max <= (cluster > 1 ? kPartMaxBlocks : 2) && 3 * ((n + h.blocks - 1) / h.blocks) <= 32 * kPartWarps &&
+           h.block_max * ordered_block_warps(n, h.blocks) <= kPartWarps * tasks;
+}
+
 void resident_add_ranges(ResidentHost &h, const int32_t *row_ptr, const int32_t *col_idx, int n, int parts, int blocks,
                          bool push_lists) {
     std::vector<int> rows(n), bounds(parts + 1, 0);

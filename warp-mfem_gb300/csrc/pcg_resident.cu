@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     // ORDERED: the part's first row, and per task of this warp (32 consecutive
     // components of a block) the lane's component, the block's end and where
     // the sum goes; -1: no task
-    constexpr int kTasks = SCOPE == kOne ? 1 : SCOPE == kGrid ? 1 : 3;
+    constexpr int kTasks = SCOPE == kCluster ? kPartTasks : 1;
     int row0 = 0, task_i[kTasks], task_end[kTasks], task_dst[kTasks];
     if (ORDERED) {
         auto block_row = [&](int b) { return (int)((long long)a.n * (part.block_lo + b) / a.blocks); };
@@ -788,10 +788,9 @@ cudaError_t resident_layout(int device, const ResidentHost &h, int cluster, bool
     if (L.own_slots > 2 || L.row_slots > 4 || h.slice_trips_max > 255) return cudaSuccess;
     if (!grid && cluster <= 1 && (L.own_slots > 1 || L.row_slots > 1)) return cudaSuccess;
     L.blocks = h.blocks;
-    L.block_max = h.block_max;
     if (L.blocks > 0) {
         // ordered sums: one own row and at most two rows a thread, nothing streamed
-        if (L.own_slots > 1 || L.row_slots > 2 || L.block_max > (grid ? 1 : kPartMaxBlocks)) return cudaSuccess;
+        if (L.own_slots > 1 || L.row_slots > 2 || !ordered_sums_fit(h, cluster, grid)) return cudaSuccess;
     } else if (!grid && L.row_slots > 2) {
         L.own_slots = 2;  // the cluster form with more than two rows a thread
     }
@@ -860,8 +859,7 @@ cudaError_t launch_resident(const BsrViews &bv, const VertexViews &vv, const Res
     a.stream_trips = L.stream_trips;
     a.push_max = L.push_max;
     a.blocks = L.blocks;
-    const int block_rows = L.blocks > 0 ? (bv.n + L.blocks - 1) / L.blocks : 0;
-    a.block_warps = std::min(kPartWarps, (3 * block_rows + 31) / 32);
+    a.block_warps = L.blocks > 0 ? ordered_block_warps(bv.n, L.blocks) : 0;
     a.pub = reinterpret_cast<float4 *>(w.pub);
     const bool wide = ir && ir->wide && L.blocks == 0;
     a.partials = wide ? static_cast<void *>(ir->partials) : w.partials;
