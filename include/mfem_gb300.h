@@ -261,9 +261,10 @@ int mfem_plan_sizes(const mfem_plan *plan, int32_t *n_particles, int32_t *n_tets
  * set), CTAs, whether each CTA keeps its slice of H in shared
  * memory, and the dynamic shared memory per CTA.  With pcg_ctas 0 the plan
  * runs the resident form where it fits, in place of variants 1 to 4 as its
- * vertex order allows them: CTAs (one, a cluster of up to 16, or a grid) that
- * each hold a compact block of rows chosen from the rest positions; the
- * variant reported is then the one it replaces, the sizes are its own.
+ * vertex order allows them (or 0 for a factor preconditioner): CTAs (one, a
+ * cluster of up to 16, or a grid) that each hold a compact block of rows chosen
+ * from the rest positions; the variant reported is then the one it replaces,
+ * the sizes are its own, also for a refinement whose inner solves run on it.
  * Diagnostics; no reference counterpart. */
 int mfem_plan_pcg_layout(const mfem_plan *plan, int32_t *variant, int32_t *ctas, int32_t *cache_matrix,
                          int64_t *smem_bytes);

@@ -52,10 +52,9 @@ struct mfem_plan {
     // (plan_refinement)
     PcgLayout ir_pl{};
     bool ir_pl_tried = false;
-    // block-Jacobi plans of a mesh that one cluster holds: its parts
-    // (mfem_plan_create); cluster 0: none
-    ResidentLayout rl{};
-    ResidentLayout rf{};  // the same with a factor preconditioner
+    // the resident PCG's parts of a one-mesh plan (mfem_plan_create), with
+    // block-Jacobi or none (rl) or a factor preconditioner (rf); cluster 0: none
+    ResidentLayout rl{}, rf{};
     bool rf_on = true;    // rf in use (mfem_plan_autotune_batch decides)
     LineSearchWork ls{};
     float stage_dt = 0.0f;     // dt of the last mfem_assemble (the line search's 1/dt^2)
@@ -273,8 +272,17 @@ bool valid_config(const mfem_config *cfg, std::string &err) {
     return false;
 }
 
-// The fp32 solve of a one-mesh plan runs on its resident factor layout.
-bool factor_resident(const mfem_plan *p) { return p->rf.cluster > 0 && p->rf_on && p->bw.n_bodies <= 1; }
+// The resident layout on which a one-mesh plan's solves run in refinement mode
+// `mode` (0: the fp32 PCG), or null: the form that the vertex order allows.
+// With block-Jacobi the 16-bit refinements keep their own kernel where the
+// reasons of launch_mixed_solve say so.
+const ResidentLayout *resident_form(const mfem_plan *p, int mode) {
+    if (p->rf.cluster > 0) return p->bw.n_bodies <= 1 && (mode != 0 || p->rf_on) ? &p->rf : nullptr;
+    if (p->rl.cluster == 0) return nullptr;
+    if (mode == 0) return p->bw.n_bodies == 0 ? &p->rl : nullptr;
+    const bool taken = mode == kIrFp32 || (mode == kIrFp16 && p->rl.blocks == 0);
+    return p->cfg.preconditioner == 1 && taken ? &p->rl : nullptr;
+}
 
 // A plan with the learned preconditioner needs its net before any assembly.
 bool net_ready(const mfem_plan *p) { return p->cfg.preconditioner != 3 || p->fv.ready; }
@@ -308,15 +316,17 @@ cudaError_t global_solve(mfem_plan *p, int slot, cudaStream_t s) {
     if (p->ir.mode != 0)
         return launch_mixed_solve(p->bv, p->vv, p->ir, p->pw, p->bw,
                                   p->pl.variant == PcgLayout::kFactor ? p->pl : p->ir_pl,
-                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr, p->rl, p->rf, p->pcg_ctas,
-                                  slot, p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
-    if (factor_resident(p))
+                                  p->pl.variant == PcgLayout::kSingleReduction ? &p->pl : nullptr,
+                                  resident_form(p, p->ir.mode), p->pcg_ctas, slot, p->cfg.cg_max_iterations,
+                                  p->cfg.preconditioner, s);
+    const ResidentLayout *resident = resident_form(p, 0);
+    if (resident && resident->factor)
         return launch_resident_factor(p->bv, p->vv, p->rf, 1, 1, p->pw, p->bw, p->bw.stats, slot, p->cfg.cg_tolerance,
                                       p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr, s);
     if (p->pl.variant == PcgLayout::kFactor)
         return launch_pcg_factor(p->bv, p->vv, p->pw, p->bw, p->pl, p->pcg_ctas, slot, p->cfg.cg_tolerance,
                                  p->cfg.cg_max_iterations, p->cfg.preconditioner, s);
-    if (p->bw.n_bodies == 0 && p->rl.cluster > 0)
+    if (resident)
         return launch_resident(p->bv, p->vv, p->rl, 1, 1, p->pw, p->pw.stats, slot, p->cfg.cg_tolerance,
                                p->cfg.cg_max_iterations, p->cfg.preconditioner, nullptr, s);
     if (p->bodies_resident) return solve_bodies(p, slot, s);
@@ -1012,16 +1022,11 @@ int mfem_plan_pcg_layout(const mfem_plan *p, int32_t *variant, int32_t *ctas, in
     if (!p) return MFEM_BAD_ARG;
     // the form the vertex order allows, with the sizes of what runs: the
     // resident PCG in place of any of them
-    const bool resident = p->rl.cluster > 0 && p->bw.n_bodies == 0 && (p->ir.mode == 0 || p->ir.mode == kIrFp32);
+    const ResidentLayout *resident = resident_form(p, p->ir.mode);
     if (variant) *variant = p->pl.variant;
-    if (ctas) *ctas = resident ? p->rl.cluster : p->pcg_ctas;
-    if (cache_matrix) *cache_matrix = resident ? p->rl.stream_trips == 0 : p->pl.cache_matrix;
-    if (smem_bytes) *smem_bytes = (int64_t)(resident ? p->rl.smem : p->pl.smem);
-    if (p->pl.variant == PcgLayout::kFactor && factor_resident(p)) {
-        if (ctas) *ctas = p->rf.cluster;
-        if (cache_matrix) *cache_matrix = p->rf.stream_trips == 0;
-        if (smem_bytes) *smem_bytes = (int64_t)p->rf.smem;
-    }
+    if (ctas) *ctas = resident ? resident->cluster : p->pcg_ctas;
+    if (cache_matrix) *cache_matrix = resident ? resident->stream_trips == 0 : p->pl.cache_matrix;
+    if (smem_bytes) *smem_bytes = (int64_t)(resident ? resident->smem : p->pl.smem);
     return MFEM_OK;
 }
 
@@ -1455,9 +1460,7 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
                              p->rf.cluster > 0) &&
                             p->cfg.preconditioner >= 1;
-    const bool resident =
-        w.mode == kIrFp16 && p->rl.cluster > 0 && p->rl.blocks == 0 && p->cfg.preconditioner == 1;
-    if (!refined32 && (persistent || resident)) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
+    if (!refined32 && (persistent || resident_form(p, w.mode))) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
     // ... and the whole refinement in one launch there, with the iterate
     // as hi / lo planes padded like the PCG's exchanged vectors
     if (persistent) {

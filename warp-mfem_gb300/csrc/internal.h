@@ -590,13 +590,12 @@ cudaError_t batch_capacity(int device, int threads, bool factor, int *ctas);
 cudaError_t launch_batched_pcg(const BsrViews &bv, const VertexViews &vv, const BatchViews &bw, int *error, int slot,
                                float tol, int maxiter, int use_precond, cudaStream_t s);
 int ir_residual_blocks(int n);
-// With fp32 blocks and block-Jacobi the inner solves run on the resident
-// layout rl where the plan has one (rl.cluster > 0), else on its
-// single-reduction layout (single, or null), with a factor preconditioner on
-// the resident factor layout rf where it has one, one launch a correction.
+// The inner solves run on `resident` where the plan has such a layout for them
+// (else null), then with fp32 blocks and block-Jacobi on its single-reduction
+// layout (single, or null), one launch a correction.
 cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const IrWork &w, const PcgWork &pw,
                                const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single,
-                               const ResidentLayout &rl, const ResidentLayout &rf, int pcg_ctas, int slot, int maxiter, int use_precond,
+                               const ResidentLayout *resident, int pcg_ctas, int slot, int maxiter, int use_precond,
                                cudaStream_t s);
 // The whole mixed refinement in one launch of the persistent factor PCG
 // (needs IrWork's xf_hi / xf_lo): the warm start in vv.dx, the solution

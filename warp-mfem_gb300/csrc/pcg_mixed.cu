@@ -710,7 +710,7 @@ int ir_residual_blocks(int n) { return std::max(1, (int)(((long long)n * kResGro
 
 cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const IrWork &w, const PcgWork &pw,
                                const BatchViews &fb, const PcgLayout &pl, const PcgLayout *single,
-                               const ResidentLayout &rl, const ResidentLayout &rf, int pcg_ctas, int slot, int maxiter, int use_precond,
+                               const ResidentLayout *resident, int pcg_ctas, int slot, int maxiter, int use_precond,
                                cudaStream_t s) {
     if (bv.n == 0) return cudaSuccess;
     const bool bf16 = w.mode == kIrBf16;
@@ -730,12 +730,9 @@ cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const 
     // BF16 H with block-Jacobi: on ill-conditioned systems its refinement
     // stalls at a level that depends on that order (3.1e-3 against 3.7e-3 on
     // one).  With a factor preconditioner the resident form takes all three.
-    const bool resident_inner =
-        use_precond == 1 && rl.cluster > 0 && (fp32 || (w.hq_words && !bf16 && rl.blocks == 0));
-    // a factor preconditioner: the resident factor PCG where the plan has it
-    const bool factor_inner = use_precond >= 2 && rf.cluster > 0 && (w.hq_words || fp32);
     const bool single_inner = fp32 && use_precond == 1 && single && single->variant == PcgLayout::kSingleReduction;
-    if (e == cudaSuccess && !resident_inner && !factor_inner && !single_inner && w.xf_hi && (w.hq_words || fp32) && pl.variant == PcgLayout::kFactor)
+    if (e == cudaSuccess && !resident && !single_inner && w.xf_hi && (w.hq_words || fp32) &&
+        pl.variant == PcgLayout::kFactor)
         // every correction inside one launch of the persistent factor PCG
         return launch_pcg_factor_refine(bv, vv, w, pw, fb, pl, pcg_ctas, slot, maxiter, use_precond, s);
     const int rb = ir_residual_blocks(vv.n);
@@ -743,10 +740,10 @@ cudaError_t launch_mixed_solve(const BsrViews &bv, const VertexViews &vv, const 
         ir_residual_kernel<<<rb, kResThreads, 0, s>>>(bv, vv, w, pw, slot);
         count_launches(1);
         e = cudaGetLastError();
-        if (e == cudaSuccess && resident_inner)
-            e = launch_resident(bv, vv, rl, 1, 1, pw, pw.stats, slot, 0.0f, maxiter, 1, &w, s);
-        else if (e == cudaSuccess && factor_inner)
-            e = launch_resident_factor(bv, vv, rf, 1, 1, pw, fb, pw.stats, slot, 0.0f, maxiter, use_precond, &w, s);
+        if (e == cudaSuccess && resident && resident->factor)
+            e = launch_resident_factor(bv, vv, *resident, 1, 1, pw, fb, pw.stats, slot, 0.0f, maxiter, use_precond, &w, s);
+        else if (e == cudaSuccess && resident)
+            e = launch_resident(bv, vv, *resident, 1, 1, pw, pw.stats, slot, 0.0f, maxiter, 1, &w, s);
         else if (e == cudaSuccess && single_inner)
             e = launch_pcg_inner(bv, vv, w, pw, *single, pcg_ctas, slot, maxiter, s);
         else if (e == cudaSuccess && (w.hq_words || fp32) && pl.variant == PcgLayout::kFactor)
