@@ -870,7 +870,8 @@ cudaError_t pcg_plan_layout(int device, PcgLayout &L, const int32_t *row_ptr, co
         return cudaErrorInvalidValue;
     }
     PcgKernel k = pick_kernel(L);
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+    // the limit is the kernel's, not the plan's: every plan sets the same one
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
 }
 
 namespace {

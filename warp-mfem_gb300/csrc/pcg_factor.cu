@@ -915,8 +915,9 @@ cudaError_t pcg_factor_layout(int device, PcgLayout &L, const int32_t *row_ptr, 
             L.cache_matrix = o[0];
             L.factor_cache = o[1];
             L.smem = bytes;
+            // the limit is the kernel's, not the plan's: every plan sets the same one
             return cudaFuncSetAttribute(pick_factor_kernel(L), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)L.smem);
+                                        (int)budget);
         }
     }
     for (const auto &o : plain) {
@@ -925,7 +926,7 @@ cudaError_t pcg_factor_layout(int device, PcgLayout &L, const int32_t *row_ptr, 
         L.cache_matrix = o[0];
         L.factor_cache = o[1];
         L.smem = bytes;
-        return cudaFuncSetAttribute(pick_factor_kernel(L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+        return cudaFuncSetAttribute(pick_factor_kernel(L), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
     }
     err = "mesh too large for the persistent factor PCG (shared memory per CTA exceeded)";
     return cudaErrorInvalidValue;
