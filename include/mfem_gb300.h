@@ -396,6 +396,16 @@ int mfem_plan_set_bodies(mfem_plan *plan, int32_t n_bodies, const int32_t *h_ver
                          const int32_t *h_tet_offsets, const int32_t *h_body_energy,
                          const float *h_body_gravity);
 
+/* mfem_plan_create and mfem_plan_set_bodies in one call, which lays nothing out
+ * for the union as one mesh.  The arguments are those of the two. */
+int mfem_plan_create_bodies(const mfem_config *cfg, int32_t n_particles, int32_t n_tets,
+                            const int32_t *h_tet_indices, const float *h_tet_poses,
+                            const float *h_tet_materials, const float *h_particle_q_rest,
+                            const float *h_particle_mass, const float *h_particle_inv_mass,
+                            const float *h_gravity, int32_t device, int32_t n_bodies,
+                            const int32_t *h_vertex_offsets, const int32_t *h_tet_offsets,
+                            const int32_t *h_body_energy, const float *h_body_gravity, mfem_plan **out);
+
 /* CTAs and threads per CTA of the batched PCG's current schedule. */
 int mfem_plan_batch_layout(const mfem_plan *plan, int32_t *ctas, int32_t *threads);
 

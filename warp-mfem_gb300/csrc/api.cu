@@ -52,9 +52,10 @@ struct mfem_plan {
     // (plan_refinement)
     PcgLayout ir_pl{};
     bool ir_pl_tried = false;
-    // the resident PCG's parts of a one-mesh plan (mfem_plan_create), with
+    // the resident PCG's parts of a one-mesh plan (create_plan), with
     // block-Jacobi or none (rl) or a factor preconditioner (rf); cluster 0: none
     ResidentLayout rl{}, rf{};
+    std::vector<void *> mesh_allocs;  // their arrays, until bodies are set
     bool rf_on = true;    // rf in use (mfem_plan_autotune_batch decides)
     LineSearchWork ls{};
     float stage_dt = 0.0f;     // dt of the last mfem_assemble (the line search's 1/dt^2)
@@ -585,8 +586,8 @@ cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q
         cudaError_t e = resident_layout(p->device, h, parts, grid, L, fits);
         if (e != cudaSuccess) return e;
         if (!fits || (!grid && L.stream_trips > 0)) continue;
-        e = upload_resident(p->allocs, h, L.v);
-        if (e == cudaSuccess) e = alloc_stream(p->allocs, h.parts.size(), L);
+        e = upload_resident(p->mesh_allocs, h, L.v);
+        if (e == cudaSuccess) e = alloc_stream(p->mesh_allocs, h.parts.size(), L);
         if (e == cudaSuccess) p->rl = L;
         return e;
     }
@@ -610,8 +611,8 @@ cudaError_t plan_resident_factor(mfem_plan *p, int max_ctas) {
     ResidentLayout L;
     cudaError_t e = resident_factor_layout(p->device, h, parts, true, L, fits);
     if (e != cudaSuccess || !fits) return e;
-    e = upload_resident(p->allocs, h, L.v);
-    if (e == cudaSuccess) e = alloc_stream(p->allocs, h.parts.size(), L);
+    e = upload_resident(p->mesh_allocs, h, L.v);
+    if (e == cudaSuccess) e = alloc_stream(p->mesh_allocs, h.parts.size(), L);
     if (e == cudaSuccess) p->rf = L;
     return e;
 }
@@ -710,6 +711,7 @@ void mfem_plan_destroy(mfem_plan *p) {
         }
         if (p->body_fork) cudaEventDestroy(p->body_fork);
         for (void *a : p->allocs) cudaFree(a);
+        for (void *a : p->mesh_allocs) cudaFree(a);
         for (void *a : p->contact_allocs) cudaFree(a);
         for (void *a : p->ir_allocs) cudaFree(a);
         for (void *a : p->batch_allocs) cudaFree(a);
@@ -720,9 +722,11 @@ void mfem_plan_destroy(mfem_plan *p) {
     delete p;
 }
 
-int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int32_t *h_tets, const float *h_poses,
-                     const float *h_materials, const float *h_rest_q, const float *h_mass, const float *h_inv_mass,
-                     const float *h_gravity, int32_t device, mfem_plan **out) {
+// mfem_plan_create; with `bodies` the mesh is a batch whose bodies the caller
+// sets next, and nothing is laid out for it as one body.
+static int create_plan(const mfem_config *cfg_in, int32_t n, int32_t T, const int32_t *h_tets, const float *h_poses,
+                       const float *h_materials, const float *h_rest_q, const float *h_mass, const float *h_inv_mass,
+                       const float *h_gravity, int32_t device, bool bodies, mfem_plan **out) {
     t_create_error.clear();
     if (!out) return fail(nullptr, MFEM_BAD_ARG, "out is NULL");
     *out = nullptr;
@@ -905,7 +909,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
             cta_info.assign(1, make_int4(0, 0, 0, 0));
         }
     }
-    if (e == cudaSuccess && !p->global_memory_pcg && cfg.preconditioner <= 1 && cfg.pcg_ctas == 0 &&
+    if (e == cudaSuccess && !bodies && !p->global_memory_pcg && cfg.preconditioner <= 1 && cfg.pcg_ctas == 0 &&
         (cfg.pcg_variant == PcgLayout::kAuto || cfg.pcg_variant == PcgLayout::kSingleReduction))
         e = plan_resident(p, sym, h_rest_q, max_ctas);
     int4 *d_cta = nullptr;
@@ -985,7 +989,7 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
         mfem_plan_destroy(p);
         return rc;
     }
-    if (p->global_memory_pcg) {
+    if (p->global_memory_pcg && !bodies) {
         const int32_t voff[2] = {0, n}, toff[2] = {0, T};
         const int rc = install_bodies(p, 1, voff, toff, nullptr, nullptr);
         if (rc != MFEM_OK) {
@@ -1005,6 +1009,29 @@ int mfem_plan_create(const mfem_config *cfg_in, int32_t n, int32_t T, const int3
     }
     *out = p;
     return MFEM_OK;
+}
+
+int mfem_plan_create(const mfem_config *cfg, int32_t n, int32_t T, const int32_t *h_tets, const float *h_poses,
+                     const float *h_materials, const float *h_rest_q, const float *h_mass, const float *h_inv_mass,
+                     const float *h_gravity, int32_t device, mfem_plan **out) {
+    return create_plan(cfg, n, T, h_tets, h_poses, h_materials, h_rest_q, h_mass, h_inv_mass, h_gravity, device, false,
+                       out);
+}
+
+int mfem_plan_create_bodies(const mfem_config *cfg, int32_t n, int32_t T, const int32_t *h_tets, const float *h_poses,
+                            const float *h_materials, const float *h_rest_q, const float *h_mass,
+                            const float *h_inv_mass, const float *h_gravity, int32_t device, int32_t n_bodies,
+                            const int32_t *h_vertex_offsets, const int32_t *h_tet_offsets,
+                            const int32_t *h_body_energy, const float *h_body_gravity, mfem_plan **out) {
+    int rc = create_plan(cfg, n, T, h_tets, h_poses, h_materials, h_rest_q, h_mass, h_inv_mass, h_gravity, device,
+                         n_bodies > 1, out);
+    if (rc != MFEM_OK) return rc;
+    rc = mfem_plan_set_bodies(*out, n_bodies, h_vertex_offsets, h_tet_offsets, h_body_energy, h_body_gravity);
+    if (rc == MFEM_OK) return rc;
+    const std::string msg = (*out)->last_error;
+    mfem_plan_destroy(*out);
+    *out = nullptr;
+    return fail(nullptr, rc, msg);
 }
 
 const char *mfem_plan_last_error(const mfem_plan *p) { return p ? p->last_error.c_str() : t_create_error.c_str(); }
@@ -1733,6 +1760,11 @@ int install_bodies(mfem_plan *p, int n_bodies, const int32_t *voff, const int32_
     drop_body_classes(p);
     for (void *a : p->batch_allocs) cudaFree(a);
     p->batch_allocs.clear();
+    if (n_bodies > 1) {  // the mesh as one body is not solved again
+        for (void *a : p->mesh_allocs) cudaFree(a);
+        p->mesh_allocs.clear();
+        p->rl = p->rf = ResidentLayout{};
+    }
     p->bw = BatchViews{};
     p->tv.energy_code = nullptr;
     p->vv.vertex_body = nullptr;

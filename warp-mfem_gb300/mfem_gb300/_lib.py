@@ -187,6 +187,8 @@ _SIGNATURES = {
     "mfem_tet_slot_map": (ctypes.c_int, [_I32, _I32, _P, _P, _P, _P]),
     "mfem_plan_create": (ctypes.c_int, [ctypes.POINTER(MfemConfig), _I32, _I32, _P, _P, _P, _P, _P, _P, _P, _I32,
                                         ctypes.POINTER(_P)]),
+    "mfem_plan_create_bodies": (ctypes.c_int, [ctypes.POINTER(MfemConfig), _I32, _I32, _P, _P, _P, _P, _P, _P, _P, _I32,
+                                               _I32, _P, _P, _P, _P, ctypes.POINTER(_P)]),
     "mfem_plan_destroy": (None, [_P]),
     "mfem_plan_last_error": (ctypes.c_char_p, [_P]),
     "mfem_plan_sizes": (ctypes.c_int, [_P, ctypes.POINTER(_I32), ctypes.POINTER(_I32), ctypes.POINTER(_I64)]),

@@ -28,18 +28,20 @@ class BatchedSolver:
                            u.tet_poses, u.tet_materials, u.gravity, device=device)
         kwargs.setdefault("cg_tolerance", u.spec.cg_tolerance)
         kwargs.setdefault("cg_max_iterations", u.spec.cg_max_iterations)
-        self.solver = MixedFEMSolver(self.model, iterations=iterations or batch.iterations, line_search=False,
-                                     **kwargs)
-        self._lib = self.solver._lib
-        self._plan = self.solver._plan
         self._host = dict(voff=np.ascontiguousarray(batch.vertex_offsets, dtype=np.int32),
                           toff=np.ascontiguousarray(batch.tet_offsets, dtype=np.int32),
                           energy=np.array([_lib.ENERGY[e] for e in batch.energies], dtype=np.int32),
                           gravity=np.ascontiguousarray(batch.gravity, dtype=np.float32))
         h = self._host
-        P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
-        _lib.check(self._lib.mfem_plan_set_bodies(self._plan, batch.n_bodies, P(h["voff"]), P(h["toff"]),
-                                                  P(h["energy"]), P(h["gravity"])), self._plan)
+        one = batch.n_bodies == 1
+        self.solver = MixedFEMSolver(self.model, iterations=iterations or batch.iterations, line_search=False,
+                                     _bodies=None if one else h, **kwargs)
+        self._lib = self.solver._lib
+        self._plan = self.solver._plan
+        if one:  # a mesh of its own, with a body's energy and gravity
+            P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+            _lib.check(self._lib.mfem_plan_set_bodies(self._plan, 1, P(h["voff"]), P(h["toff"]), P(h["energy"]),
+                                                      P(h["gravity"])), self._plan)
         if kwargs.get("preconditioner") == "learned":
             # rest positions relative to each body's centroid
             self.solver.set_factor_net(kwargs.get("factor_net_params"), vertex_offsets=h["voff"])

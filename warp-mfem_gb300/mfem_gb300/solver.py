@@ -171,10 +171,15 @@ class MixedFEMSolver:
         plan = ctypes.c_void_p()
         P = lambda a: a.ctypes.data_as(ctypes.c_void_p)
         n_rows = h["rest"].shape[0]
-        rc = self._lib.mfem_plan_create(
-            ctypes.byref(self.config), n_rows, h["tets"].shape[0], P(h["tets"]), P(h["poses"]),
-            P(h["materials"]), P(h["rest"]), P(h["mass"]), P(h["inv_mass"]), P(h["gravity"]),
-            self.device.index if self.device.index is not None else torch.cuda.current_device(), ctypes.byref(plan))
+        mesh = (ctypes.byref(self.config), n_rows, h["tets"].shape[0], P(h["tets"]), P(h["poses"]),
+                P(h["materials"]), P(h["rest"]), P(h["mass"]), P(h["inv_mass"]), P(h["gravity"]),
+                self.device.index if self.device.index is not None else torch.cuda.current_device())
+        b = kwargs.get("_bodies")  # a batch's (batched.BatchedSolver)
+        if b is None:
+            rc = self._lib.mfem_plan_create(*mesh, ctypes.byref(plan))
+        else:
+            rc = self._lib.mfem_plan_create_bodies(*mesh, len(b["energy"]), P(b["voff"]), P(b["toff"]), P(b["energy"]),
+                                                   P(b["gravity"]), ctypes.byref(plan))
         if rc != _lib.MFEM_OK:
             msg = self._lib.mfem_plan_last_error(None).decode()
             raise _lib.MfemError(rc, f"mfem_plan_create: {msg}")
