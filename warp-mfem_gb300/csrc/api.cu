@@ -1439,7 +1439,13 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     if (cfg.factor_refresh < 0) return fail(p, MFEM_BAD_ARG, "factor_refresh must be >= 0");
     p->factor_refresh = std::max(1, cfg.factor_refresh);
     if (cfg.precision == MFEM_PRECISION_FP32) return MFEM_OK;
-    e = plan_refinement(p);
+    const bool refined32 = cfg.precision == MFEM_PRECISION_FP32_REFINED;
+    const int mode = refined32 ? kIrFp32 : (cfg.precision == MFEM_PRECISION_BF16 ? kIrBf16 : kIrFp16);
+    // the fp32 blocks' inner solves on the resident form or else the windowed
+    // single-reduction one need no other layout
+    const ResidentLayout *resident = resident_form(p, mode);
+    const bool single = refined32 && p->pl.variant == PcgLayout::kSingleReduction;
+    if (!(resident && single)) e = plan_refinement(p);
     if (e != cudaSuccess) return cuda_fail(p, e, "refinement layout");
 
     const size_t n3 = (size_t)p->n * 3, nz = (size_t)p->nnzb;
@@ -1453,15 +1459,13 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
         }
     };
     IrWork w{};
-    const bool refined32 = cfg.precision == MFEM_PRECISION_FP32_REFINED;
-    w.mode = refined32 ? kIrFp32 : (cfg.precision == MFEM_PRECISION_BF16 ? kIrBf16 : kIrFp16);
+    w.mode = mode;
     w.outer_max = cfg.outer_max_iterations;
     w.inner_tol = cfg.inner_tolerance;
     w.outer_tol = cfg.outer_tolerance;
     // no windowed form of these inner solves (fp32 sums): the global-memory
     // inner PCG's place, and its fp64 sums
-    w.wide = !(p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
-               (refined32 && p->pl.variant == PcgLayout::kSingleReduction));
+    w.wide = !(p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor || single);
     alloc(&w.lowp, refined32 ? 16 : nz * 9 * 2);
     alloc(&w.row_scale, (size_t)p->n * sizeof(float));
     alloc(&w.dx_pair, 2 * n3 * sizeof(float2));
@@ -1484,13 +1488,12 @@ int mfem_plan_set_solver(mfem_plan *p, const mfem_solver_config *cfg_in) {
     alloc(&w.scale, 2 * sizeof(float));
     // a plan on the persistent factor PCG runs its inner solves there, on a
     // copy of the 16-bit blocks padded to 20 bytes (4-byte aligned loads)
-    const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor ||
-                             p->rf.cluster > 0) &&
+    const bool persistent = (p->pl.variant == PcgLayout::kFactor || p->ir_pl.variant == PcgLayout::kFactor) &&
                             p->cfg.preconditioner >= 1;
-    if (!refined32 && (persistent || resident_form(p, w.mode))) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
-    // ... and the whole refinement in one launch there, with the iterate
-    // as hi / lo planes padded like the PCG's exchanged vectors
-    if (persistent) {
+    if (!refined32 && (persistent || resident)) alloc(&w.hq_words, nz * 5 * sizeof(uint32_t));
+    // ... and, without a resident form, the whole refinement in one launch there,
+    // with the iterate as hi / lo planes padded like the PCG's exchanged vectors
+    if (persistent && !resident) {
         alloc(&w.xf_hi, (size_t)p->pw.n_pad * 3 * sizeof(float));
         alloc(&w.xf_lo, (size_t)p->pw.n_pad * 3 * sizeof(float));
     }
