@@ -5,7 +5,6 @@
 #include <atomic>
 #include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -33,7 +32,7 @@ inline void parallel_for(int count, int threads, const F &fn) {
     pool.reserve(std::max(0, std::min(threads, count) - 1));
     try {
         for (int t = 1; t < std::min(threads, count); ++t) pool.emplace_back(work);
-    } catch (const std::system_error &) {  // no more threads: the ones there are do it
+    } catch (...) {  // no more threads, or no memory for one: the ones there are do it
     }
     work();
     for (auto &t : pool) t.join();
