@@ -10,11 +10,13 @@ step; the timed run is the workload's 50 steps from its initial state.
          L2 flushed between steps outside the timed events.
   e2e    the same steps through the public solver API with the state in
          pinned host memory: H2D copy of (q, qd), step, D2H copy of (q, qd).
-  roofline  the persistent PCG kernel (the dominant kernel), from an eager
-         stage-by-stage pass timed with CUDA events on the launch stream.
+  roofline  the PCG kernel (the dominant kernel), from an eager stage-by-stage
+         pass timed with CUDA events on the launch stream.  The resident PCG
+         reads H once a solve and then waits on its exchanges, so its bytes
+         say little: the entry gives the time of an iteration beside them.
 
---workload batched512 steps the batch of 512 uneven beams (per-body PCGs in
-one persistent launch): value = batch steps/s (every body advanced one step).
+--workload batched512 steps the batch of 512 uneven beams (per-body PCGs, a
+cluster of CTAs a body): value = batch steps/s (every body advanced one step).
 
 --impl reference times the OpenMP C++ restatement of the step
 (oracle/cpu_step.cpp) on all host cores instead: the reference's own Warp
@@ -184,6 +186,40 @@ def ncu_traffic_per_launch(summary="pcg_kernel_nh_beam.md"):
         return None
     m = re.search(r"dram_bytes_per_launch:\s*([0-9.eE+]+)", text)
     return float(m.group(1)) if m else None
+
+
+def sm_count():
+    import torch
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
+def runs_resident(solver, pc):
+    """Whether a one-mesh fp32 plan of these workloads runs the resident PCG:
+    explicit CTAs and the other variants keep the windowed or global-memory
+    forms, and a part holds at most 1,024 rows, with a factor 256."""
+    cfg = solver.config
+    if cfg.pcg_ctas != 0 or cfg.pcg_variant not in (0, 2, 4):
+        return False
+    return solver.n <= sm_count() * (1024 if pc == "block_jacobi" else 256)
+
+
+def resident_roofline(pc, nnzb, n, solves, iterations, pcg_ms):
+    """The resident PCG: the bytes a solve reads and writes once -- per block of
+    H its 36 bytes, slot and column, per row M (block-Jacobi), the right-hand
+    side, x in and out; per factor block and pass 20 bytes, slot and column --
+    and the time of an iteration, which is what bounds it.  `iterations`: of
+    the longest body, with the initial residual's product."""
+    once = 42.0 * nnzb + 72.0 * n
+    if pc != "block_jacobi":
+        once += 26.0 * (nnzb + n) - 36.0 * n
+    peak, src = hbm_peak()
+    achieved = once * solves / (pcg_ms / 1000.0) / 1e9
+    return {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "us_per_iteration": 1000.0 * pcg_ms / iterations,
+            "kernel": "pcg_resident_kernel" if pc == "block_jacobi" else "pcg_resident_factor_kernel",
+            "algorithmic_bytes_per_launch": once, "avg_launch_ms": pcg_ms / solves, "peak_source": src,
+            "note": "H is read once a solve and held on the chip (what does not fit is streamed from L2); an iteration "
+                    "is a chain of product, block sums, exchange and scalars"}
 
 
 def max_over_ranks(seconds: float, world: int, device=None) -> float:
@@ -388,6 +424,7 @@ def run_batched(args, rank, world, local_rank):
     pcg_ms = 0.0
     assemble_ms = 0.0
     solves = 0
+    longest = 0.0
     bytes_pcg = 0.0
     row_ptr = solver.read_buffer("row_ptr").cpu().numpy()
     voff = batch.vertex_offsets
@@ -420,6 +457,7 @@ def run_batched(args, rank, world, local_rank):
             assemble_ms += ea.elapsed_time(e0)
             solves += 1
         st = bs.body_stats()
+        longest += float((st["iterations"].max(axis=1) + 1.0).sum())
         bytes_pcg += float(((st["iterations"].astype(np.float64) + 1.0) * per_it_b[None, :]).sum())
         Bst.particle_qd.copy_((x - A.particle_q) / batch.dt)
         A, Bst = Bst, A
@@ -433,6 +471,9 @@ def run_batched(args, rank, world, local_rank):
                 "bytes_per_body_iteration": (("64 nnzb_b + 208 n_b" if fsai else "40 nnzb_b + 172 n_b") +
                                              ", summed over bodies x (iterations_b + 1)"),
                 "avg_launch_ms": pcg_ms / solves, "peak_source": peak_src}
+    if layout["threads"] == 512:  # a cluster a body
+        roofline = resident_roofline(args.preconditioner, float(nnzb_b.sum()), u.n, solves, longest, pcg_ms)
+        roofline["traffic"] = None
 
     if rank != 0:
         return 0
@@ -650,6 +691,9 @@ def measure_variant(mesh, dev, precision, pc, steps, warmup, inner_tolerance, ou
                                "frac": achieved / peak, "bytes_per_iteration": b_it,
                                "formula": "64 nnzb + 208 n" if factor else "40 nnzb + 172 n",
                                "us_per_iteration": 1000.0 * pcg_ms / (its1 + spec.iterations)}
+        if runs_resident(solver, pc):
+            out["pcg_roofline"] = resident_roofline(pc, solver.nnzb, mesh.n, spec.iterations, its1 + spec.iterations,
+                                                    pcg_ms)
     solver.close()
     return out
 
@@ -703,7 +747,7 @@ def extra_workloads(dev, steps=3):
     (128x32x32 cells, 786,432 tets, E log-uniform [1e4, 1e7]) with the plain
     fp32 PCG, FSAI, and the fp16 / bf16 blocks in the fp64 refinement at the
     config's tolerances (inner 1e-3, outer 1e-8); and the 512 uneven bodies
-    in one launch with block-Jacobi and FSAI."""
+    in one plan with block-Jacobi and FSAI."""
     from mfem_gb300 import beams
     out = {}
     mesh = beams.build_beam("stiff_beam")
@@ -865,13 +909,16 @@ def measure_batched(dev, pc, steps, B=512):
     peak, _ = hbm_peak()
     achieved = bytes_pcg / (pcg_ms / 1000.0) / 1e9
     it_all = np.stack(its)
+    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+                "formula": ("64 nnzb_b + 208 n_b" if factor else "40 nnzb_b + 172 n_b") +
+                           " per body iteration, summed over bodies x (iterations_b + 1)"}
+    if bs.layout()["threads"] == 512:  # a cluster a body
+        longest = float((st["iterations"].max(axis=1) + 1.0).sum())
+        roofline = resident_roofline(pc, float(nnzb_b.sum()), batch.union.n, solver.iterations, longest, pcg_ms)
     return {"batch_steps_per_s": 1000.0 * steps / total_ms, "body_steps_per_s": B * 1000.0 * steps / total_ms,
             "steps": steps, "status_codes": sorted(codes), "schedule": bs.layout(),
             "pcg_iterations_per_body_step": {"mean": float(it_all.mean()), "max": int(it_all.max())},
-            "pcg_roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak,
-                             "formula": ("64 nnzb_b + 208 n_b" if factor else "40 nnzb_b + 172 n_b") +
-                                        " per body iteration, summed over bodies x (iterations_b + 1)"}}
+            "pcg_roofline": roofline}
 
 
 def run_gb300(args, rank, world, local_rank):
@@ -1065,7 +1112,17 @@ def run_gb300(args, rank, world, local_rank):
             "algorithmic_bytes_per_launch": b_it * per_launch_iters, "bytes_per_pcg_iteration": b_it,
             "bytes_per_pcg_iteration_formula": "64 nnzb + 208 n"})
         roofline["frac"] = roofline["achieved"] / peak
-    elif args.precision != "fp32" or args.preconditioner != "block_jacobi":
+    if args.precision == "fp32" and runs_resident(solver, args.preconditioner):
+        roofline = resident_roofline(args.preconditioner, nnzb, mesh.n, prof_solves, prof_iters + prof_solves,
+                                     stage_ms["pcg"])
+        roofline["pcg_iterations_per_launch"] = per_launch_iters - 1
+        captured = {("nh_beam", "block_jacobi"): "pcg_resident_kernel_nh_beam.md",
+                    ("nh_beam", "fsai"): "pcg_resident_factor_kernel_nh_beam.md",
+                    ("stiff_beam", "block_jacobi"): "pcg_resident_kernel_stiff_beam.md"}.get(
+                        (args.workload, args.preconditioner))
+        roofline["traffic"] = ncu_traffic_per_launch(captured) if captured else None
+        roofline["traffic_note"] = f"DRAM bytes of one captured launch, profiles/{captured}" if captured else None
+    elif args.precision != "fp32" or (args.preconditioner != "block_jacobi" and variant != "factor"):
         # the persistent fp32 PCG does not run: the mixed-precision or
         # global-memory factor solves are reported as a whole
         # (stage_ms_per_step["pcg"])
