@@ -314,11 +314,13 @@ void mfem_solver_config_default(mfem_solver_config *cfg);
  * the default) or the mixed-precision iterative refinement (BF16 / FP16
  * blocks, fp32 inner PCG to inner_tolerance with the plan's preconditioner,
  * fp64 residual; stops at outer_tolerance or after outer_max_iterations
- * corrections, starting from the reference's warm start).  Where the plan
- * has a persistent factor PCG layout (pcg_variant 4, or the block-Jacobi one
- * a one-mesh plan keeps when it fits) the inner solves run there, on an fp32
- * copy of the 16-bit blocks, for the residual scaled to unit norm; else in
- * the global-memory inner PCG.  It has no reference counterpart: it is the
+ * corrections, starting from the reference's warm start).  The inner solves
+ * run, for the residual scaled to unit norm, in the resident PCG where the plan
+ * has it for them, else where its vertex order allows in a windowed one (the
+ * single-reduction PCG with fp32 blocks and block-Jacobi, or the persistent
+ * factor PCG), else in the global-memory inner PCG.  The windowed forms sum
+ * dot products in fp32; the last one and the resident PCG in its place in
+ * fp64.  It has no reference counterpart: it is the
  * mixed-precision variant of src/mfem/refinement/solver.py:581-609.
  * Synchronises the device and drops the plan's captured graphs. */
 int mfem_plan_set_solver(mfem_plan *plan, const mfem_solver_config *cfg);
@@ -387,8 +389,9 @@ const char *mfem_train_last_error(void);
  * of body b are [vertex_offsets[b], vertex_offsets[b+1]), its tets
  * [tet_offsets[b], tet_offsets[b+1]), and no tet joins two bodies.  Each body
  * has its own energy (mfem_energy) and gravity [3].  The step then solves one
- * block-Jacobi PCG per body (own scalars and stopping test, the reference's
- * solve applied to each body) in a single persistent launch; the other
+ * PCG per body (own scalars and stopping test, the reference's solve applied
+ * to each body): on a cluster of CTAs a body, one launch a cluster size, where
+ * every body fits one, else all in a single persistent launch; the other
  * kernels run on the union.  Needs a plan created with line_search = 0 and
  * the FP32 solve.  No reference counterpart (the reference steps one body
  * per solver).  Synchronises the device and drops captured graphs. */

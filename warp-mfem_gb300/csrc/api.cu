@@ -73,7 +73,8 @@ struct mfem_plan {
     // reference's float32 PCG
     IrWork ir{};
     std::vector<void *> ir_allocs;
-    // independent bodies (mfem_plan_set_bodies): per-body PCGs in one launch
+    // independent bodies (mfem_plan_set_bodies): the arrays of their per-body
+    // PCGs, and the schedule of the global-memory form
     BatchViews bw{};
     std::vector<void *> batch_allocs;
     // block-Jacobi bodies on the resident PCG: one launch per cluster size, the
@@ -130,7 +131,8 @@ struct mfem_plan {
 namespace {
 
 // Rows a CTA up to which one cluster beats a grid: 16 CTAs of 370 rows 3.0 us
-// an iteration.
+// an iteration.  (Shared memory ends a cluster's range first, at some 6,000 rows
+// of a beam.)
 constexpr int kClusterRows = 400;
 // Rows up to which every solve of one mesh adds its sums in the ordered way.
 constexpr int kOrderedRows = 384;
@@ -559,8 +561,10 @@ struct FactorPattern {
 // meshes (two orders of the sums move the velocities of a step by 2e-5 at 96
 // vertices, 7e-6 at 330, 1e-6 at 2,673).  That costs 0.25 us an iteration on
 // one CTA, 0.3 in a cluster and 0.25 on a grid, and needs row ranges with
-// short halos: banded orders, or at most 1,024 rows.  Else, and where that
-// does not fit, on parts bisected by position.
+// short halos and a windowed layout that holds H: banded orders, or at most
+// 1,024 rows.  Else, and where that does not fit, on parts bisected by
+// position; there a line search's step moves with the order of the sums, by up
+// to 2.2e-5 in the velocities at the stiffest material.
 cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q, int max_ctas) {
     constexpr int kRows = kPartWarps * kPartSliceRows;
     const bool windowed = p->pl.variant == PcgLayout::kSingleReduction && p->pl.cache_matrix;
@@ -594,11 +598,12 @@ cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q
     return cudaSuccess;
 }
 
-// The resident factor PCG of one mesh with preconditioner 2 or 3, where a
-// step's result does not turn on the PCG's rounding (plan_resident): a grid
-// whose CTAs recompute the passes on their halos.  (A cluster that exchanges
-// the passes' results instead took 6.1 us an iteration against 4.4 at 637
-// vertices and 7.9 against 4.6 at 2,673.)
+// The resident factor PCG of one mesh with preconditioner 2 or 3, but for line
+// searches and small meshes, where a step follows the PCG's last bits
+// (plan_resident) and this form has no ordered sums: it moves a step's
+// velocities there by up to 2e-5.  A grid whose CTAs recompute the passes on
+// their halos.  (A cluster that exchanges the passes' results instead took 6.1
+// us an iteration against 4.4 at 637 vertices and 7.9 against 4.6 at 2,673.)
 cudaError_t plan_resident_factor(mfem_plan *p, int max_ctas) {
     if (p->cfg.line_search || p->n <= kOrderedRows) return cudaSuccess;
     const int parts = std::min(std::min(max_ctas, kPartMaxGrid), (p->n + kFactorGridRows - 1) / kFactorGridRows);

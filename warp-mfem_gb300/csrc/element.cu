@@ -35,7 +35,7 @@ __device__ __forceinline__ void load_vec3(const float *__restrict__ p, int i, fl
 // and four scalar loads for each 16-byte store.  331,200 tets: 138 -> 135 us,
 // and 126 us with four blocks an SM at 128 registers instead of three at 168
 // (160 bytes of spills a thread): latency of dependent arithmetic and fetching
-// 100 KB of straight-line code bound it, at 43% of the issue slots.
+// 100 KB of straight-line code bound it, at 48% of the issue slots (42% before).
 constexpr int kElementWarps = kElementThreads / 32;
 constexpr int kElementSmem = kElementWarps * 32 * kKeRecord * (int)sizeof(float);
 constexpr int kElementOneWave = 3 * 152;

@@ -28,17 +28,20 @@
 //                       narrow), its norm in fp64, partial sums; the last block
 //                       to finish adds the partials in a fixed order and
 //                       decides (converged / outer cap)
-//   ir_pcg_kernel<T>    persistent cooperative PCG on Hq e = r, e0 = 0
+//   ir_pcg_kernel<T>    persistent cooperative PCG on Hq e = r, e0 = 0, vectors
+//                       in global memory, dot products and scalars in fp64
 //
 // Precision FP32 (kIrFp32) keeps the fp32 H in the inner PCG from the start
 // and converts nothing: the plain fp32 PCG inside the same fp64 refinement,
 // for a solution whose fp64 residual reaches the outer tolerance.
 //
-// A plan on the persistent factor PCG (pcg_factor.cu) runs the inner solves
-// there instead: ir_convert_kernel also writes Hq padded to 20-byte blocks
-// (which that kernel widens and scales by the row scale as it loads them), and
-// the residual kernel hands over r / ||r|| (so the fp32 sums of products
-// cannot underflow) with ||r|| to scale the correction back.
+// ir_pcg_kernel is the last resort: a plan with a resident layout runs the
+// inner solves there (pcg_resident.cu, pcg_resident_factor.cu), one with a
+// windowed layout in the single-reduction PCG (pcg.cu) or the persistent factor
+// PCG (pcg_factor.cu).  For those ir_convert_kernel also writes Hq padded to
+// 20-byte blocks (which they widen and scale by the row scale as they load
+// them), and the residual kernel hands over r / ||r|| (so that fp32 sums of
+// products do not underflow) with ||r|| to scale the correction back.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

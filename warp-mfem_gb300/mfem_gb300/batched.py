@@ -2,9 +2,10 @@
 
 ``BatchedSolver`` concatenates the bodies of a ``beams.BodyBatch`` into one
 mesh and one plan: the element, assembly and local-solve kernels run on the
-union, while the global solve is one block-Jacobi PCG per body (its own
-scalars and stopping test, as if each body were stepped alone with the
-reference's ``RefinementSolver.step``) in a single persistent launch.  The
+union, while the global solve is one PCG per body (its own scalars and
+stopping test, as if each body were stepped alone with the reference's
+``RefinementSolver.step``): on a cluster of CTAs a body where every body fits
+one, else all in a single persistent launch.  The
 reference has no counterpart: it steps one body per solver.
 The plain update is used (no line search), with the fp32 PCG.
 """
