@@ -275,6 +275,16 @@ bool valid_config(const mfem_config *cfg, std::string &err) {
     return false;
 }
 
+// A system that no preconditioner scales: none, or a singular threshold above
+// the default, which makes blocks the identity.  The single-reduction
+// recurrence loses digits there that the standard one keeps: of 288 bodies
+// with attachment stiffness up to 1e4 ten broke down that the latter converged
+// on (worst true residual 3.2e-1 for 1.2e-2), and the others took 10 % more
+// iterations.  With any preconditioner both converge alike.
+bool unscaled(const mfem_config &cfg) {
+    return cfg.preconditioner == 0 || (cfg.preconditioner == 1 && cfg.preconditioner_singular_threshold > 1.0e-20f);
+}
+
 // The resident layout on which a one-mesh plan's solves run in refinement mode
 // `mode` (0: the fp32 PCG), or null: the form that the vertex order allows.
 // With block-Jacobi the 16-bit refinements keep their own kernel where the
@@ -564,8 +574,10 @@ struct FactorPattern {
 // short halos and a windowed layout that holds H: banded orders, or at most
 // 1,024 rows.  Else, and where that does not fit, on parts bisected by
 // position; there a line search's step moves with the order of the sums, by up
-// to 2.2e-5 in the velocities at the stiffest material.
+// to 2.2e-5 in the velocities at the stiffest material.  An unscaled system
+// takes it only in place of the windowed kernel of the same recurrence.
 cudaError_t plan_resident(mfem_plan *p, const Symbolic &sym, const float *rest_q, int max_ctas) {
+    if (unscaled(p->cfg) && p->pl.variant != PcgLayout::kSingleReduction) return cudaSuccess;
     constexpr int kRows = kPartWarps * kPartSliceRows;
     const bool windowed = p->pl.variant == PcgLayout::kSingleReduction && p->pl.cache_matrix;
     const bool rounding = p->cfg.line_search || p->n <= kOrderedRows;
@@ -1917,8 +1929,9 @@ int install_bodies(mfem_plan *p, int n_bodies, const int32_t *voff, const int32_
     int rc = n_bodies == 1 ? apply_batch_layout(p, 512, 2048.0, std::max(1, sms))
                            : apply_batch_layout(p, 256, 2048.0, INT_MAX);
     // pcg_variant 5 asks for the global-memory PCG; a one-body batch of a mesh
-    // too large for the persistent PCGs has no gravity of its own
-    if (rc == MFEM_OK && gravity && p->cfg.pcg_ctas == 0 &&
+    // too large for the persistent PCGs has no gravity of its own; unscaled
+    // bodies keep the standard recurrence
+    if (rc == MFEM_OK && gravity && p->cfg.pcg_ctas == 0 && !unscaled(p->cfg) &&
         (p->cfg.pcg_variant == PcgLayout::kAuto || p->cfg.pcg_variant == PcgLayout::kSingleReduction)) {
         e = plan_bodies(p, n_bodies, voff);
         if (e != cudaSuccess) rc = cuda_fail(p, e, "resident bodies");
