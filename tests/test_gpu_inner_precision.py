@@ -11,7 +11,7 @@ recurrence are allowed elsewhere."""
 import pytest
 import torch
 
-from mfem_gb300 import Model, MixedFEMSolver, beams
+from mfem_gb300 import Model, MixedFEMSolver, _lib, beams
 from test_gpu_resident import shuffled
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +42,34 @@ def test_inner_solve_reaches_a_tolerance_below_float32_sums(cells, pc, precision
     assert b["inner_iterations"] < 5000, b
     assert abs(a["inner_iterations"] - b["inner_iterations"]) <= max(2, b["inner_iterations"] // 50), (a, b)
     assert a["rel_residual"] <= 2.0 * b["rel_residual"], (a, b)
+
+
+@pytest.mark.parametrize("cells", [(16, 16, 16), (20, 20, 20)], ids=["cluster", "grid"])
+@pytest.mark.parametrize("pc", ["block_jacobi", "fsai"])
+def test_injected_timeout_is_reported_and_the_plan_recovers(cells, pc):
+    mesh = shuffled(beams.build_beam("cantilever", cells=cells))
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=2, energy=mesh.spec.energy, line_search=False, preconditioner=pc,
+                            solver_precision="fp16", outer_tolerance=1e-6, inner_tolerance=1e-2)
+    a, b = model.state(), model.state()
+    solver.step(a, b, None, None, mesh.spec.dt)
+    assert all(st["status"] == _lib.MFEM_OK for st in solver.solve_stats())
+    want = b.particle_q.clone()
+    s, lam = solver.tet_stretch.clone(), solver.tet_lambda.clone()
+    solver.inject_timeout()
+    solver.step(a, b, None, None, mesh.spec.dt)
+    with pytest.raises(_lib.MfemError) as err:
+        solver.solve_stats()
+    assert err.value.code == _lib.MFEM_TIMEOUT
+    solver.write_buffer("tet_stretch", solver_start(mesh)[0])
+    solver.write_buffer("tet_lambda", solver_start(mesh)[1])
+    solver.step(a, b, None, None, mesh.spec.dt)
+    assert all(st["status"] == _lib.MFEM_OK for st in solver.solve_stats())
+    assert torch.equal(b.particle_q, want) and torch.equal(solver.tet_stretch, s) and torch.equal(solver.tet_lambda, lam)
+
+
+def solver_start(mesh):
+    """s and lambda of a new plan."""
+    model = Model.from_beam(mesh, device=DEV)
+    solver = MixedFEMSolver(model, iterations=1, energy=mesh.spec.energy, line_search=False)
+    return solver.tet_stretch.reshape(-1).clone(), solver.tet_lambda.reshape(-1).clone()

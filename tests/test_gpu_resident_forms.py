@@ -151,6 +151,18 @@ def test_breakdown_of_an_inner_solve_falls_back_to_block_jacobi(precision, cells
     assert float((xa - xb).abs().max()) <= 1e-4 * float(xb.abs().max())
 
 
+# -- what a refined factor solve solves -----------------------------------------
+@pytest.mark.parametrize("precision", ["fp16", "bf16", "fp32_refined"])
+@pytest.mark.parametrize("pc", ["fsai", "learned"])
+def test_factor_refinement_has_the_block_jacobi_refinements_solution(precision, pc):
+    mesh = beams.build_beam("nh_beam", cells=(24, 13, 12))
+    kw = dict(outer_tolerance=1e-6, inner_tolerance=1e-2)
+    a, xa = solve(mesh, preconditioner=pc, solver_precision=precision, **kw)
+    b, xb = solve(mesh, solver_precision="fp32_refined", **kw)
+    assert a.mixed_stats()[0]["rel_residual"] <= 1e-6 and b.mixed_stats()[0]["rel_residual"] <= 1e-6
+    assert float((xa - xb).abs().max()) <= 1e-4 * float(xb.abs().max())
+
+
 # -- the forms that explicit settings select -----------------------------------
 @pytest.mark.parametrize("kw", [dict(), dict(solver_precision="fp32_refined"), dict(solver_precision="fp16"),
                                 dict(preconditioner="fsai"), dict(preconditioner="fsai", solver_precision="fp16")],

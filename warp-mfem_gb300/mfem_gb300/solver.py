@@ -48,7 +48,7 @@ class MixedFEMSolver:
     residual.
 
     ``preconditioner`` is the reference's flag (True: block-Jacobi, False:
-    none), "fsai": a factorized sparse approximate inverse M = G^T G with G
+    none, which keeps shuffled meshes and batches on the slower standard PCG), "fsai": a factorized sparse approximate inverse M = G^T G with G
     lower block-triangular on H's block pattern, recomputed after every
     assembly, or "learned": M = L L^T with L written by the factor net
     (``factor_net``; parameters ``factor_net_params`` or the shipped
