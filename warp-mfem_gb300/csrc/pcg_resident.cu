@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
     constexpr bool kWide = sizeof(Sum) > sizeof(float);
     constexpr int kSums = SCOPE == kCluster ? kPartMaxCluster * kBlocks : 1;  // partial sums of a round
     __shared__ Sum s_red[kBlocks][3][kPartWarps];
-    __shared__ __align__(16) Sum s_part[2][kSums][4];
+    __shared__ __align__(16) typename Part<Sum>::type s_part[2][kSums];
 
     __shared__ __align__(8) uint64_t s_mbar[2];
     __shared__ __align__(16) Verdict s_verdict;
@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         }
     }
     if (SCOPE == kGrid && warp == 0) target = grid_count(a.counter) / ncta * ncta;
-    for (int i = tid; SCOPE == kCluster && i < 2 * kSums * 4; i += kPartThreads) (&s_part[0][0][0])[i] = 0.0f;
+    for (int i = tid; SCOPE == kCluster && i < 2 * kSums; i += kPartThreads)
+        s_part[i / kSums][i % kSums] = typename Part<Sum>::type{};
     if (ORDERED) {
         for (int i = tid; i < kBlocks * 3 * kPartWarps; i += kPartThreads)
             s_red[i / (3 * kPartWarps)][i / kPartWarps % 3][i % kPartWarps] = 0.0f;
@@ -427,14 +428,14 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
         bool ok = true;
         if (SCOPE == kCluster && tid == 0)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&s_mbar[buf])),
-                         "r"((uint32_t)(4 * sizeof(Sum)) * (uint32_t)(ORDERED ? a.blocks : ncta) + 16u * (uint32_t)part.nhalo)
+                         "r"(16u * (uint32_t)((kWide ? 2 : 1) * (ORDERED ? a.blocks : ncta) + part.nhalo))
                          : "memory");
         if (warp < (ORDERED ? part.nblocks : 1)) {
             // a block's sum, by a warp of its own
             const int b = ORDERED ? warp : 0;
             group_sum3(s_red[b][g][i] + s_red[b][g][i + 8], sum);
             if (SCOPE == kCluster && lane < ncta)
-                push_sums(s_part[buf][ORDERED ? part.block_lo + b : rank], &s_mbar[buf], lane, sum);
+                push_sums(&s_part[buf][ORDERED ? part.block_lo + b : rank], &s_mbar[buf], lane, sum);
         }
         if (warp == 0) {
             if (SCOPE == kOne && ORDERED && part.nblocks > 1) {
@@ -450,14 +451,14 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_kernel(ResArgs a
 #pragma unroll
                     for (int b = 0; b < kSums; b += 32)  // zero past the last block
                         if (b < a.blocks) {
-                            const Sum *q = s_part[buf][b + lane < kSums ? b + lane : 0];
-                            t[0] += q[0];
-                            t[1] += q[1];
-                            t[2] += q[2];
+                            const float4 q = *reinterpret_cast<const float4 *>(&s_part[buf][b + lane < kSums ? b + lane : 0]);
+                            t[0] += q.x;
+                            t[1] += q.y;
+                            t[2] += q.z;
                         }
                     spread_sum3(warp_sum3(t, lane), sum);
                 } else {
-                    const Sum *t = s_part[buf][0] + g;
+                    const Sum *t = reinterpret_cast<const Sum *>(s_part[buf]) + g;
                     group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
                 }
             }

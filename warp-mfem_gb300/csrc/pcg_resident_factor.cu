@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
     constexpr bool kWide = sizeof(Sum) > sizeof(float);
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Sum s_red[3][kPartWarps];
-    __shared__ __align__(16) Sum s_part[2][kPartMaxCluster][4];
+    __shared__ __align__(16) typename Part<Sum>::type s_part[2][kPartMaxCluster];
     __shared__ __align__(8) uint64_t s_mbar[4];  // rounds (two), y, u
     __shared__ __align__(16) Verdict s_verdict;
     __shared__ Sum s_norm[2];
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
         }
     }
     if (SCOPE == kGrid && warp == 0) target = grid_count(a.counter) / ncta * ncta;
-    if (SCOPE == kCluster && tid < 2 * kPartMaxCluster * 4) (&s_part[0][0][0])[tid] = 0.0f;
+    if (SCOPE == kCluster && tid < 2 * kPartMaxCluster) s_part[0][tid] = typename Part<Sum>::type{};
     __syncthreads();
     int err = s_err;
     if (SCOPE == kCluster) {
@@ -365,9 +365,9 @@ __global__ void __launch_bounds__(kPartThreads, 1) pcg_resident_factor_kernel(Fa
             if (SCOPE == kCluster && lane == 0) expect(&s_mbar[buf], (int)(sizeof(Sum) / 4) * ncta + part.nhalo);
             group_sum3(s_red[g][i] + s_red[g][i + 8], sum);
             if (SCOPE == kCluster) {
-                if (lane < ncta) push_sums(s_part[buf][rank], &s_mbar[buf], lane, sum);
+                if (lane < ncta) push_sums(&s_part[buf][rank], &s_mbar[buf], lane, sum);
                 ok = __all_sync(0xffffffffu, wait_phase(&s_mbar[buf], (k >> 1) & 1u));
-                const Sum *t = s_part[buf][0] + g;
+                const Sum *t = reinterpret_cast<const Sum *>(s_part[buf]) + g;
                 group_sum3(t[4 * i] + t[4 * (i + 8)], sum);
             }
             if (SCOPE == kGrid) {

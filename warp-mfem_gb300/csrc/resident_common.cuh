@@ -156,12 +156,23 @@ __device__ __forceinline__ void group_sum3(Sum k, Sum sum[3]) {
     for (int i = 0; i < 3; ++i) sum[i] = __shfl_sync(0xffffffffu, k, 8 * i);
 }
 
-// A CTA's three partial sums (16 bytes, or 32 in fp64) into CTA `rank`'s
-// shared memory.
-__device__ __forceinline__ void push_sums(const void *dst, const void *mbar, int rank, const float s[3]) {
+// A CTA's three partial sums in shared memory, and their way into CTA `rank`'s.
+template <class Sum>
+struct Part {
+    typedef float4 type;
+};
+template <>
+struct Part<double> {
+    struct alignas(16) type {
+        double v[4];
+    };
+};
+__device__ __forceinline__ void push_sums(const float4 *dst, const void *mbar, int rank, const float s[3]) {
     push16(dst, mbar, rank, s[0], s[1], s[2]);
 }
-__device__ __forceinline__ void push_sums(const double *dst, const void *mbar, int rank, const double s[3]) {
+__device__ __forceinline__ void push_sums(const Part<double>::type *part, const void *mbar, int rank,
+                                          const double s[3]) {
+    const double *dst = part->v;
     push16(dst, mbar, rank, __int_as_float(__double2loint(s[0])), __int_as_float(__double2hiint(s[0])),
            __int_as_float(__double2loint(s[1])), __int_as_float(__double2hiint(s[1])));
     push16(dst + 2, mbar, rank, __int_as_float(__double2loint(s[2])), __int_as_float(__double2hiint(s[2])), 0.0f);
@@ -203,12 +214,13 @@ __device__ __forceinline__ void add_product(float a, float b, double &sum) { sum
 // instead of 18 (7,560 rows: 8.4 -> 7.0 us an iteration).
 __device__ __forceinline__ void add_rows(const float r[3], const float u[3], const float w[3], bool own, int,
                                          float sum[3]) {
-    if (!own) return;
+    if (own) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        add_product(r[c], u[c], sum[0]);
-        add_product(w[c], u[c], sum[1]);
-        add_product(r[c], r[c], sum[2]);
+        for (int c = 0; c < 3; ++c) {
+            add_product(r[c], u[c], sum[0]);
+            add_product(w[c], u[c], sum[1]);
+            add_product(r[c], r[c], sum[2]);
+        }
     }
 }
 __device__ __forceinline__ void add_rows(const float r[3], const float u[3], const float w[3], bool own, int lane,
